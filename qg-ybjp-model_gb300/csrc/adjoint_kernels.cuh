@@ -2,7 +2,7 @@
 // layout double2 [nz][n][n/2+1] and physical layout double [nz][n][n]).
 #pragma once
 #include "dense_kernels.cuh"
-#include "step_kernels.cuh"
+#include "step_fx.cuh"
 
 namespace qg {
 
@@ -125,36 +125,22 @@ struct AdjP {
 struct AdjIn { const double2* l[6]; };                   // (lq, lr, lBR, lBI, lcR, lcI) after the step
 struct AdjOut { double2* l[6]; double2* lpsi; double2* lAR; double2* lAI; };
 
-// transposed time update of one mode: outputs before the solves and the
-// product terms, and the adjoint tendencies of q, BR, BI
-__device__ __forceinline__ void adj_update(const AdjP& p, const AdjIn& L, long long m, double e1, double e2,
-                                           double e1w, double e2w, double2 o[6], double2& lNq, double2& lTR,
-                                           double2& lTI) {
-  const double2 lq1 = L.l[0][m], lBR1 = L.l[2][m], lBI1 = L.l[3][m];
+// transposed time update of one mode of variable w (0 q, 1 BR, 2 BI), e1, e2
+// its integrating factors: the adjoint tendency, and the outputs before the
+// solves and the product terms (new level, old level)
+__device__ __forceinline__ void adj_update(const AdjP& p, const AdjIn& L, int w, long long m, double e1, double e2,
+                                           double2& lt, double2& on, double2& oo) {
+  const int fn = w == 0 ? 0 : 1 + w, fo = w == 0 ? 1 : 3 + w;      // (lq, lr), (lBR, lcR), (lBI, lcI)
+  const double2 l1 = L.l[fn][m], lo = L.l[fo][m];
   if (p.first) {
-    const double2 lr1 = L.l[1][m], lcR1 = L.l[4][m], lcI1 = L.l[5][m];
-    o[0] = cadd(lr1, cscale(lq1, e1));
-    o[2] = cadd(lcR1, cscale(lBR1, e1w));
-    o[3] = cadd(lcI1, cscale(lBI1, e1w));
-    o[1] = o[4] = o[5] = make_double2(0.0, 0.0);
-    lNq = cscale(lq1, -p.dt * e1);
-    lTR = cscale(lBR1, -p.dt * e1w);
-    lTI = cscale(lBI1, -p.dt * e1w);
+    lt = cscale(l1, -p.dt * e1);
+    on = cadd(lo, cscale(l1, e1));
+    oo = make_double2(0.0, 0.0);
   } else {
-    const double2 lr1 = L.l[1][m], lcR1 = L.l[4][m], lcI1 = L.l[5][m];
-    const double g = p.gam, d2 = 2.0 * p.dt;
-    const double2 lqp = cadd(lq1, cscale(lr1, g));
-    const double2 lRp = cadd(lBR1, cscale(lcR1, g));
-    const double2 lIp = cadd(lBI1, cscale(lcI1, g));
-    o[0] = cscale(lr1, 1.0 - 2.0 * g);
-    o[2] = cscale(lcR1, 1.0 - 2.0 * g);
-    o[3] = cscale(lcI1, 1.0 - 2.0 * g);
-    o[1] = cadd(cscale(lr1, g), cscale(lqp, e2));
-    o[4] = cadd(cscale(lcR1, g), cscale(lRp, e2w));
-    o[5] = cadd(cscale(lcI1, g), cscale(lIp, e2w));
-    lNq = cscale(lqp, -d2 * e1);
-    lTR = cscale(lRp, -d2 * e1w);
-    lTI = cscale(lIp, -d2 * e1w);
+    const double2 lp = cadd(l1, cscale(lo, p.gam));
+    lt = cscale(lp, -2.0 * p.dt * e1);
+    on = cscale(lo, 1.0 - 2.0 * p.gam);
+    oo = cadd(cscale(lo, p.gam), cscale(lp, e2));
   }
 }
 
@@ -163,274 +149,247 @@ __device__ __forceinline__ double2 rt_scale(double2 v, int kx, int ky, double in
   return (kx == 0 && ky == 0) ? make_double2(2.0 * v.x * inv2n2, 0.0) : cscale(v, inv2n2);
 }
 
-// packed spectrum X + iY of two real rows from half-spectrum values given at
-// kk = k (k <= K) or kk = n - k (k >= n - K); imaginary parts at kx = 0 ignored
-__device__ __forceinline__ double2 pack_xy(double2 X, double2 Y, int k, int K, int n) {
-  if (k == 0) return make_double2(X.x, Y.x);
-  if (k <= K) return make_double2(X.x - Y.y, X.y + Y.x);
-  if (k >= n - K) return make_double2(X.x + Y.y, Y.x - X.y);
-  return make_double2(0.0, 0.0);
+// packed spectrum X + iY of two half spectra get(kk, X, Y) at k = j + r NB
+template <int N, class Get> __device__ __forceinline__ void adj_pack(int j, int K, double2 (&d)[8], Get get) {
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    d[r] = make_double2(0.0, 0.0);
+    if (fx_zero_in<8>(r)) continue;
+    const int k = j + r * (N / 8), kk = r < 4 ? k : N - k;
+    if (kk > K) continue;
+    double2 X, Y;
+    get(kk, X, Y);
+    if (k == 0) d[r] = make_double2(X.x, Y.x);           // imaginary parts at kx = 0 are ignored
+    else if (r < 4) d[r] = make_double2(X.x - Y.y, X.y + Y.x);
+    else d[r] = make_double2(X.x + Y.y, Y.x - X.y);
+  }
 }
 
+// y-inverse transforms of one plane of a column tile: get(row, ky) is the
+// value at a retained row; stored to plane f of S
+template <int N, class Get>
+__device__ __forceinline__ void adj_col_inverse(const FxColCtx<N>& c, const Geom& g, int kx, double2* __restrict__ dst,
+                                                Get get) {
+  constexpr int NB = N / 8;
+  double2 d[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    d[r] = make_double2(0.0, 0.0);
+    if (fx_zero_in<8>(r)) continue;
+    int row; bool cj;
+    col_src(g, kx, c.j + r * NB, row, cj);
+    if (row < 0 || !g.mask(kx, g.ky_of_row(row))) continue;
+    d[r] = get(row, g.ky_of_row(row));
+    if (cj) d[r].y = -d[r].y;
+  }
+  fxc v[8];
+  int base;
+  c.template run<false>(d, v, base);
+  if (kx > g.K) return;
+  fx_doubles<8, true>(v, d, base);
+  double2* o = dst + (long long)c.j * g.KXP + kx;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) o[(long long)r * NB * g.KXP] = d[r];
+}
+
+// the transposed products' kernels keep one transform per thread in flight,
+// as the step's (step_fx.cuh)
 template <int N>
-__global__ void __launch_bounds__(kColThreads, Tiles<double, N>::MINB)
+__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(QG_FX_COL_CTAS))
 k_adj_col_inv(Geom g, AdjP p, int zbase, AdjIn L, const double* __restrict__ e1t, const double* __restrict__ e2t,
               const double* __restrict__ e1wt, const double* __restrict__ e2wt, double2* __restrict__ SA,
               const double2* __restrict__ twg) {
-  using T = double;
-  constexpr int CT = Tiles<T, N>::CT, LD = Tiles<T, N>::LD, NT = kColThreads;
+  using F = FxCol<N>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2* tw = reinterpret_cast<double2*>(smem_raw);
-  double2* buf = tw + N;                       // [6][CT][LD]
-  const int tid = threadIdx.x;
-  const int zb = blockIdx.y, z = zbase + zb;
-  const int kx0 = blockIdx.x * CT;
-  load_tw<T, N>(tw, twg, NT);
-  const long long zoff = (long long)z * g.plane;
+  __shared__ unsigned slots[F::SLOTS];
+  const FxColCtx<N> c = fx_col_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
+  const int zb = blockIdx.y, kx = blockIdx.x * F::CT + c.c;
+  const long long zoff = (long long)(zbase + zb) * g.plane;
   const double inv2n2 = 0.5 / ((double)N * (double)N);
-  for (int e = tid; e < CT * N; e += NT) {
-    const int c = e % CT, j = e / CT;
-    const int kx = kx0 + c;
-    const int r = g.row_of_fft_index(j);
-    double2 v[6];
-#pragma unroll
-    for (int f = 0; f < 6; ++f) v[f] = make_double2(0.0, 0.0);
-    if (kx <= g.K && r >= 0) {
-      const int ky = g.ky_of_row(r);
-      if (g.mask(kx, ky)) {
-        const long long m = zoff + (long long)r * g.KXP + kx, mt = (long long)r * g.KXP + kx;
-        double2 o[6], lN, lR, lI;
-        adj_update(p, L, m, e1t[mt], e2t[mt], e1wt[mt], e2wt[mt], o, lN, lR, lI);
-        lN = rt_scale(lN, kx, ky, inv2n2);
-        lR = rt_scale(lR, kx, ky, inv2n2);
-        lI = rt_scale(lI, kx, ky, inv2n2);
-        v[0] = lN; v[1] = cscale(cmul_mi(lN), (double)ky);
-        v[2] = lR; v[3] = cscale(cmul_mi(lR), (double)ky);
-        v[4] = lI; v[5] = cscale(cmul_mi(lI), (double)ky);
-      }
-    }
-#pragma unroll
-    for (int f = 0; f < 6; ++f) buf[(f * CT + c) * LD + pad_idx(j)] = v[f];
-  }
-  __syncthreads();
-  if (kx0 == 0) {
-    for (int e = tid; e < 6 * (N / 2 - 1); e += NT) {
-      const int f = e / (N / 2 - 1), j = 1 + e % (N / 2 - 1);
-      double2* col = buf + f * CT * LD;
-      col[pad_idx(N - j)] = cconj(col[pad_idx(j)]);
-    }
-    __syncthreads();
-  }
-  fft_ip<T, N, false, 3 * CT, NT, LD>(buf, tw);
-  fft_ip<T, N, false, 3 * CT, NT, LD>(buf + 3 * CT * LD, tw);
-#pragma unroll 4
-  for (int e = tid; e < 6 * CT * N; e += NT) {
-    const int c = e % CT, y = (e / CT) % N, f = e / (CT * N);
-    SA[scr_off(zb, f, y, N, g.KXP) + kx0 + c] = buf[(f * CT + c) * LD + pad_idx(y)];
+  // l and -i ky l of the adjoint tendencies of q, BR, BI
+  for (int f = 0; f < 6; ++f) {
+    const int w = f >> 1;
+    adj_col_inverse<N>(c, g, kx, SA + scr_off(zb, f, 0, N, g.KXP), [&](int row, int ky) {
+      const long long mt = (long long)row * g.KXP + kx;
+      double2 lt, on, oo;
+      adj_update(p, L, w, zoff + mt, w == 0 ? e1t[mt] : e1wt[mt], w == 0 ? e2t[mt] : e2wt[mt], lt, on, oo);
+      lt = rt_scale(lt, kx, ky, inv2n2);
+      return (f & 1) ? cscale(cmul_mi(lt), (double)ky) : lt;
+    });
   }
 }
 
 // rows: SF holds (u, v, zeta, q, BR, BI), SA the adjoint planes
 // (lNq, -i ky lNq, lTR, -i ky lTR, lTI, -i ky lTI) after the y-inverse FFT;
-// writes SA = (F_x lu, -i kx F_x lv - kx^2 F_x lZ, F_x lZ, F_x lQ, F_x lBR, F_x lBI)
+// writes SA = (F_x lu, -i kx F_x lv - kx^2 F_x lZ, F_x lZ, F_x lQ, F_x lBR, F_x lBI).
+// The physical u, v, zeta, q, BR, BI are parked in shared memory, each thread
+// its own eight points; the six sums of products accumulate in registers.
+template <int N> struct AdjRow {
+  static constexpr size_t smem() { return FxRow<N>::smem() + (size_t)3 * FxRow<N>::RT * N * sizeof(double2); }
+};
 template <int N>
-__global__ void __launch_bounds__(kThreadsB)
+__global__ void __launch_bounds__(FxRow<N>::NT, fx_row_ctas<N>(2))
 k_adj_row(Geom g, AdjP p, const double2* __restrict__ SF, double2* __restrict__ SA, const double2* __restrict__ twg) {
-  using T = double;
-  constexpr int RT = Tiles<T, N>::RT, LD = Tiles<T, N>::LD, NT = kThreadsB;
+  using F = FxRow<N>;
+  constexpr int NB = F::NB;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2* tw = reinterpret_cast<double2*>(smem_raw);
-  double2* bA = tw + N;                 // [7][RT][LD]
-  const int tid = threadIdx.x;
-  const int zb = blockIdx.y;
-  const int y0 = blockIdx.x * RT;
-  const int K = g.K;
-  load_tw<T, N>(tw, twg, NT);
+  __shared__ unsigned slots[F::SLOTS];
+  FxRowCtx<N> c = fx_row_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
+  // point (x = j + r NB) of pair q at park[(q * 8 + r) * NT]
+  double2* park = reinterpret_cast<double2*>(smem_raw) + fx_tw_count<N>() + F::RT * F::LD + threadIdx.x;
+  const int zb = blockIdx.y, y = blockIdx.x * F::RT + c.rr, K = g.K, j = c.j;
+  auto sf = [&](int f) { return SF + scr_off(zb, f, y, N, g.KXP); };
+  auto sa = [&](int f) { return SA + scr_off(zb, f, y, N, g.KXP); };
   const double adv = p.adv, hr = 0.5 * p.refr;
-  for (int e = tid; e < 7 * RT * N; e += NT) {
-    const int k = e % N, rr = (e / N) % RT, q = e / (RT * N);
-    const int y = y0 + rr;
-    const int kk = k <= K ? k : N - k;
-    double2 v = make_double2(0.0, 0.0);
-    if (k <= K || k >= N - K) {
-      double2 X, Y;
-      if (q < 3) {
-        X = SF[scr_off(zb, 2 * q, y, N, g.KXP) + kk];
-        Y = SF[scr_off(zb, 2 * q + 1, y, N, g.KXP) + kk];
-      } else if (q < 6) {
-        const int f = q - 3;
-        X = cscale(cmul_mi(SA[scr_off(zb, 2 * f, y, N, g.KXP) + kk]), adv * (double)kk);
-        Y = cscale(SA[scr_off(zb, 2 * f + 1, y, N, g.KXP) + kk], adv);
+  for (int q = 0; q < 3; ++q) {
+    double2 d[8], o[8];
+    const double2 *X = sf(2 * q), *Y = sf(2 * q + 1);
+    adj_pack<N>(j, K, d, [&](int kk, double2& a, double2& b) { a = X[kk]; b = Y[kk]; });
+    c.inverse_d(d, o);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) park[(q * 8 + r) * F::NT] = o[r];
+  }
+  double2 luv[8], lzq[8], lbb[8];
+  // (aq, aR, aI): l of q, BR, BI times (-i kx, d/dy) in physical space
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    double2 d[8], o[8];
+    const double2 *A = sa(2 * q), *B = sa(2 * q + 1);
+    adj_pack<N>(j, K, d, [&](int kk, double2& a, double2& b) {
+      a = cscale(cmul_mi(A[kk]), adv * (double)kk);
+      b = cscale(B[kk], adv);
+    });
+    c.inverse_d(d, o);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const double2 uv = park[r * F::NT];
+      const double f = q == 0 ? park[(8 + r) * F::NT].y : (q == 1 ? park[(16 + r) * F::NT].x : park[(16 + r) * F::NT].y);
+      const double s = o[r].x * uv.x + o[r].y * uv.y;
+      if (q == 0) {
+        luv[r] = make_double2(o[r].x * f, o[r].y * f);
+        lzq[r].y = s;
       } else {
-        X = cscale(SA[scr_off(zb, 4, y, N, g.KXP) + kk], hr);
-        Y = cscale(SA[scr_off(zb, 2, y, N, g.KXP) + kk], -hr);
+        luv[r].x += o[r].x * f;
+        luv[r].y += o[r].y * f;
+        if (q == 1) lbb[r].x = s; else lbb[r].y = s;
       }
-      v = pack_xy(X, Y, k, K, N);
     }
-    bA[(q * RT + rr) * LD + pad_idx(k)] = v;
   }
-  __syncthreads();
-  fft_ip<T, N, false, 7 * RT, NT, LD>(bA, tw);
-  for (int e = tid; e < RT * N; e += NT) {
-    const int x = e % N, rr = e / N;
-    const int px = pad_idx(x);
-    const double2 uv = bA[(0 * RT + rr) * LD + px], zq = bA[(1 * RT + rr) * LD + px];
-    const double2 bb = bA[(2 * RT + rr) * LD + px];
-    const double2 aq = bA[(3 * RT + rr) * LD + px], aR = bA[(4 * RT + rr) * LD + px];
-    const double2 aI = bA[(5 * RT + rr) * LD + px], zz = bA[(6 * RT + rr) * LD + px];
-    const double u = uv.x, v = uv.y, Z = zq.x, Q = zq.y, br = bb.x, bi = bb.y;
-    const double lu = aq.x * Q + aR.x * br + aI.x * bi;
-    const double lv = aq.y * Q + aR.y * br + aI.y * bi;
-    const double lZ = zz.x * br + zz.y * bi;
-    const double lQ = aq.x * u + aq.y * v;
-    const double lBR = aR.x * u + aR.y * v + zz.x * Z;
-    const double lBI = aI.x * u + aI.y * v + zz.y * Z;
-    bA[(0 * RT + rr) * LD + px] = make_double2(lu, lv);
-    bA[(1 * RT + rr) * LD + px] = make_double2(lZ, lQ);
-    bA[(2 * RT + rr) * LD + px] = make_double2(lBR, lBI);
+  {
+    // refraction: (lTI, -lTR)/2
+    double2 d[8], o[8];
+    const double2 *A = sa(4), *B = sa(2);
+    adj_pack<N>(j, K, d, [&](int kk, double2& a, double2& b) { a = cscale(A[kk], hr); b = cscale(B[kk], -hr); });
+    c.inverse_d(d, o);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const double2 bb = park[(16 + r) * F::NT];
+      const double Z = park[(8 + r) * F::NT].x;
+      lzq[r].x = o[r].x * bb.x + o[r].y * bb.y;
+      lbb[r].x += o[r].x * Z;
+      lbb[r].y += o[r].y * Z;
+    }
   }
-  __syncthreads();
-  fft_ip<T, N, true, 3 * RT, NT, LD>(bA, tw);
-  for (int e = tid; e < RT * (K + 1); e += NT) {
-    const int k = e % (K + 1), rr = e / (K + 1);
-    const int y = y0 + rr;
-    double2 lu, lv, lZ, lQ, lBR, lBI;
-    unpack_pad<T>(bA + (0 * RT + rr) * LD, k, N, lu, lv);
-    unpack_pad<T>(bA + (1 * RT + rr) * LD, k, N, lZ, lQ);
-    unpack_pad<T>(bA + (2 * RT + rr) * LD, k, N, lBR, lBI);
+  double2 lv[3];
+  c.forward_d(luv, K, [&](int q, int k, double2 X, double2 Y) { sa(0)[k] = X; lv[q] = Y; });
+  c.forward_d(lzq, K, [&](int q, int k, double2 lZ, double2 lQ) {
     const double kx = (double)k;
-    SA[scr_off(zb, 0, y, N, g.KXP) + k] = lu;
-    SA[scr_off(zb, 1, y, N, g.KXP) + k] = csub(cscale(cmul_mi(lv), kx), cscale(lZ, kx * kx));
-    SA[scr_off(zb, 2, y, N, g.KXP) + k] = lZ;
-    SA[scr_off(zb, 3, y, N, g.KXP) + k] = lQ;
-    SA[scr_off(zb, 4, y, N, g.KXP) + k] = lBR;
-    SA[scr_off(zb, 5, y, N, g.KXP) + k] = lBI;
+    sa(1)[k] = csub(cscale(cmul_mi(lv[q]), kx), cscale(lZ, kx * kx));
+    sa(2)[k] = lZ;
+    sa(3)[k] = lQ;
+  });
+  c.forward_d(lbb, K, [&](int, int k, double2 X, double2 Y) { sa(4)[k] = X; sa(5)[k] = Y; });
+}
+
+// Forward transform of plane P of a column tile times the weight of C^T (2,
+// and 1 with the real part at (0,0)), at the retained rows: use(r, row, ky, m, v)
+template <int N, class Use>
+__device__ __forceinline__ void adj_col_plane(const FxColCtx<N>& c, const Geom& g, const double2* __restrict__ P, int kx,
+                                              Use use) {
+  constexpr int NB = N / 8;
+  double2 d[8];
+  const double2* p = P + (long long)c.j * g.KXP + kx;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) d[r] = kx <= g.K ? p[(long long)r * NB * g.KXP] : make_double2(0.0, 0.0);
+  fxc v[8];
+  int base;
+  c.template run<true>(d, v, base);
+  if (kx > g.K) return;
+  fx_doubles<8, false>(v, d, base);
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    if (fx_zero_in<8>(r)) continue;
+    const int row = g.row_of_fft_index(c.j + r * NB);
+    if (row < 0) continue;
+    const int ky = g.ky_of_row(row);
+    double2 h = make_double2(0.0, 0.0);
+    if (g.mask(kx, ky)) {
+      h = d[r];
+      if (kx == 0 && ky == 0) h.y = 0.0;
+      else h = cscale(h, 2.0);
+    }
+    use(r, (long long)row * g.KXP + kx, ky, h);
   }
 }
 
 template <int N>
-__global__ void __launch_bounds__(kColThreads, Tiles<double, N>::MINB)
+__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(QG_FX_COL_CTAS))
 k_adj_col_fwd(Geom g, AdjP p, int zbase, AdjIn L, AdjOut O, const double* __restrict__ e1t,
               const double* __restrict__ e2t, const double* __restrict__ e1wt, const double* __restrict__ e2wt,
               const double2* __restrict__ SA, const double2* __restrict__ twg) {
-  using T = double;
-  constexpr int CT = Tiles<T, N>::CT, LD = Tiles<T, N>::LD, NT = kColThreads;
+  using F = FxCol<N>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2* tw = reinterpret_cast<double2*>(smem_raw);
-  double2* buf = tw + N;                 // [6][CT][LD]
-  const int tid = threadIdx.x;
-  const int zb = blockIdx.y, z = zbase + zb;
-  const int kx0 = blockIdx.x * CT;
-  load_tw<T, N>(tw, twg, NT);
-#pragma unroll 4
-  for (int e = tid; e < 6 * CT * N; e += NT) {
-    const int c = e % CT, y = (e / CT) % N, h = e / (CT * N);
-    const int kx = kx0 + c;
-    cp_async_c<T>(buf + (h * CT + c) * LD + pad_idx(y), SA + scr_off(zb, h, y, N, g.KXP) + kx, kx <= g.K);
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  fft_ip<T, N, true, 3 * CT, NT, LD>(buf, tw);
-  fft_ip<T, N, true, 3 * CT, NT, LD>(buf + 3 * CT * LD, tw);
-  const long long zoff = (long long)z * g.plane;
-  for (int e = tid; e < CT * g.KY; e += NT) {
-    const int c = e % CT, r = e / CT;
-    const int kx = kx0 + c;
-    if (kx > g.K) continue;
-    const int ky = g.ky_of_row(r);
-    const long long m = zoff + (long long)r * g.KXP + kx, mt = (long long)r * g.KXP + kx;
-    double2 o[6], lpsi = make_double2(0.0, 0.0), lAR = lpsi, lAI = lpsi;
-#pragma unroll
-    for (int f = 0; f < 6; ++f) o[f] = lpsi;
-    if (g.mask(kx, ky)) {
-      const int j = pad_idx(g.fft_index_of_row(r));
-      const bool dc = kx == 0 && ky == 0;
-      const double wt = dc ? 1.0 : 2.0, fky = (double)ky, kh2 = (double)(kx * kx + ky * ky);
-      double2 hv[6];
-#pragma unroll
-      for (int f = 0; f < 6; ++f) {
-        hv[f] = cscale(buf[(f * CT + c) * LD + j], wt);
-        if (dc) hv[f].y = 0.0;
+  __shared__ unsigned slots[F::SLOTS];
+  const FxColCtx<N> c = fx_col_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
+  const int zb = blockIdx.y, kx = blockIdx.x * F::CT + c.c;
+  const long long zoff = (long long)(zbase + zb) * g.plane;
+  auto plane = [&](int f) { return SA + scr_off(zb, f, 0, N, g.KXP); };
+  // psi -> (u, v, zeta) = (-i ky, i kx, -kh^2) psi: transposes i ky, -i kx, -kh^2
+  double2 a[8];
+  adj_col_plane<N>(c, g, plane(0), kx, [&](int r, long long, int ky, double2 h) { a[r] = cscale(cmul_i(h), (double)ky); });
+  adj_col_plane<N>(c, g, plane(1), kx, [&](int r, long long, int, double2 h) { a[r] = cadd(a[r], h); });
+  adj_col_plane<N>(c, g, plane(2), kx, [&](int r, long long mt, int ky, double2 h) {
+    O.lpsi[zoff + mt] = csub(a[r], cscale(h, (double)ky * (double)ky));
+  });
+  for (int w = 0; w < 3; ++w) {
+    adj_col_plane<N>(c, g, plane(3 + w), kx, [&](int, long long mt, int ky, double2 h) {
+      const long long m = zoff + mt;
+      double2 lt = make_double2(0.0, 0.0), on = lt, oo = lt;
+      if (g.mask(kx, ky)) {
+        adj_update(p, L, w, m, w == 0 ? e1t[mt] : e1wt[mt], w == 0 ? e2t[mt] : e2wt[mt], lt, on, oo);
+        on = cadd(on, h);
       }
-      double2 lN, lR, lI;
-      adj_update(p, L, m, e1t[mt], e2t[mt], e1wt[mt], e2wt[mt], o, lN, lR, lI);
-      // psi -> (u, v, zeta) = (-i ky, i kx, -kh^2) psi: transposes i ky, -i kx, -kh^2
-      lpsi = csub(cadd(cscale(cmul_i(hv[0]), fky), hv[1]), cscale(hv[2], fky * fky));
-      o[0] = cadd(o[0], hv[3]);
-      o[2] = cadd(o[2], hv[4]);
-      o[3] = cadd(o[3], hv[5]);
+      O.l[w == 0 ? 0 : 1 + w][m] = on;
+      O.l[w == 0 ? 1 : 3 + w][m] = oo;
       // T_R = N_BR + c kh^2 A_I - r_BI/2, T_I = N_BI - c kh^2 A_R + r_BR/2
-      lAI = cscale(lR, p.cdisp * kh2);
-      lAR = cscale(lI, -p.cdisp * kh2);
-    }
-#pragma unroll
-    for (int f = 0; f < 6; ++f) O.l[f][m] = o[f];
-    O.lpsi[m] = lpsi;
-    O.lAR[m] = lAR;
-    O.lAI[m] = lAI;
+      const double ck = p.cdisp * (double)(kx * kx + ky * ky);
+      if (w == 1) O.lAI[m] = cscale(lt, ck);
+      if (w == 2) O.lAR[m] = cscale(lt, -ck);
+    });
   }
 }
 
 // y-inverse FFTs for the q^w transpose: BR, i ky BR, BI, i ky BI, w', ky^2 w'
 // with w' = w/(2N^2) ((0,0): Re w/N^2), into SF
 template <int N>
-__global__ void __launch_bounds__(kColThreads, Tiles<double, N>::MINB)
+__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(QG_FX_COL_CTAS))
 k_adj_qw_col_inv(Geom g, int zbase, const double2* __restrict__ BR, const double2* __restrict__ BI,
                  const double2* __restrict__ w, double2* __restrict__ SF, const double2* __restrict__ twg) {
-  using T = double;
-  constexpr int CT = Tiles<T, N>::CT, LD = Tiles<T, N>::LD, NT = kColThreads;
+  using F = FxCol<N>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2* tw = reinterpret_cast<double2*>(smem_raw);
-  double2* buf = tw + N;                 // [6][CT][LD]
-  const int tid = threadIdx.x;
-  const int zb = blockIdx.y, z = zbase + zb;
-  const int kx0 = blockIdx.x * CT;
-  load_tw<T, N>(tw, twg, NT);
-  const long long zoff = (long long)z * g.plane;
-#pragma unroll
-  for (int src = 0; src < 3; ++src) {
-    const double2* F = src == 0 ? BR : (src == 1 ? BI : w);
-    double2* slot = buf + 2 * src * CT * LD;
-#pragma unroll 4
-    for (int e = tid; e < CT * N; e += NT) {
-      const int c = e % CT, j = e / CT;
-      const int kx = kx0 + c;
-      const int r = g.row_of_fft_index(j);
-      const bool in = kx <= g.K && r >= 0;
-      cp_async_c<T>(slot + c * LD + pad_idx(j), in ? F + zoff + (long long)r * g.KXP + kx : F, in);
-    }
-  }
-  cp_async_wait_all();
-  __syncthreads();
+  __shared__ unsigned slots[F::SLOTS];
+  const FxColCtx<N> c = fx_col_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
+  const int zb = blockIdx.y, kx = blockIdx.x * F::CT + c.c;
+  const long long zoff = (long long)(zbase + zb) * g.plane;
   const double inv2n2 = 0.5 / ((double)N * (double)N);
-  for (int e = tid; e < CT * N; e += NT) {
-    const int c = e % CT, j = e / CT;
-    const int kx = kx0 + c;
-    const int r = g.row_of_fft_index(j);
-    const int ky = r >= 0 ? g.ky_of_row(r) : 0;
-    const int o = c * LD + pad_idx(j);
-    const double fky = (double)ky;
-    buf[1 * CT * LD + o] = cscale(cmul_i(buf[0 * CT * LD + o]), fky);
-    buf[3 * CT * LD + o] = cscale(cmul_i(buf[2 * CT * LD + o]), fky);
-    const double2 wv = rt_scale(buf[4 * CT * LD + o], kx, ky, inv2n2);
-    buf[4 * CT * LD + o] = wv;
-    buf[5 * CT * LD + o] = cscale(wv, fky * fky);
-  }
-  __syncthreads();
-  if (kx0 == 0) {
-    for (int e = tid; e < 6 * (N / 2 - 1); e += NT) {
-      const int f = e / (N / 2 - 1), j = 1 + e % (N / 2 - 1);
-      double2* col = buf + f * CT * LD;
-      col[pad_idx(N - j)] = cconj(col[pad_idx(j)]);
-    }
-    __syncthreads();
-  }
-  fft_ip<T, N, false, 3 * CT, NT, LD>(buf, tw);
-  fft_ip<T, N, false, 3 * CT, NT, LD>(buf + 3 * CT * LD, tw);
-#pragma unroll 4
-  for (int e = tid; e < 6 * CT * N; e += NT) {
-    const int c = e % CT, y = (e / CT) % N, f = e / (CT * N);
-    SF[scr_off(zb, f, y, N, g.KXP) + kx0 + c] = buf[(f * CT + c) * LD + pad_idx(y)];
+  for (int f = 0; f < 6; ++f) {
+    const double2* X = f < 2 ? BR : (f < 4 ? BI : w);
+    adj_col_inverse<N>(c, g, kx, SF + scr_off(zb, f, 0, N, g.KXP), [&](int row, int ky) {
+      double2 x = X[zoff + (long long)row * g.KXP + kx];
+      const double fky = (double)ky;
+      if (f >= 4) x = rt_scale(x, kx, ky, inv2n2);
+      return f == 5 ? cscale(x, fky * fky) : ((f & 1) ? cscale(cmul_i(x), fky) : x);
+    });
   }
 }
 
@@ -438,123 +397,95 @@ k_adj_qw_col_inv(Geom g, int zbase, const double2* __restrict__ BR, const double
 // q^w = s R(P1) - s kh^2/4 R(P2); writes (G_R, H_R, G_I, H_I) with
 // lB = w_k [F_y(G) - i ky F_y(H)], G = -i kx F_x(a) + F_x(c), H = F_x(b)
 template <int N>
-__global__ void __launch_bounds__(kThreadsB)
+__global__ void __launch_bounds__(FxRow<N>::NT, fx_row_ctas<N>(QG_FX_ROW_CTAS))
 k_adj_qw_row(Geom g, AdjP p, double2* __restrict__ SF, const double2* __restrict__ twg) {
-  using T = double;
-  constexpr int RT = Tiles<T, N>::RT, LD = Tiles<T, N>::LD, NT = kThreadsB;
+  using F = FxRow<N>;
+  constexpr int NB = F::NB;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2* tw = reinterpret_cast<double2*>(smem_raw);
-  double2* bA = tw + N;                 // [4][RT][LD]
-  const int tid = threadIdx.x;
-  const int zb = blockIdx.y;
-  const int y0 = blockIdx.x * RT;
-  const int K = g.K;
-  load_tw<T, N>(tw, twg, NT);
+  __shared__ unsigned slots[F::SLOTS];
+  FxRowCtx<N> c = fx_row_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
+  const int zb = blockIdx.y, y = blockIdx.x * F::RT + c.rr, K = g.K, j = c.j;
+  auto sf = [&](int f) { return SF + scr_off(zb, f, y, N, g.KXP); };
   const double s = p.s;
-  for (int e = tid; e < 4 * RT * N; e += NT) {
-    const int k = e % N, rr = (e / N) % RT, q = e / (RT * N);
-    const int y = y0 + rr;
-    const int kk = k <= K ? k : N - k;
-    double2 v = make_double2(0.0, 0.0);
-    if (k <= K || k >= N - K) {
-      const double fk = (double)kk;
-      double2 X, Y;
-      if (q == 0) {
-        X = SF[scr_off(zb, 0, y, N, g.KXP) + kk]; Y = SF[scr_off(zb, 2, y, N, g.KXP) + kk];
-      } else if (q == 1) {
-        X = cscale(cmul_i(SF[scr_off(zb, 0, y, N, g.KXP) + kk]), fk);
-        Y = cscale(cmul_i(SF[scr_off(zb, 2, y, N, g.KXP) + kk]), fk);
-      } else if (q == 2) {
-        X = SF[scr_off(zb, 1, y, N, g.KXP) + kk]; Y = SF[scr_off(zb, 3, y, N, g.KXP) + kk];
-      } else {
-        const double2 w1 = SF[scr_off(zb, 4, y, N, g.KXP) + kk], w2 = SF[scr_off(zb, 5, y, N, g.KXP) + kk];
-        X = cscale(w1, -s);
-        Y = cscale(cadd(cscale(w1, fk * fk), w2), 0.25 * s);
-      }
-      v = pack_xy(X, Y, k, K, N);
-    }
-    bA[(q * RT + rr) * LD + pad_idx(k)] = v;
+  fxc l[8], b[8], v[8];
+  int el, eb;
+  double2 d[8];
+  {
+    const double2 *W1 = sf(4), *W2 = sf(5);
+    adj_pack<N>(j, K, d, [&](int kk, double2& X, double2& Y) {
+      const double2 w1 = W1[kk], w2 = W2[kk];
+      X = cscale(w1, -s);
+      Y = cscale(cadd(cscale(w1, (double)kk * (double)kk), w2), 0.25 * s);
+    });
+    c.inverse(d, l, el);           // l.y: lP1, l.x: lP2
   }
-  __syncthreads();
-  fft_ip<T, N, false, 4 * RT, NT, LD>(bA, tw);
-  for (int e = tid; e < RT * N; e += NT) {
-    const int x = e % N, rr = e / N;
-    const int px = pad_idx(x);
-    const double2 b = bA[(0 * RT + rr) * LD + px], bx = bA[(1 * RT + rr) * LD + px];
-    const double2 by = bA[(2 * RT + rr) * LD + px], lp = bA[(3 * RT + rr) * LD + px];
-    const double l1 = lp.x, l2 = lp.y;
-    bA[(0 * RT + rr) * LD + px] = make_double2(-l1 * by.y, l1 * by.x);          // a_R, a_I
-    bA[(1 * RT + rr) * LD + px] = make_double2(l1 * bx.y, -l1 * bx.x);          // b_R, b_I
-    bA[(2 * RT + rr) * LD + px] = make_double2(2.0 * b.x * l2, 2.0 * b.y * l2); // c_R, c_I
+  // (a_R, a_I) = lP1 (-BIy, BRy)
+  fx_pack<N>(sf(1), sf(3), j, K, d);
+  c.inverse(d, b, eb);
+#pragma unroll
+  for (int r = 0; r < 8; ++r) { v[r].x = -fx_mulhi(l[r].y, b[r].x); v[r].y = fx_mulhi(l[r].y, b[r].y); }
+  double2 aR[3], aI[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) aR[q] = aI[q] = make_double2(0.0, 0.0);
+  c.forward(v, el + eb - 1023 + 64, K, [&](int q, int, double2 X, double2 Y) { aR[q] = X; aI[q] = Y; });
+  // (b_R, b_I) = lP1 (BIx, -BRx)
+  fx_pack<N>(sf(0), sf(2), j, K, d);
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const double k = (double)(j + r * NB - (r < 4 ? 0 : N));
+    d[r] = make_double2(-k * d[r].y, k * d[r].x);
   }
-  __syncthreads();
-  fft_ip<T, N, true, 3 * RT, NT, LD>(bA, tw);
-  for (int e = tid; e < RT * (K + 1); e += NT) {
-    const int k = e % (K + 1), rr = e / (K + 1);
-    const int y = y0 + rr;
-    double2 aR, aI, bR, bI, cR, cI;
-    unpack_pad<T>(bA + (0 * RT + rr) * LD, k, N, aR, aI);
-    unpack_pad<T>(bA + (1 * RT + rr) * LD, k, N, bR, bI);
-    unpack_pad<T>(bA + (2 * RT + rr) * LD, k, N, cR, cI);
+  c.inverse(d, b, eb);
+#pragma unroll
+  for (int r = 0; r < 8; ++r) { v[r].x = fx_mulhi(l[r].y, b[r].x); v[r].y = -fx_mulhi(l[r].y, b[r].y); }
+  c.forward(v, el + eb - 1023 + 64, K, [&](int, int k, double2 X, double2 Y) { sf(1)[k] = X; sf(3)[k] = Y; });
+  // (c_R, c_I) = 2 lP2 (BR, BI)
+  fx_pack<N>(sf(0), sf(2), j, K, d);
+  c.inverse(d, b, eb);
+#pragma unroll
+  for (int r = 0; r < 8; ++r) { v[r].x = fx_mulhi(l[r].x, b[r].y); v[r].y = fx_mulhi(l[r].x, b[r].x); }
+  c.forward(v, el + eb - 1023 + 64 + 1, K, [&](int q, int k, double2 X, double2 Y) {
     const double kx = (double)k;
-    SF[scr_off(zb, 0, y, N, g.KXP) + k] = cadd(cscale(cmul_mi(aR), kx), cR);
-    SF[scr_off(zb, 1, y, N, g.KXP) + k] = bR;
-    SF[scr_off(zb, 2, y, N, g.KXP) + k] = cadd(cscale(cmul_mi(aI), kx), cI);
-    SF[scr_off(zb, 3, y, N, g.KXP) + k] = bI;
-  }
+    sf(0)[k] = cadd(cscale(cmul_mi(aR[q]), kx), X);
+    sf(2)[k] = cadd(cscale(cmul_mi(aI[q]), kx), Y);
+  });
 }
 
 // final adds: lq += w, lB += A_solver(lA) (+ q^w transpose when with_qw)
 template <int N>
-__global__ void __launch_bounds__(kColThreads, Tiles<double, N>::MINB)
-k_adj_qw_col_fwd(Geom g, int zbase, int with_qw, double2* __restrict__ lq, double2* __restrict__ lBR,
-                 double2* __restrict__ lBI, const double2* __restrict__ w, const double2* __restrict__ lBRa,
-                 const double2* __restrict__ lBIa, const double2* __restrict__ SF, const double2* __restrict__ twg) {
-  using T = double;
-  constexpr int CT = Tiles<T, N>::CT, LD = Tiles<T, N>::LD, NT = kColThreads;
+__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(QG_FX_COL_CTAS))
+k_adj_qw_col_fwd(Geom g, int zbase, double2* __restrict__ lBR, double2* __restrict__ lBI, const double2* __restrict__ SF,
+                 const double2* __restrict__ twg) {
+  using F = FxCol<N>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2* tw = reinterpret_cast<double2*>(smem_raw);
-  double2* buf = tw + N;                 // [4][CT][LD]
-  const int tid = threadIdx.x;
-  const int zb = blockIdx.y, z = zbase + zb;
-  const int kx0 = blockIdx.x * CT;
-  if (with_qw) {
-    load_tw<T, N>(tw, twg, NT);
-#pragma unroll 4
-    for (int e = tid; e < 4 * CT * N; e += NT) {
-      const int c = e % CT, y = (e / CT) % N, h = e / (CT * N);
-      const int kx = kx0 + c;
-      cp_async_c<T>(buf + (h * CT + c) * LD + pad_idx(y), SF + scr_off(zb, h, y, N, g.KXP) + kx, kx <= g.K);
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    fft_ip<T, N, true, 4 * CT, NT, LD>(buf, tw);
+  __shared__ unsigned slots[F::SLOTS];
+  const FxColCtx<N> c = fx_col_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
+  const int zb = blockIdx.y, kx = blockIdx.x * F::CT + c.c;
+  const long long zoff = (long long)(zbase + zb) * g.plane;
+  for (int b = 0; b < 2; ++b) {
+    double2* lB = b == 0 ? lBR : lBI;
+    double2 a[8];
+    adj_col_plane<N>(c, g, SF + scr_off(zb, 2 * b, 0, N, g.KXP), kx, [&](int r, long long, int, double2 h) { a[r] = h; });
+    adj_col_plane<N>(c, g, SF + scr_off(zb, 2 * b + 1, 0, N, g.KXP), kx, [&](int r, long long mt, int ky, double2 h) {
+      double2* o = lB + zoff + mt;
+      // (a(0,0) is real; ky = 0 there, so the second term vanishes)
+      *o = cadd(*o, csub(a[r], cscale(cmul_i(h), (double)ky)));
+    });
   }
-  const long long zoff = (long long)z * g.plane;
-  for (int e = tid; e < CT * g.KY; e += NT) {
-    const int c = e % CT, r = e / CT;
-    const int kx = kx0 + c;
-    if (kx > g.K) continue;
-    const int ky = g.ky_of_row(r);
-    const long long m = zoff + (long long)r * g.KXP + kx;
-    double2 oq = make_double2(0.0, 0.0), oR = oq, oI = oq;
-    if (g.mask(kx, ky)) {
-      oq = cadd(lq[m], w[m]);
-      oR = cadd(lBR[m], lBRa[m]);
-      oI = cadd(lBI[m], lBIa[m]);
-      if (with_qw) {
-        const int j = pad_idx(g.fft_index_of_row(r));
-        const bool dc = kx == 0 && ky == 0;
-        const double wt = dc ? 1.0 : 2.0, fky = (double)ky;
-        double2 dR = csub(buf[(0 * CT + c) * LD + j], cscale(cmul_i(buf[(1 * CT + c) * LD + j]), fky));
-        double2 dI = csub(buf[(2 * CT + c) * LD + j], cscale(cmul_i(buf[(3 * CT + c) * LD + j]), fky));
-        dR = cscale(dR, wt); dI = cscale(dI, wt);
-        if (dc) { dR.y = 0.0; dI.y = 0.0; }
-        oR = cadd(oR, dR);
-        oI = cadd(oI, dI);
-      }
-    }
-    lq[m] = oq; lBR[m] = oR; lBI[m] = oI;
+}
+
+// lq += w, lB += A_solver(lA) on the compact layout (zeros off the retained modes)
+static __global__ void k_adj_solved(Geom g, long long tot, double2* __restrict__ lq, double2* __restrict__ lBR,
+                                    double2* __restrict__ lBI, const double2* __restrict__ w,
+                                    const double2* __restrict__ lBRa, const double2* __restrict__ lBIa) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot; i += (long long)gridDim.x * blockDim.x) {
+    const long long mm = i % g.plane;
+    const int r = (int)(mm / g.KXP), kx = (int)(mm % g.KXP);
+    const bool in = g.mask(kx, g.ky_of_row(r));
+    const double2 z = make_double2(0.0, 0.0);
+    lq[i] = in ? cadd(lq[i], w[i]) : z;
+    lBR[i] = in ? cadd(lBR[i], lBRa[i]) : z;
+    lBI[i] = in ? cadd(lBI[i], lBIa[i]) : z;
   }
 }
 

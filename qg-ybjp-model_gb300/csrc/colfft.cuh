@@ -287,6 +287,40 @@ __device__ __forceinline__ void ip_passes_but_last(cplx<T>* buf, const cplx<T>* 
   }
 }
 
+// Row transforms with the first pass fed from registers and the last pass
+// handed back in registers, NF*RT transforms (f*RT + rr) of LD entries:
+// pro(rr, j, v) fills v[f][r] with the input at j + r N/R0, epi(rr, j, v)
+// gets the output at j + r NS_last.  NT = RT * N/R0 threads.
+template <typename T, int N, bool FWD, int NF, int RT, int NT, int LD, class Pro, class Epi>
+__device__ __forceinline__ void row_fft(cplx<T>* __restrict__ sm, const cplx<T>* __restrict__ tw, Pro pro, Epi epi) {
+  constexpr int R0 = radix_of(N), NS = LastNS<N>::value;
+  row_pass0<T, N, FWD, NF, RT, NT, LD>(sm, pro);
+  __syncthreads();
+  ip_passes_but_last<T, N, FWD, NF * RT, NT, LD, R0>(sm, tw);
+  constexpr int R = N / NS, TASKS = RT * NS, PER = (TASKS + NT - 1) / NT, off = tw_off<N>(NS);
+#pragma unroll
+  for (int p = 0; p < PER; ++p) {
+    const int t = threadIdx.x + p * NT;
+    if ((TASKS % NT) == 0 || t < TASKS) {
+      const int j = t % NS, rr = t / NS;
+      cplx<T> v[NF][R];
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[f][r] = sm[(f * RT + rr) * LD + pad_idx(j + r * NS)];
+#pragma unroll
+        for (int r = 1; r < R; ++r) {
+          cplx<T> w = tw[off + (r - 1) * NS + j];
+          if (!FWD) w.y = -w.y;
+          v[f][r] = cmul(v[f][r], w);
+        }
+        dftR<T, R, FWD>(v[f]);
+      }
+      epi(rr, j, v);
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Forward row transforms of N = 512 (radices 8 x 8 x 8) ending in registers.
 //

@@ -4,34 +4,74 @@
 // the Fortran routines give.
 #pragma once
 #include "step_kernels.cuh"
+#include "fxctx.cuh"
 
 namespace qg {
 
 // dense spectral: double2 [nz][n][iktx]; W: cplx<T> [nz][n(y)][iktxP]; phys: T [nz][n][n]
 
+// Column tiles of CT columns, rows in pairs (one packed complex transform
+// each), RT pairs per CTA with one first-pass butterfly per thread; doubles
+// on the block fixed-point contexts (fxctx.cuh).
+template <typename T, int N> struct Dense {
+  static constexpr bool FX = sizeof(T) == 8;
+  static constexpr int CT = FX ? FxCol<N>::CT : Tiles<T, N>::CT, CNT = FX ? FxCol<N>::NT : Tiles<T, N>::CNT;
+  static constexpr int NB = FX ? N / 8 : N / radix_of(N);
+  static constexpr int RT = FX ? imin(FxRow<N>::RT, N / 2) : imin(N / 2, imax(1, 256 / NB));
+  static constexpr int RNT = FX ? FxRow<N>::NT : RT * NB;
+  static constexpr int LD = FX ? FxRow<N>::LD : PadLD<N>::value;
+  static constexpr size_t sm_col() { return FX ? FxCol<N>::smem() : (size_t)(N + ColLay<N, CT>::FS) * sizeof(cplx<T>); }
+  static constexpr size_t sm_row() { return FX ? FxRow<N>::smem() : (size_t)(N + RT * LD) * sizeof(cplx<T>); }
+};
+// row length of the (kx, y) intermediate: whole column tiles of every n
+__host__ __device__ constexpr int dense_kxp(int n) { return n < 32 ? 16 : (n / 2 + 1 + 7) / 8 * 8; }
+
+// realit (fft.f90:88-107): the kx = 0 entries of negative ky are the
+// conjugates of the positive ones
 template <typename T, int N>
-__global__ void __launch_bounds__(kThreads)
+__device__ __forceinline__ cplx<T> dense_in(const double2* __restrict__ in, long long z, int i, int kx) {
+  constexpr int IKTX = N / 2 + 1;
+  const bool cj = kx == 0 && i > N / 2;
+  if (kx >= IKTX) return mk<T>(0, 0);
+  const double2 d = in[(z * N + (cj ? N - i : i)) * IKTX + kx];
+  return mk<T>((T)d.x, cj ? -(T)d.y : (T)d.y);
+}
+
+template <typename T, int N>
+__global__ void __launch_bounds__(Dense<T, N>::CNT)
 k_dcol_inv(int iktxP, const double2* __restrict__ in, cplx<T>* __restrict__ W, const cplx<T>* __restrict__ twg) {
-  constexpr int CT = Tile<T>::CT, LD = N + 1, IKTX = N / 2 + 1;
+  constexpr int CT = Dense<T, N>::CT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* tw = reinterpret_cast<cplx<T>*>(smem_raw);
-  cplx<T>* bufA = tw + N;
-  cplx<T>* bufB = bufA + CT * LD;
   const int z = blockIdx.y, kx0 = blockIdx.x * CT;
-  load_twiddles<T, N>(tw, twg);
-  for (int idx = threadIdx.x; idx < CT * N; idx += blockDim.x) {
-    const int c = idx % CT, j = idx / CT, kx = kx0 + c;
-    cplx<T> v = mk<T>(0, 0);
-    if (kx < IKTX) { const double2 d = in[((long long)z * N + j) * IKTX + kx]; v = mk<T>((T)d.x, (T)d.y); }
-    bufA[c * LD + j] = v;
-  }
-  __syncthreads();
-  if (kx0 == 0) realit_col<T>(bufA, N);
-  __syncthreads();
-  cplx<T>* res = block_fft<T, N, false>(bufA, bufB, LD, CT, tw);
-  for (int idx = threadIdx.x; idx < CT * N; idx += blockDim.x) {
-    const int c = idx % CT, y = idx / CT;
-    W[((long long)z * N + y) * iktxP + kx0 + c] = res[c * LD + y];
+  if constexpr (Dense<T, N>::FX) {
+    constexpr int NB = N / 8;
+    __shared__ unsigned slots[FxCol<N>::SLOTS];
+    const FxColCtx<N> c = fx_col_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
+    const int kx = kx0 + c.c;
+    double2 d[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) d[r] = dense_in<T, N>(in, z, c.j + r * NB, kx);
+    fxc v[8];
+    int base;
+    c.template run<false, false>(d, v, base);
+    fx_doubles<8, true>(v, d, base);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) W[((long long)z * N + c.j + r * NB) * iktxP + kx] = d[r];
+  } else {
+    constexpr int NT = Dense<T, N>::CNT, R0 = radix_of(N), NB0 = N / R0, NSL = LastNS<N>::value, RL = N / NSL;
+    cplx<T>* tw = reinterpret_cast<cplx<T>*>(smem_raw);
+    cplx<T>* sm = tw + N;
+    load_tw<T, N>(tw, twg, NT);
+    auto pro = [&](int c, int j, cplx<T> (&v)[1][R0]) {
+#pragma unroll
+      for (int r = 0; r < R0; ++r) v[0][r] = dense_in<T, N>(in, z, j + r * NB0, kx0 + c);
+    };
+    auto epi = [&](int c, int j, cplx<T> (&v)[1][RL]) {
+#pragma unroll
+      for (int r = 0; r < RL; ++r) W[((long long)z * N + j + r * NSL) * iktxP + kx0 + c] = v[0][r];
+    };
+    __syncthreads();
+    col_fft<T, N, false, 1, CT, NT>(sm, tw, pro, epi);
   }
 }
 
@@ -44,94 +84,175 @@ __device__ __forceinline__ cplx<T> pack_full(const cplx<T>* X, const cplx<T>* Y,
   const int kk = n - k; cplx<T> a = X[kk], b = Y[kk]; return mk<T>(a.x + b.y, b.x - a.y);
 }
 
+// one CTA: RT pairs of rows of level z; put(y, x, value) stores the outputs
+template <typename T, int N, class Put>
+__device__ __forceinline__ void drow_c2r(int iktxP, const cplx<T>* __restrict__ W, const cplx<T>* __restrict__ twg,
+                                         unsigned char* smem_raw, int z, int p0, Put put) {
+  using D = Dense<T, N>;
+  if constexpr (D::FX) {
+    constexpr int NB = N / 8;
+    __shared__ unsigned slots[FxRow<N>::SLOTS];
+    FxRowCtx<N> c = fx_row_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
+    const bool live = c.rr < D::RT;
+    const int y = 2 * (p0 + c.rr);
+    const double2* X = W + ((long long)z * N + y) * iktxP;
+    double2 d[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) d[r] = live ? pack_full<T>(X, X + iktxP, c.j + r * NB, N) : make_double2(0.0, 0.0);
+    fxc v[8];
+    int base = fx_ints<8, false, false>(d, v, c.template reduce<false>(fx_maxp<8, false>(d)));
+    c.core(v, base);
+    if (!live) return;
+    fx_doubles<8, true>(v, d, base);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      put(y, c.j + r * NB, d[r].x);
+      put(y + 1, c.j + r * NB, d[r].y);
+    }
+  } else {
+    constexpr int R0 = radix_of(N), NB0 = N / R0, NSL = LastNS<N>::value, RL = N / NSL;
+    cplx<T>* tw = reinterpret_cast<cplx<T>*>(smem_raw);
+    cplx<T>* sm = tw + N;
+    load_tw<T, N>(tw, twg, D::RNT);
+    auto pro = [&](int rr, int j, cplx<T> (&v)[1][R0]) {
+      const cplx<T>* X = W + ((long long)z * N + 2 * (p0 + rr)) * iktxP;
+#pragma unroll
+      for (int r = 0; r < R0; ++r) v[0][r] = pack_full<T>(X, X + iktxP, j + r * NB0, N);
+    };
+    auto epi = [&](int rr, int j, cplx<T> (&v)[1][RL]) {
+#pragma unroll
+      for (int r = 0; r < RL; ++r) {
+        put(2 * (p0 + rr), j + r * NSL, v[0][r].x);
+        put(2 * (p0 + rr) + 1, j + r * NSL, v[0][r].y);
+      }
+    };
+    __syncthreads();
+    row_fft<T, N, false, 1, D::RT, D::RNT, D::LD>(sm, tw, pro, epi);
+  }
+}
+
 template <typename T, int N>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(Dense<T, N>::RNT)
 k_drow_c2r(int iktxP, const cplx<T>* __restrict__ W, T* __restrict__ phys, const cplx<T>* __restrict__ twg) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* tw = reinterpret_cast<cplx<T>*>(smem_raw);
-  cplx<T>* bA = tw + N;
-  cplx<T>* bB = bA + N;
-  const int z = blockIdx.y, y0 = 2 * blockIdx.x;
-  load_twiddles<T, N>(tw, twg);
-  const cplx<T>* X = W + ((long long)z * N + y0) * iktxP;
-  const cplx<T>* Y = X + iktxP;
-  for (int k = threadIdx.x; k < N; k += blockDim.x) bA[k] = pack_full<T>(X, Y, k, N);
-  __syncthreads();
-  cplx<T>* res = block_fft<T, N, false>(bA, bB, N, 1, tw);
-  for (int x = threadIdx.x; x < N; x += blockDim.x) {
-    phys[((long long)z * N + y0) * N + x] = res[x].x;
-    phys[((long long)z * N + y0 + 1) * N + x] = res[x].y;
-  }
+  const int z = blockIdx.y;
+  T* o = phys + (long long)z * N * N;
+  drow_c2r<T, N>(iktxP, W, twg, smem_raw, z, blockIdx.x * Dense<T, N>::RT, [&](int y, int x, T v) { o[y * N + x] = v; });
 }
 
 // Same transform as k_drow_c2r, written straight into the reference's padded
 // physical layout double[nz][N][N+2] (the two padding values of a row are 0).
 template <typename T, int N>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(Dense<T, N>::RNT)
 k_drow_c2r_pad(int iktxP, const cplx<T>* __restrict__ W, double* __restrict__ out, const cplx<T>* __restrict__ twg) {
+  using D = Dense<T, N>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* tw = reinterpret_cast<cplx<T>*>(smem_raw);
-  cplx<T>* bA = tw + N;
-  cplx<T>* bB = bA + N;
-  const int z = blockIdx.y, y0 = 2 * blockIdx.x;
-  load_twiddles<T, N>(tw, twg);
-  const cplx<T>* X = W + ((long long)z * N + y0) * iktxP;
-  const cplx<T>* Y = X + iktxP;
-  for (int k = threadIdx.x; k < N; k += blockDim.x) bA[k] = pack_full<T>(X, Y, k, N);
-  __syncthreads();
-  cplx<T>* res = block_fft<T, N, false>(bA, bB, N, 1, tw);
-  double* r0 = out + ((long long)z * N + y0) * (N + 2);
-  double* r1 = r0 + (N + 2);
-  for (int x = threadIdx.x; x < N + 2; x += blockDim.x) {
-    r0[x] = x < N ? (double)res[x].x : 0.0;
-    r1[x] = x < N ? (double)res[x].y : 0.0;
-  }
+  const int z = blockIdx.y, p0 = blockIdx.x * D::RT;
+  double* o = out + (long long)z * N * (N + 2);
+  for (int e = threadIdx.x; e < 4 * D::RT; e += D::RNT) o[(2 * p0 + e / 2) * (N + 2) + N + e % 2] = 0.0;
+  drow_c2r<T, N>(iktxP, W, twg, smem_raw, z, p0, [&](int y, int x, T v) { o[y * (N + 2) + x] = (double)v; });
 }
 
 template <typename T, int N>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(Dense<T, N>::RNT)
 k_drow_r2c(int iktxP, const T* __restrict__ phys, cplx<T>* __restrict__ W, const cplx<T>* __restrict__ twg) {
+  using D = Dense<T, N>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* tw = reinterpret_cast<cplx<T>*>(smem_raw);
-  cplx<T>* bA = tw + N;
-  cplx<T>* bB = bA + N;
-  const int z = blockIdx.y, y0 = 2 * blockIdx.x;
-  load_twiddles<T, N>(tw, twg);
-  for (int x = threadIdx.x; x < N; x += blockDim.x)
-    bA[x] = mk<T>(phys[((long long)z * N + y0) * N + x], phys[((long long)z * N + y0 + 1) * N + x]);
-  __syncthreads();
-  cplx<T>* F = block_fft<T, N, true>(bA, bB, N, 1, tw);
-  for (int k = threadIdx.x; k <= N / 2; k += blockDim.x) {
-    cplx<T> a, b;
-    unpack_spec<T>(F, k, N, a, b);
-    W[((long long)z * N + y0) * iktxP + k] = a;
-    W[((long long)z * N + y0 + 1) * iktxP + k] = b;
+  const int z = blockIdx.y, p0 = blockIdx.x * D::RT;
+  if constexpr (D::FX) {
+    constexpr int NB = N / 8;
+    __shared__ unsigned slots[FxRow<N>::SLOTS];
+    FxRowCtx<N> c = fx_row_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
+    const bool live = c.rr < D::RT;
+    const long long y = (long long)z * N + 2 * (p0 + c.rr);
+    double2 d[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const T* a = phys + y * N + c.j + r * NB;
+      d[r] = live ? make_double2(a[0], a[N]) : make_double2(0.0, 0.0);
+    }
+    fxc v[8];
+    int base = fx_ints<8, true, false>(d, v, c.template reduce<false>(fx_maxp<8, false>(d)));
+    c.core(v, base);
+    double2* o = W + y * iktxP;
+    c.template split<5>(v, base, N / 2, [&](int, int k, double2 X, double2 Y) {
+      if (!live) return;
+      o[k] = X;
+      o[iktxP + k] = Y;
+    });
+  } else {
+    constexpr int R0 = radix_of(N), NB0 = N / R0, NSL = LastNS<N>::value, RL = N / NSL;
+    cplx<T>* tw = reinterpret_cast<cplx<T>*>(smem_raw);
+    cplx<T>* sm = tw + N;
+    load_tw<T, N>(tw, twg, D::RNT);
+    const T* a = phys + (long long)z * N * N;
+    auto pro = [&](int rr, int j, cplx<T> (&v)[1][R0]) {
+      const T* p = a + 2 * (p0 + rr) * N + j;
+#pragma unroll
+      for (int r = 0; r < R0; ++r) v[0][r] = mk<T>(p[r * NB0], p[N + r * NB0]);
+    };
+    // a row's last-pass tasks write back the entries they alone have read
+    auto epi = [&](int rr, int j, cplx<T> (&v)[1][RL]) {
+#pragma unroll
+      for (int r = 0; r < RL; ++r) sm[rr * D::LD + pad_idx(j + r * NSL)] = v[0][r];
+    };
+    __syncthreads();
+    row_fft<T, N, true, 1, D::RT, D::RNT, D::LD>(sm, tw, pro, epi);
+    __syncthreads();
+    for (int e = threadIdx.x; e < D::RT * (N / 2 + 1); e += D::RNT) {
+      const int k = e % (N / 2 + 1), rr = e / (N / 2 + 1);
+      cplx<T> x, y;
+      unpack_pad<T>(sm + rr * D::LD, k, N, x, y);
+      cplx<T>* o = W + ((long long)z * N + 2 * (p0 + rr)) * iktxP + k;
+      o[0] = x;
+      o[iktxP] = y;
+    }
   }
 }
 
 template <typename T, int N>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(Dense<T, N>::CNT)
 k_dcol_fwd(int iktxP, const cplx<T>* __restrict__ W, double2* __restrict__ out, const cplx<T>* __restrict__ twg) {
-  constexpr int CT = Tile<T>::CT, LD = N + 1, IKTX = N / 2 + 1;
+  constexpr int CT = Dense<T, N>::CT, IKTX = N / 2 + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* tw = reinterpret_cast<cplx<T>*>(smem_raw);
-  cplx<T>* bufA = tw + N;
-  cplx<T>* bufB = bufA + CT * LD;
   const int z = blockIdx.y, kx0 = blockIdx.x * CT;
-  load_twiddles<T, N>(tw, twg);
-  for (int idx = threadIdx.x; idx < CT * N; idx += blockDim.x) {
-    const int c = idx % CT, y = idx / CT;
-    bufA[c * LD + y] = W[((long long)z * N + y) * iktxP + kx0 + c];
-  }
-  __syncthreads();
-  cplx<T>* res = block_fft<T, N, true>(bufA, bufB, LD, CT, tw);
-  const double s = 1.0 / ((double)N * (double)N);
-  for (int idx = threadIdx.x; idx < CT * N; idx += blockDim.x) {
-    const int c = idx % CT, j = idx / CT, kx = kx0 + c;
-    if (kx < IKTX) {
-      const cplx<T> v = res[c * LD + j];
-      out[((long long)z * N + j) * IKTX + kx] = make_double2((double)v.x * s, (double)v.y * s);
-    }
+  // the columns past the spectrum are not written by the row kernels
+  auto get = [&](int y, int kx) { return kx < IKTX ? W[((long long)z * N + y) * iktxP + kx] : mk<T>(0, 0); };
+  if constexpr (Dense<T, N>::FX) {
+    constexpr int NB = N / 8;
+    __shared__ unsigned slots[FxCol<N>::SLOTS];
+    const FxColCtx<N> c = fx_col_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
+    const int kx = kx0 + c.c;
+    double2 d[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) d[r] = get(c.j + r * NB, kx);
+    fxc v[8];
+    int base;
+    c.template run<true, false>(d, v, base);
+    base -= 2 * fx_ilog2(N);               // divided by n^2
+    if (kx >= IKTX) return;
+    fx_doubles<8, false>(v, d, base);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) out[((long long)z * N + c.j + r * NB) * IKTX + kx] = d[r];
+  } else {
+    constexpr int NT = Dense<T, N>::CNT, R0 = radix_of(N), NB0 = N / R0, NSL = LastNS<N>::value, RL = N / NSL;
+    cplx<T>* tw = reinterpret_cast<cplx<T>*>(smem_raw);
+    cplx<T>* sm = tw + N;
+    load_tw<T, N>(tw, twg, NT);
+    auto pro = [&](int c, int j, cplx<T> (&v)[1][R0]) {
+#pragma unroll
+      for (int r = 0; r < R0; ++r) v[0][r] = get(j + r * NB0, kx0 + c);
+    };
+    const double s = 1.0 / ((double)N * (double)N);
+    auto epi = [&](int c, int j, cplx<T> (&v)[1][RL]) {
+      const int kx = kx0 + c;
+      if (kx >= IKTX) return;
+#pragma unroll
+      for (int r = 0; r < RL; ++r)
+        out[((long long)z * N + j + r * NSL) * IKTX + kx] = make_double2((double)v[0][r].x * s, (double)v[0][r].y * s);
+    };
+    __syncthreads();
+    col_fft<T, N, true, 1, CT, NT>(sm, tw, pro, epi);
   }
 }
 

@@ -179,10 +179,6 @@ class AdjEngine final : public Engine<double> {
     return v;
   }
 
-  template <int NN> static constexpr size_t sm_col4() {
-    return (size_t)(NN + 4 * Tiles<double, NN>::CT * Tiles<double, NN>::LD) * sizeof(C);
-  }
-
   int ensure_adj() {
     if (ready) return QG_OK;
     // the transposes use psi_solver and A_solver as self-adjoint (rho = 1)
@@ -215,12 +211,13 @@ class AdjEngine final : public Engine<double> {
     part_h.assign(kObjBlocks, 0.0);
     const int mx = cudaFuncAttributeMaxDynamicSharedMemorySize;
     QG_SWITCH_N(g.n, {
-      QG_CK(cudaFuncSetAttribute(k_adj_col_inv<NN>, (cudaFuncAttribute)mx, (int)sm_col6<NN>()));
-      QG_CK(cudaFuncSetAttribute(k_adj_row<NN>, (cudaFuncAttribute)mx, (int)sm_row7<NN>()));
-      QG_CK(cudaFuncSetAttribute(k_adj_col_fwd<NN>, (cudaFuncAttribute)mx, (int)sm_col6<NN>()));
-      QG_CK(cudaFuncSetAttribute(k_adj_qw_col_inv<NN>, (cudaFuncAttribute)mx, (int)sm_col6<NN>()));
-      QG_CK(cudaFuncSetAttribute(k_adj_qw_row<NN>, (cudaFuncAttribute)mx, (int)sm_row4<NN>()));
-      QG_CK(cudaFuncSetAttribute(k_adj_qw_col_fwd<NN>, (cudaFuncAttribute)mx, (int)sm_col4<NN>()));
+      const int sc = (int)FxCol<NN>::smem(), sr = (int)FxRow<NN>::smem();
+      QG_CK(cudaFuncSetAttribute(k_adj_col_inv<NN>, (cudaFuncAttribute)mx, sc));
+      QG_CK(cudaFuncSetAttribute(k_adj_row<NN>, (cudaFuncAttribute)mx, (int)AdjRow<NN>::smem()));
+      QG_CK(cudaFuncSetAttribute(k_adj_col_fwd<NN>, (cudaFuncAttribute)mx, sc));
+      QG_CK(cudaFuncSetAttribute(k_adj_qw_col_inv<NN>, (cudaFuncAttribute)mx, sc));
+      QG_CK(cudaFuncSetAttribute(k_adj_qw_row<NN>, (cudaFuncAttribute)mx, sr));
+      QG_CK(cudaFuncSetAttribute(k_adj_qw_col_fwd<NN>, (cudaFuncAttribute)mx, sc));
     });
     ready = true;
     return QG_OK;
@@ -237,6 +234,7 @@ class AdjEngine final : public Engine<double> {
   }
   int restore(const std::vector<C*>& s) {
     const int f9[9] = {F_Q, F_QO, F_BR, F_BI, F_BRO, F_BIO, F_PSI, F_AR, F_AI};
+    q_valid = false;     // B changes under the kept planes
     for (int i = 0; i < kCk; ++i)
       QG_CK(cudaMemcpyAsync(F[f9[i]], s[i], field_bytes(), cudaMemcpyDeviceToDevice, st));
     return QG_OK;
@@ -366,31 +364,35 @@ class AdjEngine final : public Engine<double> {
     for (int z0 = 0; z0 < g.n3; z0 += Zb) {
       const int zc = std::min(Zb, g.n3 - z0);
       QG_SWITCH_N(g.n, {
-        const dim3 gc(g.KXP / Tiles<double, NN>::CT, zc), gr(g.n / Tiles<double, NN>::RT, zc);
-        k_col_inv<double, NN><<<gc, Tiles<double, NN>::CNT, sm_ci<NN, Tiles<double, NN>::CIP>(Tiles<double, NN>::CINF), st>>>(g, z0, psi, q, BR, BI, S, tw, nullptr, 0);
+        using FC = FxCol<NN>;
+        using FR = FxRow<NN>;
+        const dim3 gc((g.K + FC::CT) / FC::CT, zc), gr(g.n / FR::RT, zc);
+        launch_col_inv<NN>(z0, zc, psi, q, BR, BI, S, nullptr, 0, st);
         QG_LAUNCHED();
-        k_adj_col_inv<NN><<<gc, kColThreads, sm_col6<NN>(), st>>>(g, p, z0, L, e1, e2, e1w, e2w, SA, tw);
+        k_adj_col_inv<NN><<<gc, FC::NT, FC::smem(), st>>>(g, p, z0, L, e1, e2, e1w, e2w, SA, tw);
         QG_LAUNCHED();
-        k_adj_row<NN><<<gr, kThreadsB, sm_row7<NN>(), st>>>(g, p, S, SA, tw);
+        k_adj_row<NN><<<gr, FR::NT, AdjRow<NN>::smem(), st>>>(g, p, S, SA, tw);
         QG_LAUNCHED();
-        k_adj_col_fwd<NN><<<gc, kColThreads, sm_col6<NN>(), st>>>(g, p, z0, L, O, e1, e2, e1w, e2w, SA, tw);
+        k_adj_col_fwd<NN><<<gc, FC::NT, FC::smem(), st>>>(g, p, z0, L, O, e1, e2, e1w, e2w, SA, tw);
         QG_LAUNCHED();
       });
     }
     int rc = solve_generic(Af[A_LPSI], Af[A_LAR], Af[A_LAI], Af[A_W], Af[A_LBRA], Af[A_LBIA], 1, 1);
     if (rc) return rc;
-    for (int z0 = 0; z0 < g.n3; z0 += Zb) {
+    const long long tot = (long long)g.n3 * g.plane;
+    k_adj_solved<<<grid_for(tot), 256, 0, st>>>(g, tot, lo[0], lo[2], lo[3], Af[A_W], Af[A_LBRA], Af[A_LBIA]);
+    QG_LAUNCHED();
+    for (int z0 = 0; need_qw && z0 < g.n3; z0 += Zb) {
       const int zc = std::min(Zb, g.n3 - z0);
       QG_SWITCH_N(g.n, {
-        const dim3 gc(g.KXP / Tiles<double, NN>::CT, zc), gr(g.n / Tiles<double, NN>::RT, zc);
-        if (need_qw) {
-          k_adj_qw_col_inv<NN><<<gc, kColThreads, sm_col6<NN>(), st>>>(g, z0, BR, BI, Af[A_W], S, tw);
-          QG_LAUNCHED();
-          k_adj_qw_row<NN><<<gr, kThreadsB, sm_row4<NN>(), st>>>(g, p, S, tw);
-          QG_LAUNCHED();
-        }
-        k_adj_qw_col_fwd<NN><<<gc, kColThreads, sm_col4<NN>(), st>>>(g, z0, need_qw ? 1 : 0, lo[0], lo[2], lo[3],
-                                                                     Af[A_W], Af[A_LBRA], Af[A_LBIA], S, tw);
+        using FC = FxCol<NN>;
+        using FR = FxRow<NN>;
+        const dim3 gc((g.K + FC::CT) / FC::CT, zc), gr(g.n / FR::RT, zc);
+        k_adj_qw_col_inv<NN><<<gc, FC::NT, FC::smem(), st>>>(g, z0, BR, BI, Af[A_W], S, tw);
+        QG_LAUNCHED();
+        k_adj_qw_row<NN><<<gr, FR::NT, FR::smem(), st>>>(g, p, S, tw);
+        QG_LAUNCHED();
+        k_adj_qw_col_fwd<NN><<<gc, FC::NT, FC::smem(), st>>>(g, z0, lo[2], lo[3], S, tw);
         QG_LAUNCHED();
       });
     }

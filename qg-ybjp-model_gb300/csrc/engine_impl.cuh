@@ -9,6 +9,8 @@
 #include <algorithm>
 #include "engine.h"
 #include "dense_kernels.cuh"
+#include "step_fx.cuh"
+#include "fx_twiddles.h"
 
 namespace qg {
 
@@ -95,10 +97,17 @@ class Engine : public EngineBase {
         QG_CK(cudaMemcpy(*dst[k], om[k]->data(), (size_t)g.n3 * sizeof(double), cudaMemcpyHostToDevice));
       }
     }
-    std::vector<C> twh(g.n);
-    for (int m = 0; m < g.n; ++m) twh[m] = mk<T>((T)t.tw[2 * m], (T)t.tw[2 * m + 1]);
+    // twiddles: W_n^m in FP32, the per-pass integer tables in FP64 (fxfft.cuh)
     QG_CK(cudaMalloc(&tw, g.n * sizeof(C)));
-    QG_CK(cudaMemcpy(tw, twh.data(), g.n * sizeof(C), cudaMemcpyHostToDevice));
+    if (sizeof(T) == 8) {
+      const std::vector<int32_t> twi = fx_twiddles(g.n);
+      static_assert(sizeof(T) != 8 || sizeof(C) == 4 * sizeof(int32_t), "one table entry per complex double");
+      QG_CK(cudaMemcpy(tw, twi.data(), g.n * sizeof(C), cudaMemcpyHostToDevice));
+    } else {
+      std::vector<C> twh(g.n);
+      for (int m = 0; m < g.n; ++m) twh[m] = mk<T>((T)t.tw[2 * m], (T)t.tw[2 * m + 1]);
+      QG_CK(cudaMemcpy(tw, twh.data(), g.n * sizeof(C), cudaMemcpyHostToDevice));
+    }
     QG_CK(cudaMalloc(&tab_idx, g.plane * sizeof(int)));
     QG_CK(cudaMemcpy(tab_idx, t.tab_idx.data(), g.plane * sizeof(int), cudaMemcpyHostToDevice));
     // columns of the solves: every column of the rectangle (any output
@@ -196,8 +205,8 @@ class Engine : public EngineBase {
     sp.ybj = cfg.ybj_plus ? 1 : 0;
     sp.mpar = mpar;
     need_qw = (!cfg.fixed_flow && !cfg.no_feedback);
-    // kept y-inverse planes of B (FP32 YBJ+ runs whose update transforms B^{n+1} for q^w)
-    if (kReuseB && sizeof(T) == 4 && need_qw && cfg.ybj_plus && kColInvNF2) {
+    // kept y-inverse planes of B (YBJ+ runs whose update transforms B^{n+1} for q^w)
+    if (kReuseB && need_qw && cfg.ybj_plus) {
       QG_CK(cudaMalloc(&Qp, (size_t)g.n3 * kNQ * g.n * g.KXP * sizeof(C)));
     }
     int r0 = set_smem_attrs();
@@ -862,8 +871,6 @@ class Engine : public EngineBase {
   template <int NN, int CP = 16> static constexpr size_t sm_ci(int nf) {
     return (size_t)(NN + nf * ColLay<NN, Tiles<T, NN>::CT, CP>::FS) * sizeof(C);
   }
-  template <int NN> static constexpr size_t sm_col6() { return (size_t)(NN + 6 * Tiles<T, NN>::CT * Tiles<T, NN>::LD) * sizeof(C); }
-  template <int NN> static constexpr size_t sm_row7() { return (size_t)(NN + 7 * Tiles<T, NN>::RT * Tiles<T, NN>::LD) * sizeof(C); }
   template <int NN> static constexpr size_t sm_rr3() { return (size_t)(NN + 3 * Tiles<T, NN>::QRT * Tiles<T, NN>::LD) * sizeof(C); }
   template <int NN> static constexpr size_t sm_rm4() { return (size_t)(NN + 4 * Tiles<T, NN>::RTM * Tiles<T, NN>::LD) * sizeof(C); }
   // the persistent row kernels add a staging copy of an item's scratch rows
@@ -876,30 +883,38 @@ class Engine : public EngineBase {
   template <int NN> static constexpr size_t sm_rq(int kxp) {
     return sm_rr3<NN>() + (Tiles<T, NN>::QPRE ? (size_t)4 * Tiles<T, NN>::QRT * kxp * sizeof(C) + 16 : 0);
   }
-  template <int NN> static constexpr size_t sm_row4() { return (size_t)(NN + 4 * Tiles<T, NN>::RT * Tiles<T, NN>::LD) * sizeof(C); }
-  // shared memory of the dense (routine-level) kernels
-  size_t sm_colinv() const { return (size_t)(g.n + 2 * Tile<T>::CT * (g.n + 1)) * sizeof(C); }
-  size_t sm_drow() const { return (size_t)(3 * g.n) * sizeof(C); }
 
   int set_smem_attrs() {
     const int mx = cudaFuncAttributeMaxDynamicSharedMemorySize;
     QG_SWITCH_N(g.n, {
-      QG_CK(cudaFuncSetAttribute(k_col_inv<T, NN>, (cudaFuncAttribute)mx, (int)sm_ci<NN, Tiles<T, NN>::CIP>(Tiles<T, NN>::CINF)));
-      QG_CK(cudaFuncSetAttribute(k_row_main<T, NN>, (cudaFuncAttribute)mx, (int)sm_rm<NN>(kxp_max<NN>())));
-      QG_CK(cudaFuncSetAttribute(k_col_update<T, NN>, (cudaFuncAttribute)mx, (int)UpdLay<T, NN>::bytes()));
-      QG_CK(cudaFuncSetAttribute(k_row_qw<T, NN>, (cudaFuncAttribute)mx, (int)sm_rq<NN>(kxp_max<NN>())));
-      QG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_rm, k_row_main<T, NN>, kRowThreads, sm_rm<NN>(g.KXP)));
-      QG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_rq, k_row_qw<T, NN>, Tiles<T, NN>::QTHREADS,
-                                                          sm_rq<NN>(g.KXP)));
+      if constexpr (kFx) {
+        const int sc = (int)FxCol<NN>::smem(), sr = (int)FxRow<NN>::smem();
+        QG_CK(cudaFuncSetAttribute(k_fx_col_inv<NN>, (cudaFuncAttribute)mx, sc));
+        QG_CK(cudaFuncSetAttribute(k_fx_col_update<NN>, (cudaFuncAttribute)mx, sc));
+        QG_CK(cudaFuncSetAttribute(k_fx_col_qw<NN>, (cudaFuncAttribute)mx, sc));
+        QG_CK(cudaFuncSetAttribute(k_fx_row_main<NN>, (cudaFuncAttribute)mx, sr));
+        QG_CK(cudaFuncSetAttribute(k_fx_row_qw<NN>, (cudaFuncAttribute)mx, sr));
+        QG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_rm, k_fx_row_main<NN>, FxRow<NN>::NT, sr));
+        QG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_rq, k_fx_row_qw<NN>, FxRow<NN>::NT, sr));
+      } else {
+        QG_CK(cudaFuncSetAttribute(k_col_inv<T, NN>, (cudaFuncAttribute)mx, (int)sm_ci<NN, Tiles<T, NN>::CIP>(Tiles<T, NN>::CINF)));
+        QG_CK(cudaFuncSetAttribute(k_row_main<T, NN>, (cudaFuncAttribute)mx, (int)sm_rm<NN>(kxp_max<NN>())));
+        QG_CK(cudaFuncSetAttribute(k_col_update<T, NN>, (cudaFuncAttribute)mx, (int)UpdLay<T, NN>::bytes()));
+        QG_CK(cudaFuncSetAttribute(k_row_qw<T, NN>, (cudaFuncAttribute)mx, (int)sm_rq<NN>(kxp_max<NN>())));
+        QG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_rm, k_row_main<T, NN>, kRowThreads, sm_rm<NN>(g.KXP)));
+        QG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_rq, k_row_qw<T, NN>, Tiles<T, NN>::QTHREADS,
+                                                            sm_rq<NN>(g.KXP)));
+        QG_CK(cudaFuncSetAttribute(k_col_qw<T, NN>, (cudaFuncAttribute)mx, (int)sm_ci<NN, Tiles<T, NN>::CQP>(2)));
+      }
       occ_rm = std::max(occ_rm, 1);
       occ_rq = std::max(occ_rq, 1);
-      QG_CK(cudaFuncSetAttribute(k_col_qw<T, NN>, (cudaFuncAttribute)mx, (int)sm_ci<NN, Tiles<T, NN>::CQP>(2)));
       // per-function attribute shared by every handle: set it for the deepest supported column
       QG_CK(cudaFuncSetAttribute(k_solve<T>, (cudaFuncAttribute)mx, (int)solve_smem(kMaxN3)));
-      QG_CK(cudaFuncSetAttribute(k_dcol_inv<T, NN>, (cudaFuncAttribute)mx, (int)sm_colinv()));
-      QG_CK(cudaFuncSetAttribute(k_dcol_fwd<T, NN>, (cudaFuncAttribute)mx, (int)sm_colinv()));
-      QG_CK(cudaFuncSetAttribute(k_drow_c2r<T, NN>, (cudaFuncAttribute)mx, (int)sm_drow()));
-      QG_CK(cudaFuncSetAttribute(k_drow_r2c<T, NN>, (cudaFuncAttribute)mx, (int)sm_drow()));
+      using DN = Dense<T, NN>;
+      QG_CK(cudaFuncSetAttribute(k_dcol_inv<T, NN>, (cudaFuncAttribute)mx, (int)DN::sm_col()));
+      QG_CK(cudaFuncSetAttribute(k_dcol_fwd<T, NN>, (cudaFuncAttribute)mx, (int)DN::sm_col()));
+      QG_CK(cudaFuncSetAttribute(k_drow_c2r<T, NN>, (cudaFuncAttribute)mx, (int)DN::sm_row()));
+      QG_CK(cudaFuncSetAttribute(k_drow_r2c<T, NN>, (cudaFuncAttribute)mx, (int)DN::sm_row()));
     });
     return QG_OK;
   }
@@ -955,6 +970,28 @@ class Engine : public EngineBase {
   }
 
  protected:
+  // FP64 steps run on the kernels of step_fx.cuh
+  static constexpr bool kFx = sizeof(T) == 8;
+  template <int NN> static constexpr int col_ct() {
+    if constexpr (kFx) return FxCol<NN>::CT;
+    else return Tiles<T, NN>::CT;
+  }
+
+  // k_col_inv on levels [z0, z0 + zc): mode 0 all six fields into Sb, 1 the
+  // first four (BR, BI are kept in Qb), 2 BR and BI into Qb
+  template <int NN>
+  void launch_col_inv(int z0, int zc, const C* psi, const C* q, const C* br, const C* bi, C* Sb, C* Qb, int mode,
+                      cudaStream_t on) {
+    // column tiles up to kx = K (the padding columns beyond K are never read)
+    const dim3 gc((g.K + col_ct<NN>()) / col_ct<NN>(), zc);
+    if constexpr (kFx)
+      k_fx_col_inv<NN><<<gc, FxCol<NN>::NT, FxCol<NN>::smem(), on>>>(g, z0, psi, q, br, bi, Sb, tw, Qb,
+                                                                     mode == 2 ? 4 : 0, mode == 1 ? 4 : 6);
+    else
+      k_col_inv<T, NN><<<gc, Tiles<T, NN>::CNT, sm_ci<NN, Tiles<T, NN>::CIP>(Tiles<T, NN>::CINF), on>>>(
+          g, z0, psi, q, br, bi, Sb, tw, Qb, mode);
+  }
+
   // Enqueue one step on st (no synchronisation; graph-capturable).
   int enqueue_step(int euler) {
     StepParams s = sp;
@@ -988,16 +1025,19 @@ class Engine : public EngineBase {
       C* Sb = S + lane * slot;
       QG_SWITCH_N(g.n, {
         // column tiles up to kx = K (the padding columns beyond K are never read)
-        const dim3 gc((g.K + Tiles<T, NN>::CT) / Tiles<T, NN>::CT, zc), gr(g.n / Tiles<T, NN>::QRT, zc),
+        const dim3 gc((g.K + col_ct<NN>()) / col_ct<NN>(), zc), gr(g.n / Tiles<T, NN>::QRT, zc),
             grm(g.n / Tiles<T, NN>::RTM, zc);
         if (int rc0 = pbeg(QG_K_COL_INV, bs)) return rc0;
         C* Qb = Qp ? Qp + (size_t)z0 * kNQ * g.n * g.KXP : nullptr;
-        k_col_inv<T, NN><<<gc, Tiles<T, NN>::CNT, sm_ci<NN, Tiles<T, NN>::CIP>(Tiles<T, NN>::CINF), bs>>>(g, z0, F[F_PSI], F[F_Q], F[F_BR], F[F_BI], Sb, tw,
-                                                                Qb, Qb ? 1 : 0);
+        launch_col_inv<NN>(z0, zc, F[F_PSI], F[F_Q], F[F_BR], F[F_BI], Sb, Qb, Qb ? 1 : 0, bs);
         QG_LAUNCHED();
         if (int rc0 = pend(bs)) return rc0;
         if (int rc0 = pbeg(QG_K_ROW_MAIN, bs)) return rc0;
-        if constexpr (Tiles<T, NN>::RPRE) {
+        if constexpr (kFx) {
+          const int items = zc * (NN / FxRow<NN>::RT);
+          k_fx_row_main<NN><<<std::min(items, std::max(1, nsm * occ_rm / L)), FxRow<NN>::NT, FxRow<NN>::smem(), bs>>>(
+              g, s, Sb, tw, items, Qb);
+        } else if constexpr (Tiles<T, NN>::RPRE) {
           const int items = zc * (NN / Tiles<T, NN>::RTM);
           k_row_main<T, NN><<<std::min(items, std::max(1, nsm * occ_rm / L)), kRowThreads, sm_rm<NN>(g.KXP), bs>>>(g, s, Sb, tw, items,
                                                                                                  wflag, Qb);
@@ -1014,7 +1054,11 @@ class Engine : public EngineBase {
           QG_CK(cudaStreamWaitEvent(bs, ev_diag, cs == cudaStreamCaptureStatusActive ? cudaEventWaitExternal : 0));
         }
         if (int rc0 = pbeg(QG_K_COL_UPDATE, bs)) return rc0;
-        k_col_update<T, NN><<<gc, Tiles<T, NN>::CNT, UpdLay<T, NN>::bytes(), bs>>>(g, s, z0, sptr, e1, e2, e1w, e2w, Sb, tw,
+        if constexpr (kFx)
+          k_fx_col_update<NN><<<gc, FxCol<NN>::NT, FxCol<NN>::smem(), bs>>>(g, s, z0, sptr, e1, e2, e1w, e2w, Sb, tw,
+                                                                           need_qw ? 1 : 0, Qb);
+        else
+          k_col_update<T, NN><<<gc, Tiles<T, NN>::CNT, UpdLay<T, NN>::bytes(), bs>>>(g, s, z0, sptr, e1, e2, e1w, e2w, Sb, tw,
                                                                 need_qw ? 1 : 0, Qb);
         QG_LAUNCHED();
         if (int rc0 = pend(bs)) return rc0;
@@ -1028,7 +1072,11 @@ class Engine : public EngineBase {
         }
         if (need_qw) {
           if (int rc0 = pbeg(QG_K_ROW_QW, bs)) return rc0;
-          if constexpr (Tiles<T, NN>::QPRE) {
+          if constexpr (kFx) {
+            const int items = zc * (NN / FxRow<NN>::RT);
+            k_fx_row_qw<NN><<<std::min(items, std::max(1, nsm * occ_rq / L)), FxRow<NN>::NT, FxRow<NN>::smem(), bs>>>(
+                g, Sb, tw, items, Qb);
+          } else if constexpr (Tiles<T, NN>::QPRE) {
             const int items = zc * (NN / Tiles<T, NN>::QRT);
             const int per_sm = (split && last) ? std::max(1, occ_rq - kQwReserve) : occ_rq;
             k_row_qw<T, NN><<<std::min(items, std::max(1, nsm * per_sm / L)), Tiles<T, NN>::QTHREADS, sm_rq<NN>(g.KXP), bs>>>(
@@ -1039,7 +1087,10 @@ class Engine : public EngineBase {
           QG_LAUNCHED();
           if (int rc0 = pend(bs)) return rc0;
           if (int rc0 = pbeg(QG_K_COL_QW, bs)) return rc0;
-          k_col_qw<T, NN><<<gc, Tiles<T, NN>::CNT, sm_ci<NN, Tiles<T, NN>::CQP>(2), bs>>>(g, s, z0, F[F_Q], F[F_QSTAR], Sb, tw, nflag);
+          if constexpr (kFx)
+            k_fx_col_qw<NN><<<gc, FxCol<NN>::NT, FxCol<NN>::smem(), bs>>>(g, s, z0, F[F_Q], F[F_QSTAR], Sb, tw, nflag);
+          else
+            k_col_qw<T, NN><<<gc, Tiles<T, NN>::CNT, sm_ci<NN, Tiles<T, NN>::CQP>(2), bs>>>(g, s, z0, F[F_Q], F[F_QSTAR], Sb, tw, nflag);
           QG_LAUNCHED();
           if (int rc0 = pend(bs)) return rc0;
         }
@@ -1116,9 +1167,7 @@ class Engine : public EngineBase {
     for (int z0 = 0; z0 < g.n3; z0 += Zb) {
       const int zc = std::min(Zb, g.n3 - z0);
       QG_SWITCH_N(g.n, {
-        const dim3 gc((g.K + Tiles<T, NN>::CT) / Tiles<T, NN>::CT, zc);
-        k_col_inv<T, NN><<<gc, Tiles<T, NN>::CNT, sm_ci<NN, Tiles<T, NN>::CIP>(Tiles<T, NN>::CINF), st>>>(g, z0, F[F_PSI], F[F_Q], F[F_BR], F[F_BI], S, tw,
-                                                                Qp + (size_t)z0 * kNQ * g.n * g.KXP, 2);
+        launch_col_inv<NN>(z0, zc, F[F_PSI], F[F_Q], F[F_BR], F[F_BI], S, Qp + (size_t)z0 * kNQ * g.n * g.KXP, 2, st);
         QG_LAUNCHED();
       });
     }
@@ -1146,7 +1195,7 @@ class Engine : public EngineBase {
 
   // ---- dense drop-in plumbing ---------------------------------------------
   size_t dense_bytes(int nz) const { return (size_t)nz * g.n * (g.n / 2 + 1) * sizeof(double2); }
-  int iktxP() const { const int ct = Tile<T>::CT; return ((g.n / 2 + 1 + ct - 1) / ct) * ct; }
+  int iktxP() const { return dense_kxp(g.n); }
 
   int prep_dense(int nz) {
     if (nz <= 0) { err = "nz must be positive"; return QG_ERR_ARG; }
@@ -1165,22 +1214,22 @@ class Engine : public EngineBase {
   }
 
   int d_c2r(const double2* spec, T* phys, int nz) {
-    const int CT = Tile<T>::CT;
     QG_SWITCH_N(g.n, {
-      k_dcol_inv<T, NN><<<dim3(iktxP() / CT, nz), kThreads, sm_colinv(), st>>>(iktxP(), spec, W, tw);
+      using DN = Dense<T, NN>;
+      k_dcol_inv<T, NN><<<dim3(iktxP() / DN::CT, nz), DN::CNT, DN::sm_col(), st>>>(iktxP(), spec, W, tw);
       QG_LAUNCHED();
-      k_drow_c2r<T, NN><<<dim3(g.n / 2, nz), kThreads, sm_drow(), st>>>(iktxP(), W, phys, tw);
+      k_drow_c2r<T, NN><<<dim3(g.n / 2 / DN::RT, nz), DN::RNT, DN::sm_row(), st>>>(iktxP(), W, phys, tw);
       QG_LAUNCHED();
     });
     return QG_OK;
   }
 
   int d_r2c(const T* phys, double2* spec, int nz) {
-    const int CT = Tile<T>::CT;
     QG_SWITCH_N(g.n, {
-      k_drow_r2c<T, NN><<<dim3(g.n / 2, nz), kThreads, sm_drow(), st>>>(iktxP(), phys, W, tw);
+      using DN = Dense<T, NN>;
+      k_drow_r2c<T, NN><<<dim3(g.n / 2 / DN::RT, nz), DN::RNT, DN::sm_row(), st>>>(iktxP(), phys, W, tw);
       QG_LAUNCHED();
-      k_dcol_fwd<T, NN><<<dim3(iktxP() / CT, nz), kThreads, sm_colinv(), st>>>(iktxP(), W, spec, tw);
+      k_dcol_fwd<T, NN><<<dim3(iktxP() / DN::CT, nz), DN::CNT, DN::sm_col(), st>>>(iktxP(), W, spec, tw);
       QG_LAUNCHED();
     });
     return QG_OK;

@@ -1,4 +1,4 @@
-// Batched power-of-two FFTs held in shared memory, executed by a whole CTA.
+// Batched power-of-two FP32 FFTs held in shared memory, executed by a whole CTA.
 //
 // Stockham autosort, decimation in time, radices 8/4/2: pass p with radix R
 // reads x[j + r*N/R], twiddles by W_{Ns*R}^{(j mod Ns) r}, does a length-R DFT
@@ -77,61 +77,6 @@ __host__ __device__ constexpr int radix_of(int rem) {
   return (m % 3 == 0 || m >= 7) ? 8 : (m % 3 == 2 ? 4 : 2);
 }
 template <int REM> struct PassRadix { static constexpr int value = radix_of(REM); };
-
-// One Stockham pass over `batch` transforms of length N stored with leading
-// dimension ld; tw[m] = W_N^m (forward sign).
-template <typename T, int N, int R, int NS, bool FWD>
-__device__ __forceinline__ void stockham_pass(const cplx<T>* __restrict__ src, cplx<T>* __restrict__ dst,
-                                              int ld, int batch, const cplx<T>* __restrict__ tw) {
-  constexpr int NB = N / R;
-  const int total = batch * NB;
-  for (int t = threadIdx.x; t < total; t += blockDim.x) {
-    const int b = t / NB;
-    const int j = t - b * NB;
-    const cplx<T>* s = src + (long)b * ld;
-    cplx<T>* d = dst + (long)b * ld;
-    cplx<T> v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = s[j + r * NB];
-    const int k = j & (NS - 1);
-    if constexpr (NS > 1) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) {
-        cplx<T> w = tw[k * r * (N / (NS * R))];
-        if (!FWD) w.y = -w.y;
-        v[r] = cmul(v[r], w);
-      }
-    }
-    dftR<T, R, FWD>(v);
-    const int base = (j - k) * R + k;
-#pragma unroll
-    for (int r = 0; r < R; ++r) d[base + r * NS] = v[r];
-  }
-}
-
-template <typename T, int N, bool FWD, int NS>
-__device__ __forceinline__ cplx<T>* fft_passes(cplx<T>* a, cplx<T>* b, int ld, int batch, const cplx<T>* tw) {
-  if constexpr (NS >= N) {
-    return a;
-  } else {
-    constexpr int R = PassRadix<N / NS>::value;
-    stockham_pass<T, N, R, NS, FWD>(a, b, ld, batch, tw);
-    __syncthreads();
-    return fft_passes<T, N, FWD, NS * R>(b, a, ld, batch, tw);
-  }
-}
-
-// All threads of the CTA must call.  Input in `a`, `b` is scratch of the same
-// size; returns the buffer that holds the result.  Ends with __syncthreads().
-template <typename T, int N, bool FWD>
-__device__ __forceinline__ cplx<T>* block_fft(cplx<T>* a, cplx<T>* b, int ld, int batch, const cplx<T>* tw) {
-  return fft_passes<T, N, FWD, 1>(a, b, ld, batch, tw);
-}
-
-template <typename T, int N>
-__device__ __forceinline__ void load_twiddles(cplx<T>* tw_s, const cplx<T>* __restrict__ tw_g) {
-  for (int i = threadIdx.x; i < N; i += blockDim.x) tw_s[i] = tw_g[i];
-}
 
 }  // namespace qg
 

@@ -1,0 +1,256 @@
+// FP64-grade FFTs on the integer pipes: transforms of doubles carried out in
+// 64-bit block fixed point.
+//
+// GB300 issues FP64 at 2 lanes per clock and SM; 64-bit integer additions run
+// at 62 and 32x32->64 multiply-adds at 30 (measured).  A radix-8 butterfly
+// with its twiddles is 82 FP64 operations (1312 SM clocks per warp) or about
+// 290 integer ones (about 160 clocks), so the FP64 path transforms integers:
+//
+//   * Each transform finds the largest exponent among its inputs (|x| < 2^E)
+//     and scales every input to an integer m = x 2^(59-E) (values below
+//     2^(E-59) lose bits there, where a double keeps them; against the
+//     transform's largest input that is 64 times finer than FP64's own
+//     rounding).
+//   * A radix-R pass lets the modulus grow by at most R, so the integers stay
+//     below 2^62.5 when every later pass divides its inputs by the earlier
+//     pass's radix.  The division is part of the twiddle factor, w = W 2^(64-s)
+//     and x w taken as the high word of the product; the untwiddled input is
+//     shifted.  All roundings are to nearest at 2^-62 of the growth bound.
+//   * The outputs are normalised back to doubles, rounded to nearest.
+// The rounding noise relative to the output's rms is at most about 2^-55.5
+// even for an input with a single nonzero value per transform (the worst
+// ratio of bound to rms), where an FP64 transform of the same length is at
+// 2^-53; measured errors against 113-bit transforms are in the tests.
+// A transform with a NaN or infinity among its inputs returns NaN; tiny and
+// huge scales (subnormal inputs, overflowing outputs) take exact slow paths.
+//
+// Only the forward sign is implemented: the inverse is the forward transform
+// with real and imaginary parts exchanged on the way in and out.
+#pragma once
+#include "fft_block.cuh"
+
+namespace qg {
+
+struct __align__(16) fxc { long long x, y; };
+
+// radix of the pass with stride ns of a length-n transform: radix 8 first
+// (eight values per thread throughout), then as radix_of
+__host__ __device__ constexpr int fx_radix(int n, int ns) { return ns == 1 ? 8 : (n < 64 ? n / 8 : radix_of(n / ns)); }
+// stride of the last pass
+template <int N> struct FxLast {
+  static constexpr int calc() {
+    int ns = 1;
+    while (ns * fx_radix(N, ns) < N) ns *= fx_radix(N, ns);
+    return ns;
+  }
+  static constexpr int value = calc();
+};
+// offset of the pass ns in the per-pass twiddle table
+template <int N> __host__ __device__ constexpr int fx_tw_off(int ns) {
+  int off = 0;
+  for (int s = 8; s < ns; s *= fx_radix(N, s)) off += s * (fx_radix(N, s) - 1);
+  return off;
+}
+
+// log2 of the factor a pass divides its inputs by: the earlier pass's radix
+// (at least 4: the factor 1 of a division by 2 would not fit a signed word)
+__host__ __device__ constexpr int fx_log2(int r) { return r == 8 ? 3 : (r == 4 ? 2 : 1); }
+template <int N> __host__ __device__ constexpr int fx_shift(int ns) {   // pass with stride ns > 1
+  int s = 1, r = 1;
+  while (s < ns) { r = fx_radix(N, s); s *= r; }
+  return fx_log2(r) < 2 ? 2 : fx_log2(r);
+}
+template <int N> __host__ __device__ constexpr int fx_shift_total() {
+  int t = 0;
+  for (int s = 8; s < N; s *= fx_radix(N, s)) t += fx_shift<N>(s);
+  return t;
+}
+
+__host__ __device__ constexpr int fx_ilog2(int n) { int m = 0; while ((1 << m) < n) ++m; return m; }
+// transforms this long take back the room that a peaked spectrum leaves
+// unused below the growth bound, before each later pass
+template <int N> __host__ __device__ constexpr bool fx_renorm() { return N >= 1024; }
+
+// radix of the pass before the one with stride ns > 1
+template <int N> __host__ __device__ constexpr int fx_prev_radix(int ns) {
+  int s = 1, r = 1;
+  while (s < ns) { r = fx_radix(N, s); s *= r; }
+  return r;
+}
+
+// (x + i y) * w with w = (c.hi, c.lo, s.hi, s.lo), c = c.hi 2^32 + c.lo with a
+// signed low word: the high 64 bits of the products, without low x low.  The
+// operands' low words are made signed too, so that every partial product is a
+// signed 32x32->64 multiply-add.  |x|, |y| < 2^62.5 and |w| <= 2^62 keep the
+// cross terms below 2^63.
+__device__ __forceinline__ void fx_cmul(fxc& v, const int4 w) {
+  const int xl = (int)v.x, yl = (int)v.y;
+  const int xh = (int)(v.x >> 32) + (int)((unsigned)xl >> 31);
+  const int yh = (int)(v.y >> 32) + (int)((unsigned)yl >> 31);
+  const int nsh = -w.z, nsl = -w.w;
+  long long cr = (long long)xh * w.y + 0x80000000LL;
+  long long ci = (long long)xh * w.w + 0x80000000LL;
+  cr += (long long)xl * w.x;
+  ci += (long long)xl * w.z;
+  cr += (long long)yh * nsl;
+  ci += (long long)yh * w.y;
+  cr += (long long)yl * nsh;
+  ci += (long long)yl * w.x;
+  long long re = (long long)xh * w.x + (cr >> 32);
+  long long im = (long long)xh * w.z + (ci >> 32);
+  re += (long long)yh * nsh;
+  im += (long long)yh * w.x;
+  v.x = re;
+  v.y = im;
+}
+
+// x / sqrt(2): x + x (h - 1), h = 2^-1/2, (h - 1) 2^64 split as above
+__device__ __forceinline__ long long fx_mulh(long long x) {
+  constexpr long long W = -0x4AFB0CCC06219B7CLL;    // round((2^-1/2 - 1) 2^64)
+  constexpr int cl = (int)W;
+  constexpr int ch = (int)((W - (long long)cl) >> 32);
+  const int xl = (int)x, xh = (int)(x >> 32) + (int)((unsigned)xl >> 31);
+  long long c = (long long)xh * cl + 0x80000000LL;
+  c += (long long)xl * ch;
+  return x + ((long long)xh * ch + (c >> 32));
+}
+
+__device__ __forceinline__ fxc fx_add(fxc a, fxc b) { a.x += b.x; a.y += b.y; return a; }
+__device__ __forceinline__ fxc fx_sub(fxc a, fxc b) { a.x -= b.x; a.y -= b.y; return a; }
+__device__ __forceinline__ fxc fx_mul_mi(fxc a) { fxc r; r.x = a.y; r.y = -a.x; return r; }   // * -i
+
+// (x + 2^(s-1)) >> s
+__device__ __forceinline__ fxc fx_shr(fxc a, int s) {
+  const long long h = 1LL << (s - 1);
+  a.x = (a.x + h) >> s;
+  a.y = (a.y + h) >> s;
+  return a;
+}
+
+// forward DFTs of 4, 8 and R values
+__device__ __forceinline__ void fx_dft4(fxc* v) {
+  const fxc s02 = fx_add(v[0], v[2]), d02 = fx_sub(v[0], v[2]);
+  const fxc s13 = fx_add(v[1], v[3]), t = fx_sub(v[1], v[3]);
+  v[0] = fx_add(s02, s13);
+  v[2] = fx_sub(s02, s13);
+  // d02 +- (-i) t
+  v[1].x = d02.x + t.y; v[1].y = d02.y - t.x;
+  v[3].x = d02.x - t.y; v[3].y = d02.y + t.x;
+}
+__device__ __forceinline__ void fx_dft8(fxc* v) {
+  fxc a[4], b[4];
+#pragma unroll
+  for (int n = 0; n < 4; ++n) { a[n] = fx_add(v[n], v[n + 4]); b[n] = fx_sub(v[n], v[n + 4]); }
+  // b[n] *= W8^n
+  fxc t = b[1];
+  b[1].x = fx_mulh(t.x + t.y);
+  b[1].y = fx_mulh(t.y - t.x);
+  b[2] = fx_mul_mi(b[2]);
+  t = b[3];
+  b[3].x = fx_mulh(t.y - t.x);
+  b[3].y = -fx_mulh(t.x + t.y);
+  fx_dft4(a);
+  fx_dft4(b);
+  v[0] = a[0]; v[2] = a[1]; v[4] = a[2]; v[6] = a[3];
+  v[1] = b[0]; v[3] = b[1]; v[5] = b[2]; v[7] = b[3];
+}
+template <int R> __device__ __forceinline__ void fx_dft(fxc* v) {
+  if constexpr (R == 8) fx_dft8(v);
+  else if constexpr (R == 4) fx_dft4(v);
+  else { const fxc t = v[0]; v[0] = fx_add(t, v[1]); v[1] = fx_sub(t, v[1]); }
+}
+
+// one later pass's butterfly: scale, twiddle, DFT; twp: the pass's table
+template <int N, int R, int NS> __device__ __forceinline__ void fx_butterfly(fxc* v, const int4* __restrict__ tw, int k) {
+  constexpr int s = fx_shift<N>(NS), off = fx_tw_off<N>(NS);
+  v[0] = fx_shr(v[0], s);
+#pragma unroll
+  for (int r = 1; r < R; ++r) fx_cmul(v[r], tw[off + (r - 1) * NS + k]);
+  fx_dft<R>(v);
+}
+
+// --- doubles <-> integers ---------------------------------------------------
+// hi word of |x|: its maximum orders the inputs' magnitudes
+__device__ __forceinline__ unsigned fx_mag(double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; }
+// transforms whose largest biased exponent is below this are scaled by 2^512
+// first (exact), so that subnormal inputs need no case of their own
+constexpr int kFxTiny = 64;
+// x 2^(59-E) truncated, be >= kFxTiny the largest biased exponent (E = be - 1022)
+__device__ __forceinline__ long long fx_in1(double x, int be) {
+  const int hi = __double2hiint(x);
+  const unsigned lo = (unsigned)__double2loint(x);
+  const int d = min(be - ((hi >> 20) & 0x7ff), 63);
+  unsigned long long m = ((unsigned long long)((hi & 0xfffff) | 0x100000) << 32 | lo) << 6;
+  m >>= d;
+  const long long s = (long long)(hi >> 31);
+  return ((long long)m ^ s) - s;
+}
+// m 2^(base-1075-...) to the nearest double: base is the biased exponent of
+// the integer's bit 0, 1 <= base and base + 63 <= 2046
+__device__ __forceinline__ double fx_out1(long long m, int base) {
+  const long long s = m >> 63;
+  const unsigned long long a = (unsigned long long)((m ^ s) - s);
+  const int lz = __clzll((long long)a);
+  const unsigned long long t = a << (lz & 63);
+  unsigned long long r = (t >> 11) + ((t >> 10) & 1ull) + ((unsigned long long)(unsigned)(base + 62 - lz) << 52);
+  r = a ? r : 0ull;
+  return __longlong_as_double((long long)(r | ((unsigned long long)s & 0x8000000000000000ull)));
+}
+// Exponents: an integer m stands for m 2^(base-1023).  kFxNan: a transform
+// with a non-finite input (bases are sums of a few of these).
+constexpr int kFxNan = 1 << 20;
+__device__ __forceinline__ bool fx_is_nan(int base) { return base > (1 << 18); }
+// whether every integer's double is a normal number (or zero)
+__device__ __forceinline__ bool fx_fast(int base) { return base >= 1 && base + 63 <= 2046; }
+// 2^e, -1022 <= e <= 1023
+__device__ __forceinline__ double fx_pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+// o <- o 2^(base-1023) for normal o in [1, 2^63] or 0, at scales where the
+// result may be subnormal, zero, infinite or NaN: three exact powers of two,
+// of which only the last can round
+template <int M> __device__ __forceinline__ void fx_rescale(double2* o, int base) {
+  const int e = min(max(base - 1023, -2400), 2400), t = e / 3;
+  const double a = fx_is_nan(base) ? __longlong_as_double(0x7ff8000000000000ll) : fx_pow2(t), b = fx_pow2(t),
+               c = fx_pow2(e - 2 * t);
+#pragma unroll
+  for (int r = 0; r < M; ++r) { o[r].x = ((o[r].x * a) * b) * c; o[r].y = ((o[r].y * a) * b) * c; }
+}
+// doubles of the integers v 2^(base-1023), M complex values; SWAP exchanges
+// the parts.  One branch for all of them: a rescaling per value was predicated
+// into every conversion and made the kernels 25-50 % slower.
+template <int M, bool SWAP> __device__ __forceinline__ void fx_doubles(const fxc* v, double2* o, int base) {
+  const bool fast = fx_fast(base);
+  const int b = fast ? base : 1023;
+#pragma unroll
+  for (int r = 0; r < M; ++r) {
+    const double x = fx_out1(v[r].x, b), y = fx_out1(v[r].y, b);
+    o[r] = SWAP ? make_double2(y, x) : make_double2(x, y);
+  }
+  if (!fast) fx_rescale<M>(o, base);
+}
+// bits set in any of the magnitudes' high words (x ^ sign)
+template <int R> __device__ __forceinline__ unsigned fx_bits(const fxc* v) {
+  unsigned o = 0;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int a = (int)(v[r].x >> 32), b = (int)(v[r].y >> 32);
+    o |= (unsigned)(a ^ (a >> 31)) | (unsigned)(b ^ (b >> 31));
+  }
+  return o;
+}
+// left shift that brings components with these bits below 2^61 (the sums of
+// two outputs of a transform then stay below 2^63)
+__device__ __forceinline__ int fx_room(unsigned o) { return max(__clz((int)o) - 3, 0); }
+template <int R> __device__ __forceinline__ void fx_shl(fxc* v, int s) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) { v[r].x <<= s; v[r].y <<= s; }
+}
+// shared copy of the per-pass integer twiddles (at most N entries; the host
+// lays them out as load_tw_passes does, see fx_twiddles)
+template <int N> __host__ __device__ constexpr int fx_tw_count() {
+  return fx_tw_off<N>(N);
+}
+template <int N> __device__ __forceinline__ void fx_load_tw(double2* tw_s, const double2* __restrict__ tw_g, int nt) {
+  for (int i = threadIdx.x; i < fx_tw_count<N>(); i += nt) tw_s[i] = tw_g[i];
+}
+
+}  // namespace qg

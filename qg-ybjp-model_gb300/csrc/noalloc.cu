@@ -16,15 +16,16 @@
 #include <vector>
 #include "dense_kernels.cuh"
 #include "engine.h"
+#include "fx_twiddles.h"
 #include "noalloc_check.h"
 
 namespace {
 
 // Scratch for the (kx, y) intermediate of one chunk of levels: 8 MiB holds at
-// least one level for every n <= 512 (n * (n/2+1 rounded up to 4) * 16 bytes).
+// least one level for every n <= 512 (n * (n/2+1 rounded up to 8) * 16 bytes).
 constexpr size_t kScratchBytes = size_t(8) << 20;
 __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
-// Twiddles W_n^m = exp(-2 pi i m / n) of every supported n, packed: n = 16, 32, ..., 512.
+// Integer twiddle tables (fx_twiddles.h) of every supported n, packed: n = 16, 32, ..., 512.
 constexpr int kTwEntries = 16 + 32 + 64 + 128 + 256 + 512;
 __device__ __align__(256) double2 g_noalloc_tw[kTwEntries];
 
@@ -41,11 +42,6 @@ int tw_offset(int n) {
   int off = 0;
   for (int m = 16; m < n; m *= 2) off += m;
   return off;
-}
-
-int iktxp(int n) {
-  constexpr int ct = qg::Tile<double>::CT;
-  return ((n / 2 + 1 + ct - 1) / ct) * ct;
 }
 
 int fail(int code, const std::string& msg) {
@@ -70,28 +66,18 @@ int setup_device(int dev, DeviceSetup** out) {
     s.scratch = static_cast<double2*>(p);
     NA_CK(cudaGetSymbolAddress(&p, g_noalloc_tw));
     s.tw = static_cast<double2*>(p);
-    std::vector<double2> tw(kTwEntries);
-    const double twopi = 4.0 * std::asin(1.0);
-    for (int n = 16, off = 0; n <= 512; off += n, n *= 2) {
-      for (int m = 0; m < n; ++m) {
-        double cs, sn;
-        if ((4 * m) % n == 0) {
-          const double C4[4] = {1, 0, -1, 0}, S4[4] = {0, 1, 0, -1};
-          cs = C4[(4 * m) / n]; sn = S4[(4 * m) / n];
-        } else {
-          const double th = twopi * (double)m / (double)n;
-          cs = std::cos(th); sn = std::sin(th);
-        }
-        tw[off + m] = make_double2(cs, -sn);
-      }
+    std::vector<int32_t> tw;
+    for (int n = 16; n <= 512; n *= 2) {
+      const std::vector<int32_t> t = qg::fx_twiddles(n);
+      tw.insert(tw.end(), t.begin(), t.end());
     }
     NA_CK(cudaMemcpyToSymbol(g_noalloc_tw, tw.data(), sizeof(double2) * kTwEntries));
     const int mx = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    const int ct = qg::Tile<double>::CT;
 #define NA_ATTR(NN)                                                                                        \
     NA_CK(cudaFuncSetAttribute(qg::k_dcol_inv<double, NN>, (cudaFuncAttribute)mx,                          \
-                               (int)((NN + 2 * ct * (NN + 1)) * sizeof(double2))));                        \
-    NA_CK(cudaFuncSetAttribute(qg::k_drow_c2r_pad<double, NN>, (cudaFuncAttribute)mx, (int)(3 * NN * sizeof(double2))));
+                               (int)qg::Dense<double, NN>::sm_col()));                                     \
+    NA_CK(cudaFuncSetAttribute(qg::k_drow_c2r_pad<double, NN>, (cudaFuncAttribute)mx,                      \
+                               (int)qg::Dense<double, NN>::sm_row()));
     NA_ATTR(16) NA_ATTR(32) NA_ATTR(64) NA_ATTR(128) NA_ATTR(256) NA_ATTR(512)
 #undef NA_ATTR
     s.ready = true;
@@ -137,19 +123,17 @@ int check_device_pointer(const void* p, int dev, uintptr_t align, const char* na
 
 template <int N>
 int launch_chunks(const double2* in, double* out, int nz, cudaStream_t st, const DeviceSetup& s) {
-  const int ip = iktxp(N);
+  using DN = qg::Dense<double, N>;
+  constexpr int ip = qg::dense_kxp(N);
   const size_t per_level = (size_t)N * ip * sizeof(double2);
   const int chunk = (int)(kScratchBytes / per_level);
-  const int ct = qg::Tile<double>::CT;
-  const size_t sm_col = (size_t)(N + 2 * ct * (N + 1)) * sizeof(double2);
-  const size_t sm_row = (size_t)(3 * N) * sizeof(double2);
   const double2* tw = s.tw + tw_offset(N);
   for (int z0 = 0; z0 < nz; z0 += chunk) {
     const int zc = nz - z0 < chunk ? nz - z0 : chunk;
-    qg::k_dcol_inv<double, N><<<dim3(ip / ct, zc), qg::kThreads, sm_col, st>>>(
+    qg::k_dcol_inv<double, N><<<dim3(ip / DN::CT, zc), DN::CNT, DN::sm_col(), st>>>(
         ip, in + (size_t)z0 * N * (N / 2 + 1), s.scratch, tw);
     NA_LAUNCH_CK();
-    qg::k_drow_c2r_pad<double, N><<<dim3(N / 2, zc), qg::kThreads, sm_row, st>>>(
+    qg::k_drow_c2r_pad<double, N><<<dim3(N / 2 / DN::RT, zc), DN::RNT, DN::sm_row(), st>>>(
         ip, s.scratch, out + (size_t)z0 * N * (N + 2), tw);
     NA_LAUNCH_CK();
   }
