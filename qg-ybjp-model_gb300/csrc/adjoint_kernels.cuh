@@ -207,6 +207,7 @@ k_adj_col_inv(Geom g, AdjP p, int zbase, AdjIn L, const double* __restrict__ e1t
   const long long zoff = (long long)(zbase + zb) * g.plane;
   const double inv2n2 = 0.5 / ((double)N * (double)N);
   // l and -i ky l of the adjoint tendencies of q, BR, BI
+#pragma unroll 1
   for (int f = 0; f < 6; ++f) {
     const int w = f >> 1;
     adj_col_inverse<N>(c, g, kx, SA + scr_off(zb, f, 0, N, g.KXP), [&](int row, int ky) {
@@ -241,64 +242,69 @@ k_adj_row(Geom g, AdjP p, const double2* __restrict__ SF, double2* __restrict__ 
   auto sf = [&](int f) { return SF + scr_off(zb, f, y, N, g.KXP); };
   auto sa = [&](int f) { return SA + scr_off(zb, f, y, N, g.KXP); };
   const double adv = p.adv, hr = 0.5 * p.refr;
-  for (int q = 0; q < 3; ++q) {
-    double2 d[8], o[8];
-    const double2 *X = sf(2 * q), *Y = sf(2 * q + 1);
-    adj_pack<N>(j, K, d, [&](int kk, double2& a, double2& b) { a = X[kk]; b = Y[kk]; });
-    c.inverse_d(d, o);
-#pragma unroll
-    for (int r = 0; r < 8; ++r) park[(q * 8 + r) * F::NT] = o[r];
-  }
   double2 luv[8], lzq[8], lbb[8];
-  // (aq, aR, aI): l of q, BR, BI times (-i kx, d/dy) in physical space
 #pragma unroll
-  for (int q = 0; q < 3; ++q) {
+  for (int r = 0; r < 8; ++r) luv[r] = lzq[r] = lbb[r] = make_double2(0.0, 0.0);
+  // (u, v), (zeta, q), (br, bi); (aq, aR, aI): l of q, BR, BI times (-i kx,
+  // d/dy); the refraction's (lTI, -lTR)/2
+#pragma unroll 1
+  for (int q = 0; q < 7; ++q) {
+    const double2 *A = q < 3 ? sf(2 * q) : (q < 6 ? sa(2 * (q - 3)) : sa(4));
+    const double2 *B = q < 3 ? sf(2 * q + 1) : (q < 6 ? sa(2 * (q - 3) + 1) : sa(2));
+    const double sb = q < 3 ? 1.0 : (q < 6 ? adv : -hr);
     double2 d[8], o[8];
-    const double2 *A = sa(2 * q), *B = sa(2 * q + 1);
     adj_pack<N>(j, K, d, [&](int kk, double2& a, double2& b) {
-      a = cscale(cmul_mi(A[kk]), adv * (double)kk);
-      b = cscale(B[kk], adv);
+      a = A[kk];
+      b = cscale(B[kk], sb);
+      if (q >= 3) a = q < 6 ? cscale(cmul_mi(a), adv * (double)kk) : cscale(a, hr);
     });
     c.inverse_d(d, o);
+    if (q < 3) {
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const double2 uv = park[r * F::NT];
-      const double f = q == 0 ? park[(8 + r) * F::NT].y : (q == 1 ? park[(16 + r) * F::NT].x : park[(16 + r) * F::NT].y);
-      const double s = o[r].x * uv.x + o[r].y * uv.y;
-      if (q == 0) {
-        luv[r] = make_double2(o[r].x * f, o[r].y * f);
-        lzq[r].y = s;
-      } else {
+      for (int r = 0; r < 8; ++r) park[(q * 8 + r) * F::NT] = o[r];
+    } else if (q < 6) {
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const double2 uv = park[r * F::NT], x = park[((q == 3 ? 8 : 16) + r) * F::NT];
+        const double f = q == 4 ? x.x : x.y;
+        const double s = o[r].x * uv.x + o[r].y * uv.y;
         luv[r].x += o[r].x * f;
         luv[r].y += o[r].y * f;
-        if (q == 1) lbb[r].x = s; else lbb[r].y = s;
+        if (q == 3) lzq[r].y = s;
+        else if (q == 4) lbb[r].x = s;
+        else lbb[r].y = s;
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const double2 bb = park[(16 + r) * F::NT];
+        const double Z = park[(8 + r) * F::NT].x;
+        lzq[r].x = o[r].x * bb.x + o[r].y * bb.y;
+        lbb[r].x += o[r].x * Z;
+        lbb[r].y += o[r].y * Z;
       }
     }
   }
-  {
-    // refraction: (lTI, -lTR)/2
-    double2 d[8], o[8];
-    const double2 *A = sa(4), *B = sa(2);
-    adj_pack<N>(j, K, d, [&](int kk, double2& a, double2& b) { a = cscale(A[kk], hr); b = cscale(B[kk], -hr); });
-    c.inverse_d(d, o);
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const double2 bb = park[(16 + r) * F::NT];
-      const double Z = park[(8 + r) * F::NT].x;
-      lzq[r].x = o[r].x * bb.x + o[r].y * bb.y;
-      lbb[r].x += o[r].x * Z;
-      lbb[r].y += o[r].y * Z;
-    }
-  }
   double2 lv[3];
-  c.forward_d(luv, K, [&](int q, int k, double2 X, double2 Y) { sa(0)[k] = X; lv[q] = Y; });
-  c.forward_d(lzq, K, [&](int q, int k, double2 lZ, double2 lQ) {
-    const double kx = (double)k;
-    sa(1)[k] = csub(cscale(cmul_mi(lv[q]), kx), cscale(lZ, kx * kx));
-    sa(2)[k] = lZ;
-    sa(3)[k] = lQ;
-  });
-  c.forward_d(lbb, K, [&](int, int k, double2 X, double2 Y) { sa(4)[k] = X; sa(5)[k] = Y; });
+#pragma unroll 1
+  for (int f = 0; f < 3; ++f) {
+    c.forward_d(luv, K, [&](int q, int k, double2 X, double2 Y) {
+      if (f == 0) {
+        sa(0)[k] = X;
+        lv[q] = Y;
+      } else if (f == 1) {
+        const double kx = (double)k;
+        sa(1)[k] = csub(cscale(cmul_mi(lv[q]), kx), cscale(X, kx * kx));
+        sa(2)[k] = X;
+        sa(3)[k] = Y;
+      } else {
+        sa(4)[k] = X;
+        sa(5)[k] = Y;
+      }
+    });
+#pragma unroll
+    for (int r = 0; r < 8; ++r) { luv[r] = lzq[r]; lzq[r] = lbb[r]; }
+  }
 }
 
 // Forward transform of plane P of a column tile times the weight of C^T (2,
@@ -343,28 +349,32 @@ k_adj_col_fwd(Geom g, AdjP p, int zbase, AdjIn L, AdjOut O, const double* __rest
   const FxColCtx<N> c = fx_col_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
   const int zb = blockIdx.y, kx = blockIdx.x * F::CT + c.c;
   const long long zoff = (long long)(zbase + zb) * g.plane;
-  auto plane = [&](int f) { return SA + scr_off(zb, f, 0, N, g.KXP); };
   // psi -> (u, v, zeta) = (-i ky, i kx, -kh^2) psi: transposes i ky, -i kx, -kh^2
   double2 a[8];
-  adj_col_plane<N>(c, g, plane(0), kx, [&](int r, long long, int ky, double2 h) { a[r] = cscale(cmul_i(h), (double)ky); });
-  adj_col_plane<N>(c, g, plane(1), kx, [&](int r, long long, int, double2 h) { a[r] = cadd(a[r], h); });
-  adj_col_plane<N>(c, g, plane(2), kx, [&](int r, long long mt, int ky, double2 h) {
-    O.lpsi[zoff + mt] = csub(a[r], cscale(h, (double)ky * (double)ky));
-  });
-  for (int w = 0; w < 3; ++w) {
-    adj_col_plane<N>(c, g, plane(3 + w), kx, [&](int, long long mt, int ky, double2 h) {
+#pragma unroll 1
+  for (int f = 0; f < 6; ++f) {
+    adj_col_plane<N>(c, g, SA + scr_off(zb, f, 0, N, g.KXP), kx, [&](int r, long long mt, int ky, double2 h) {
       const long long m = zoff + mt;
-      double2 lt = make_double2(0.0, 0.0), on = lt, oo = lt;
-      if (g.mask(kx, ky)) {
-        adj_update(p, L, w, m, w == 0 ? e1t[mt] : e1wt[mt], w == 0 ? e2t[mt] : e2wt[mt], lt, on, oo);
-        on = cadd(on, h);
+      if (f == 0) {
+        a[r] = cscale(cmul_i(h), (double)ky);
+      } else if (f == 1) {
+        a[r] = cadd(a[r], h);
+      } else if (f == 2) {
+        O.lpsi[m] = csub(a[r], cscale(h, (double)ky * (double)ky));
+      } else {
+        const int w = f - 3;
+        double2 lt = make_double2(0.0, 0.0), on = lt, oo = lt;
+        if (g.mask(kx, ky)) {
+          adj_update(p, L, w, m, w == 0 ? e1t[mt] : e1wt[mt], w == 0 ? e2t[mt] : e2wt[mt], lt, on, oo);
+          on = cadd(on, h);
+        }
+        O.l[w == 0 ? 0 : 1 + w][m] = on;
+        O.l[w == 0 ? 1 : 3 + w][m] = oo;
+        // T_R = N_BR + c kh^2 A_I - r_BI/2, T_I = N_BI - c kh^2 A_R + r_BR/2
+        const double ck = p.cdisp * (double)(kx * kx + ky * ky);
+        if (w == 1) O.lAI[m] = cscale(lt, ck);
+        if (w == 2) O.lAR[m] = cscale(lt, -ck);
       }
-      O.l[w == 0 ? 0 : 1 + w][m] = on;
-      O.l[w == 0 ? 1 : 3 + w][m] = oo;
-      // T_R = N_BR + c kh^2 A_I - r_BI/2, T_I = N_BI - c kh^2 A_R + r_BR/2
-      const double ck = p.cdisp * (double)(kx * kx + ky * ky);
-      if (w == 1) O.lAI[m] = cscale(lt, ck);
-      if (w == 2) O.lAR[m] = cscale(lt, -ck);
     });
   }
 }
@@ -382,6 +392,7 @@ k_adj_qw_col_inv(Geom g, int zbase, const double2* __restrict__ BR, const double
   const int zb = blockIdx.y, kx = blockIdx.x * F::CT + c.c;
   const long long zoff = (long long)(zbase + zb) * g.plane;
   const double inv2n2 = 0.5 / ((double)N * (double)N);
+#pragma unroll 1
   for (int f = 0; f < 6; ++f) {
     const double2* X = f < 2 ? BR : (f < 4 ? BI : w);
     adj_col_inverse<N>(c, g, kx, SF + scr_off(zb, f, 0, N, g.KXP), [&](int row, int ky) {
@@ -462,13 +473,14 @@ k_adj_qw_col_fwd(Geom g, int zbase, double2* __restrict__ lBR, double2* __restri
   const FxColCtx<N> c = fx_col_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
   const int zb = blockIdx.y, kx = blockIdx.x * F::CT + c.c;
   const long long zoff = (long long)(zbase + zb) * g.plane;
-  for (int b = 0; b < 2; ++b) {
-    double2* lB = b == 0 ? lBR : lBI;
-    double2 a[8];
-    adj_col_plane<N>(c, g, SF + scr_off(zb, 2 * b, 0, N, g.KXP), kx, [&](int r, long long, int, double2 h) { a[r] = h; });
-    adj_col_plane<N>(c, g, SF + scr_off(zb, 2 * b + 1, 0, N, g.KXP), kx, [&](int r, long long mt, int ky, double2 h) {
-      double2* o = lB + zoff + mt;
+  double2 a[8];
+#pragma unroll 1
+  for (int f = 0; f < 4; ++f) {
+    double2* lB = f < 2 ? lBR : lBI;
+    adj_col_plane<N>(c, g, SF + scr_off(zb, f, 0, N, g.KXP), kx, [&](int r, long long mt, int ky, double2 h) {
+      if ((f & 1) == 0) { a[r] = h; return; }
       // (a(0,0) is real; ky = 0 there, so the second term vanishes)
+      double2* o = lB + zoff + mt;
       *o = cadd(*o, csub(a[r], cscale(cmul_i(h), (double)ky)));
     });
   }

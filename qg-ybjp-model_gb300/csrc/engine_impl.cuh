@@ -892,9 +892,10 @@ class Engine : public EngineBase {
         QG_CK(cudaFuncSetAttribute(k_fx_col_inv<NN>, (cudaFuncAttribute)mx, sc));
         QG_CK(cudaFuncSetAttribute(k_fx_col_update<NN>, (cudaFuncAttribute)mx, sc));
         QG_CK(cudaFuncSetAttribute(k_fx_col_qw<NN>, (cudaFuncAttribute)mx, sc));
-        QG_CK(cudaFuncSetAttribute(k_fx_row_main<NN>, (cudaFuncAttribute)mx, sr));
+        QG_CK(cudaFuncSetAttribute(k_fx_row_main<NN>, (cudaFuncAttribute)mx, (int)FxMain<NN>::smem()));
         QG_CK(cudaFuncSetAttribute(k_fx_row_qw<NN>, (cudaFuncAttribute)mx, sr));
-        QG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_rm, k_fx_row_main<NN>, FxRow<NN>::NT, sr));
+        QG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_rm, k_fx_row_main<NN>, FxMain<NN>::F::NT,
+                                                            FxMain<NN>::smem()));
         QG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_rq, k_fx_row_qw<NN>, FxRow<NN>::NT, sr));
       } else {
         QG_CK(cudaFuncSetAttribute(k_col_inv<T, NN>, (cudaFuncAttribute)mx, (int)sm_ci<NN, Tiles<T, NN>::CIP>(Tiles<T, NN>::CINF)));
@@ -1034,8 +1035,8 @@ class Engine : public EngineBase {
         if (int rc0 = pend(bs)) return rc0;
         if (int rc0 = pbeg(QG_K_ROW_MAIN, bs)) return rc0;
         if constexpr (kFx) {
-          const int items = zc * (NN / FxRow<NN>::RT);
-          k_fx_row_main<NN><<<std::min(items, std::max(1, nsm * occ_rm / L)), FxRow<NN>::NT, FxRow<NN>::smem(), bs>>>(
+          const int items = zc * (NN / FxMain<NN>::F::RT);
+          k_fx_row_main<NN><<<std::min(items, std::max(1, nsm * occ_rm / L)), FxMain<NN>::F::NT, FxMain<NN>::smem(), bs>>>(
               g, s, Sb, tw, items, Qb);
         } else if constexpr (Tiles<T, NN>::RPRE) {
           const int items = zc * (NN / Tiles<T, NN>::RTM);

@@ -123,9 +123,9 @@ __device__ __forceinline__ void fx_core(fxc (&v)[8], int& base, fxc* __restrict_
 // Rows: one row per NB threads, synchronised by the row (its warp, or a named
 // barrier of its warps)
 // ===========================================================================
-template <int N> struct FxRow {
+template <int N, int T = 128> struct FxRow {
   static constexpr int NB = N / 8, LD = fx_idx(N);
-  static constexpr int RT = 128 / NB < N ? 128 / NB : N;  // rows per CTA
+  static constexpr int RT = T / NB < N ? T / NB : N;      // rows per CTA of T threads
   static constexpr int NT = RT * NB;                      // threads per CTA
   static constexpr int W = NB > 32 ? NB / 32 : 1;         // warps per row
   static constexpr int SLOTS = 3 * RT * W;
@@ -161,7 +161,7 @@ template <int NB, bool OR> __device__ __forceinline__ unsigned fx_row_reduce(uns
 }
 
 // The thread's view of its row: transforms of eight values per thread.
-template <int N> struct FxRowCtx {
+template <int N, int T = 128> struct FxRowCtx {
   static constexpr int NB = N / 8;
   fxc* buf;
   const int4* tw;
@@ -170,12 +170,12 @@ template <int N> struct FxRowCtx {
   int set = 0;         // reductions alternate between two sets: one follows another without a further barrier
   __device__ __forceinline__ void sync() const { fx_row_sync<NB>(rr); }
   template <bool OR> __device__ __forceinline__ unsigned reduce(unsigned m) {
-    set ^= FxRow<N>::RT * FxRow<N>::W;
+    set ^= FxRow<N, T>::RT * FxRow<N, T>::W;
     return fx_row_reduce<NB, OR>(m, slots + set, rr);
   }
   __device__ __forceinline__ void core(fxc (&v)[8], int& base) const {
     fx_core<N>(v, base, buf, tw, j, [](int i) { return fx_idx(i); }, [&]() { sync(); },
-               [&](unsigned m) { return fx_row_reduce<NB, true>(m, slots + 2 * FxRow<N>::RT * FxRow<N>::W, rr); });
+               [&](unsigned m) { return fx_row_reduce<NB, true>(m, slots + 2 * FxRow<N, T>::RT * FxRow<N, T>::W, rr); });
   }
   // inverse transform of the packed spectrum d (zeros at |k| > K) into
   // integers of 61 bits: v.y the first (real) row, v.x the second
@@ -231,11 +231,12 @@ template <int N> struct FxRowCtx {
   }
 };
 
-template <int N> __device__ __forceinline__ FxRowCtx<N> fx_row_ctx(double2* smem, unsigned* slots, const double2* twg) {
-  using F = FxRow<N>;
+template <int N, int T = 128>
+__device__ __forceinline__ FxRowCtx<N, T> fx_row_ctx(double2* smem, unsigned* slots, const double2* twg) {
+  using F = FxRow<N, T>;
   fx_load_tw<N>(smem, twg, F::NT);
   __syncthreads();
-  FxRowCtx<N> c;
+  FxRowCtx<N, T> c;
   c.rr = threadIdx.x / F::NB;
   c.j = threadIdx.x % F::NB;
   c.buf = reinterpret_cast<fxc*>(smem + fx_tw_count<N>()) + c.rr * F::LD;
@@ -295,12 +296,18 @@ template <int N> struct FxColCtx {
     for (int i = 0; i < F::W; ++i) m = OR ? (m | s[i * F::CT + c]) : max(m, s[i * F::CT + c]);
     return m;
   }
-  // transform of the doubles d (index j + r NB); v.x, v.y exchanged when
+  // the doubles d (index j + r NB) as integers, v.x, v.y exchanged when
   // inverse; PRUNED: zeros at |k| >= 3N/8
-  template <bool FWD, bool PRUNED = !FWD> __device__ __forceinline__ void run(double2 (&d)[8], fxc (&v)[8], int& base) const {
-    base = fx_ints<8, FWD, PRUNED>(d, v, reduce<false>(fx_maxp<8, PRUNED>(d), 0));
+  template <bool FWD, bool PRUNED = !FWD> __device__ __forceinline__ int load(double2 (&d)[8], fxc (&v)[8]) const {
+    return fx_ints<8, FWD, PRUNED>(d, v, reduce<false>(fx_maxp<8, PRUNED>(d), 0));
+  }
+  __device__ __forceinline__ void core(fxc (&v)[8], int& base) const {
     fx_core<N>(v, base, buf, tw, j, [&](int i) { return fx_idx(i) * F::CT + c; }, []() { __syncthreads(); },
                [&](unsigned m) { return reduce<true>(m, 1); });
+  }
+  template <bool FWD, bool PRUNED = !FWD> __device__ __forceinline__ void run(double2 (&d)[8], fxc (&v)[8], int& base) const {
+    base = load<FWD, PRUNED>(d, v);
+    core(v, base);
   }
 };
 template <int N> __device__ __forceinline__ FxColCtx<N> fx_col_ctx(double2* smem, unsigned* slots, const double2* twg) {

@@ -15,76 +15,95 @@
 
 namespace qg {
 
+// CTAs per SM (of 128 threads) that the register budgets target
 #ifndef QG_FX_ROW_CTAS
 #define QG_FX_ROW_CTAS 4
 #endif
-template <int N> __host__ __device__ constexpr int fx_row_ctas(int want) {
-  return imax(1, (want * 128) / FxRow<N>::NT);
+template <int N, int T = 128> __host__ __device__ constexpr int fx_row_ctas(int want) {
+  return imin(32, imax(1, (want * 128) / FxRow<N, T>::NT));
 }
 
 // ===========================================================================
 // Rows of convol_waqg / refraction_waqg (k_row_main's planes and results)
 // ===========================================================================
+// 256 threads, so that two CTAs' shared memory (transform buffers, and the
+// physical zeta, q, BR, BI parked as integers, each thread its own eight
+// points) fits an SM with one twiddle table each
+constexpr int kFxMainT = 256;
+template <int N> struct FxMain {
+  using F = FxRow<N, kFxMainT>;
+  static constexpr size_t smem() { return (size_t)(fx_tw_count<N>() + F::RT * F::LD + 2 * F::RT * N) * sizeof(double2); }
+};
 template <int N>
-__global__ void __launch_bounds__(FxRow<N>::NT, fx_row_ctas<N>(QG_FX_ROW_CTAS))
+__global__ void __launch_bounds__(FxMain<N>::F::NT, fx_row_ctas<N, kFxMainT>(QG_FX_ROW_CTAS))
 k_fx_row_main(Geom g, StepParams sp, double2* __restrict__ S, const double2* __restrict__ twg, int nitems,
               const double2* __restrict__ Qb) {
-  using F = FxRow<N>;
-  constexpr int NB = F::NB;
+  using F = typename FxMain<N>::F;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned slots[F::SLOTS];
-  FxRowCtx<N> c = fx_row_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
+  FxRowCtx<N, kFxMainT> c = fx_row_ctx<N, kFxMainT>(reinterpret_cast<double2*>(smem_raw), slots, twg);
+  fxc* zq = reinterpret_cast<fxc*>(smem_raw) + fx_tw_count<N>() + F::RT * F::LD + threadIdx.x;   // point r at zq[r * NT]
+  fxc* bb = zq + 8 * F::NT;
   const int K = g.K, j = c.j;
   constexpr int NG = N / F::RT;
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const int zb = it / NG, y = (it % NG) * F::RT + c.rr;
     auto plane = [&](int f) -> double2* { return S + scr_off(zb, f, y, N, g.KXP); };
-    fxc zq[8], bb[8], w[8];
-    int ezq, ebb, euv;
-    {
+    // inverse transforms of (zeta, q), (BR, BI), parked, and (u, v); then the
+    // forward transforms of (zeta br, zeta bi) (refraction) and of u and v
+    // times q, br, bi.  Two copies of the transform, each in a loop: with one
+    // per use the kernel's code outgrew the instruction cache, with one copy
+    // for both directions the loop's selects cost as much
+    fxc uv[8];
+    int ezq = 0, ebb = 0, euv = 0;
+#pragma unroll 1
+    for (int t = 0; t < 3; ++t) {
+      const double2 *X = plane(0), *Y = plane(1);
+      if (t == 0) { X = plane(2); Y = plane(3); }
+      else if (t == 1) { X = Qb ? Qb + q_off(zb, 0, y, N, g.KXP) : plane(4); Y = Qb ? Qb + q_off(zb, 1, y, N, g.KXP) : plane(5); }
       double2 d[8];
-      fx_pack<N>(plane(2), plane(3), j, K, d);
-      c.inverse(d, zq, ezq);
+      fx_pack<N>(X, Y, j, K, d);
+      c.inverse(d, uv, euv);
+      if (t < 2) {
+        if (t == 0) ezq = euv;
+        else ebb = euv;
+        fxc* pk = t == 0 ? zq : bb;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) pk[r * F::NT] = uv[r];
+      }
     }
-    {
-      double2 d[8];
-      const double2* pr = Qb ? Qb + q_off(zb, 0, y, N, g.KXP) : plane(4);
-      const double2* pi = Qb ? Qb + q_off(zb, 1, y, N, g.KXP) : plane(5);
-      fx_pack<N>(pr, pi, j, K, d);
-      c.inverse(d, bb, ebb);
-    }
-    // refraction: (zeta br, zeta bi); half its spectra enter planes 2 and 4
     double2 zr[3], zi[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) zr[q] = zi[q] = make_double2(0.0, 0.0);
-    if (sp.refr) {
+#pragma unroll 1
+    for (int f = sp.refr ? -1 : 0; f < 3; ++f) {
+      fxc w[8];
+      int base;
+      if (f < 0) {
+        base = ezq + ebb - 1023 + 63;      // (one exponent less: half of the spectra enters planes 2 and 4)
 #pragma unroll
-      for (int r = 0; r < 8; ++r) { w[r].x = fx_mulhi(zq[r].y, bb[r].y); w[r].y = fx_mulhi(zq[r].y, bb[r].x); }
-      // (one exponent less: the halves)
-      c.forward(w, ezq + ebb - 1023 + 63, K, [&](int q, int, double2 X, double2 Y) { zr[q] = X; zi[q] = Y; });
-    }
-    fxc uv[8];
-    {
-      double2 d[8];
-      fx_pack<N>(plane(0), plane(1), j, K, d);
-      c.inverse(d, uv, euv);
-    }
-    // G = i kx F(uX) (+- refraction), H = F(vX); tendency = F_y(G) + i ky F_y(H)
+        for (int r = 0; r < 8; ++r) {
+          const long long z = zq[r * F::NT].y;
+          const fxc b = bb[r * F::NT];
+          w[r].x = fx_mulhi(z, b.y);
+          w[r].y = fx_mulhi(z, b.x);
+        }
+      } else {
+        base = euv + (f == 0 ? ezq : ebb) - 1023 + 64;
+        const long long* px = f == 0 ? &zq->x : (f == 1 ? &bb->y : &bb->x);
 #pragma unroll
-    for (int f = 0; f < 3; ++f) {
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const long long x = f == 0 ? zq[r].x : (f == 1 ? bb[r].y : bb[r].x);
-        w[r].x = fx_mulhi(uv[r].y, x);
-        w[r].y = fx_mulhi(uv[r].x, x);
+        for (int r = 0; r < 8; ++r) {
+          const long long x = px[2 * r * F::NT];
+          w[r].x = fx_mulhi(uv[r].y, x);
+          w[r].y = fx_mulhi(uv[r].x, x);
+        }
       }
-      c.forward(w, euv + (f == 0 ? ezq : ebb) - 1023 + 64, K, [&](int q, int k, double2 X, double2 Y) {
+      c.forward(w, base, K, [&](int q, int k, double2 X, double2 Y) {
+        if (f < 0) { zr[q] = X; zi[q] = Y; return; }
+        // G = i kx F(uX) (+- refraction), H = F(vX); tendency = F_y(G) + i ky F_y(H)
         const double kx = (double)k;
         double2 G = make_double2(0.0, 0.0), H = G;
-        if (sp.adv) {
-          G = make_double2(-kx * X.y, kx * X.x);
-          H = Y;
-        }
+        if (sp.adv) { G = make_double2(-kx * X.y, kx * X.x); H = Y; }
         if (f == 1) { G.x -= zi[q].x; G.y -= zi[q].y; }
         if (f == 2) { G.x += zr[q].x; G.y += zr[q].y; }
         plane(2 * f)[k] = G;
@@ -99,7 +118,7 @@ k_fx_row_main(Geom g, StepParams sp, double2* __restrict__ S, const double2* __r
 // Rows of compute_qw (k_row_qw's planes and results)
 // ===========================================================================
 #ifndef QG_FX_QW_CTAS
-#define QG_FX_QW_CTAS 5
+#define QG_FX_QW_CTAS 4
 #endif
 template <int N>
 __global__ void __launch_bounds__(FxRow<N>::NT, fx_row_ctas<N>(QG_FX_QW_CTAS))
@@ -116,46 +135,57 @@ k_fx_row_qw(Geom g, double2* __restrict__ S, const double2* __restrict__ twg, in
     auto plane = [&](int f) -> double2* { return S + scr_off(zb, f, y, N, g.KXP); };
     const double2* pr = Qb ? Qb + q_off(zb, 0, y, N, g.KXP) : plane(0);
     const double2* pi = Qb ? Qb + q_off(zb, 1, y, N, g.KXP) : plane(2);
-    fxc a[8], b[8], w[8];
-    int ea, eb, e1, e2;
-    {
-      // (BRx, BIx): i kx times the packed spectrum of (BR, BI)
-      double2 d[8];
-      fx_pack<N>(pr, pi, j, K, d);
+    // inverse transforms of (BRx, BIx), (BRy, BIy), (BR, BI), then the forward
+    // transform of (P1, P2), through one copy of the transform
+    fxc a[8], p[8], w[8];
+    int ea = 0, e1 = 0, base = 0;
+#pragma unroll 1
+    for (int t = 0; t < 4; ++t) {
+      if (t < 3) {
+        double2 d[8];
+        fx_pack<N>(t == 1 ? plane(1) : pr, t == 1 ? plane(3) : pi, j, K, d);
+        if (t == 0) {
+          // i kx times the packed spectrum of (BR, BI)
 #pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const double k = (double)(j + r * NB - (r < 4 ? 0 : N));
-        d[r] = make_double2(-k * d[r].y, k * d[r].x);
+          for (int r = 0; r < 8; ++r) {
+            const double k = (double)(j + r * NB - (r < 4 ? 0 : N));
+            d[r] = make_double2(-k * d[r].y, k * d[r].x);
+          }
+        }
+        base = fx_ints<8, false, true>(d, w, c.template reduce<false>(fx_maxp<8, true>(d)));
+      } else {
+        fx_norm<8, 59>(w, c.template reduce<true>(fx_bits<8>(w)), base);
       }
-      c.inverse(d, a, ea);
-    }
-    {
-      double2 d[8];
-      fx_pack<N>(plane(1), plane(3), j, K, d);
-      c.inverse(d, b, eb);
-    }
-    // P1 = BRy BIx - BRx BIy (derivatives.f90:973)
+      c.core(w, base);
+      if (t < 3) fx_norm<8, 61>(w, c.template reduce<true>(fx_bits<8>(w)), base);
+      if (t == 0) {
 #pragma unroll
-    for (int r = 0; r < 8; ++r) w[r].x = fx_mulhi(b[r].y, a[r].x) - fx_mulhi(a[r].y, b[r].x);
-    e1 = ea + eb - 1023 + 64;
-    {
-      double2 d[8];
-      fx_pack<N>(pr, pi, j, K, d);
-      c.inverse(d, a, ea);
-    }
-    // P2 = BR^2 + BI^2 (derivatives.f90:996), then both to the larger exponent
-    e2 = 2 * ea - 1023 + 64;
-    const int s1 = min(max(e2 - e1, 0), 63), s2 = min(max(e1 - e2, 0), 63);
+        for (int r = 0; r < 8; ++r) a[r] = w[r];
+        ea = base;
+      } else if (t == 1) {
+        // P1 = BRy BIx - BRx BIy (derivatives.f90:973)
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      w[r].x >>= s1;
-      w[r].y = (fx_mulhi(a[r].y, a[r].y) + fx_mulhi(a[r].x, a[r].x)) >> s2;
+        for (int r = 0; r < 8; ++r) p[r].x = fx_mulhi(w[r].y, a[r].x) - fx_mulhi(a[r].y, w[r].x);
+        e1 = ea + base - 1023 + 64;
+      } else if (t == 2) {
+        // P2 = BR^2 + BI^2 (derivatives.f90:996), then both to the larger exponent
+        const int e2 = 2 * base - 1023 + 64;
+        const int s1 = min(max(e2 - e1, 0), 63), s2 = min(max(e1 - e2, 0), 63);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const long long P2 = fx_mulhi(w[r].y, w[r].y) + fx_mulhi(w[r].x, w[r].x);
+          w[r].x = p[r].x >> s1;
+          w[r].y = P2 >> s2;
+        }
+        base = max(e1, e2);
+      } else {
+        c.template split<3>(w, base, K, [&](int, int k, double2 P1, double2 P2) {
+          const double qk = 0.25 * (double)(k * k);
+          plane(0)[k] = make_double2(P1.x - qk * P2.x, P1.y - qk * P2.y);
+          plane(1)[k] = P2;
+        });
+      }
     }
-    c.forward(w, max(e1, e2), K, [&](int, int k, double2 P1, double2 P2) {
-      const double qk = 0.25 * (double)(k * k);
-      plane(0)[k] = make_double2(P1.x - qk * P2.x, P1.y - qk * P2.y);
-      plane(1)[k] = P2;
-    });
   }
 }
 
@@ -163,7 +193,7 @@ k_fx_row_qw(Geom g, double2* __restrict__ S, const double2* __restrict__ twg, in
 // Columns
 // ===========================================================================
 #ifndef QG_FX_COL_CTAS
-#define QG_FX_COL_CTAS 6
+#define QG_FX_COL_CTAS 7
 #endif
 template <int N> __host__ __device__ constexpr int fx_col_ctas(int want) { return imin(32, (want * 128) / FxCol<N>::NT); }
 
@@ -181,6 +211,7 @@ k_fx_col_inv(Geom g, int zbase, const double2* __restrict__ psi, const double2* 
   const FxColCtx<N> c = fx_col_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
   const int zb = blockIdx.y, kx = blockIdx.x * F::CT + c.c;
   const long long zoff = (long long)(zbase + zb) * g.plane;
+#pragma unroll 1
   for (int f = f0; f < f1; ++f) {
     const double2* X = f < 3 ? psi : (f == 3 ? q : (f == 4 ? BR : BI));
     double2 d[8];
@@ -254,11 +285,57 @@ k_fx_col_update(Geom g, StepParams sp, int zbase, StateP<double> st, const doubl
   const double cdisp = sp.disp ? (sp.mpar ? sp.mpar[4 * mem + 1] : sp.cdisp) : 0.0;
   const double gam = sp.gamma, dt2 = 2.0 * dt;
   const bool eul = sp.euler != 0;
-  for (int which = 0; which < 3; ++which) {
-    double2 G[8], H[8];
-    fx_col_plane<N>(c, g, S + scr_off(zb, 2 * which + 1, 0, N, g.KXP), kx, H);
-    fx_col_plane<N>(c, g, S + scr_off(zb, 2 * which, 0, N, g.KXP), kx, G);
+  // H and G of q, BR, BI, then the y-inverse transforms of B and i ky B at n+1
+  // (compute_qw, derivatives.f90:929-957: planes BR, i ky BR, BI, i ky BI =
+  // 0..3, BR and BI to the kept planes when given), through one copy of the
+  // transform
+  double2 H[8];
+  const int nt = qw_prep ? 10 : 6;
+#pragma unroll 1
+  for (int t = 0; t < nt; ++t) {
+    double2 d[8];
+    fxc v[8];
+    int base;
+    if (t < 6) {
+      const double2* p = S + scr_off(zb, t ^ 1, 0, N, g.KXP) + (long long)c.j * g.KXP + kx;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) d[r] = kx <= g.K ? p[(long long)r * NB * g.KXP] : make_double2(0.0, 0.0);
+      base = c.template load<true>(d, v);
+    } else {
+      if (t == 6) __syncthreads();      // B^{n+1}: this CTA's own stores
+      const double2* X = t < 8 ? st.BR : st.BI;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        d[r] = make_double2(0.0, 0.0);
+        if (fx_zero_in<8>(r)) continue;
+        int row; bool cj;
+        col_src(g, kx, c.j + r * NB, row, cj);
+        if (row < 0) continue;
+        double2 x = X[zoff + (long long)row * g.KXP + kx];
+        if (t & 1) { const double ky = (double)g.ky_of_row(row); x = make_double2(-ky * x.y, ky * x.x); }
+        if (cj) x.y = -x.y;
+        d[r] = x;
+      }
+      base = c.template load<false>(d, v);
+    }
+    c.core(v, base);
     if (kx > g.K) continue;
+    if (t >= 6) {
+      fx_doubles<8, true>(v, d, base);
+      const int p = t - 6;
+      double2* dst = (Qb && (p & 1) == 0) ? Qb + q_off(zb, p >> 1, 0, N, g.KXP) : S + scr_off(zb, p, 0, N, g.KXP);
+      dst += (long long)c.j * g.KXP + kx;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) dst[(long long)r * NB * g.KXP] = d[r];
+      continue;
+    }
+    fx_doubles<8, false>(v, d, base - 2 * fx_ilog2(N));     // (d[3], d[4] are not used)
+    if ((t & 1) == 0) {
+#pragma unroll
+      for (int r = 0; r < 8; ++r) H[r] = d[r];
+      continue;
+    }
+    const int which = t >> 1;
     double2* X = which == 0 ? st.q : (which == 1 ? st.BR : st.BI);
     double2* Xo = which == 0 ? st.qo : (which == 1 ? st.BRo : st.BIo);
     const double2* X3 = which == 0 ? st.dq : (which == 1 ? st.AI : st.AR);
@@ -274,7 +351,7 @@ k_fx_col_update(Geom g, StepParams sp, int zbase, StateP<double> st, const doubl
       const int ky = g.ky_of_row(row);
       const long long mt = (long long)row * g.KXP + kx, m = zoff + mt;
       const double fky = (double)ky;
-      const double2 tnd = make_double2(G[r].x - fky * H[r].y, G[r].y + fky * H[r].x);   // G + i ky H
+      const double2 tnd = make_double2(d[r].x - fky * H[r].y, d[r].y + fky * H[r].x);   // G + i ky H
       const double2 x0 = X[m];
       const double2 xo = eul ? x0 : Xo[m];
       double2 xn = make_double2(0.0, 0.0), xf = eul ? xo : xn;
@@ -282,18 +359,19 @@ k_fx_col_update(Geom g, StepParams sp, int zbase, StateP<double> st, const doubl
       if (live) {
         const double2 x3 = need3 ? X3[m] : make_double2(0.0, 0.0);
         const double e1 = t1[mt], e2 = t2[mt];
-        if (which == 0) {
-          if (eul) xn = cscale(cadd(csub(xo, cscale(tnd, dt)), cscale(x3, dt)), e1);
-          else xn = cadd(csub(cscale(xo, e2), cscale(cscale(tnd, dt2), e1)), cscale(cscale(x3, dt2), e2));
+        // q: tnd - dq; BR: nBR - 0.5 rBI + c kh2 AI; BI: nBI + 0.5 rBR - c kh2 AR
+        const double ck = which == 0 ? 0.0 : (which == 1 ? cdisp : -cdisp) * (double)(kx * kx + ky * ky);
+        const double2 fr = cadd(tnd, cscale(x3, ck));
+        if (eul) {
+          xn = csub(xo, cscale(fr, dt));
+          if (which == 0 && sp.use_dq) xn = cadd(xn, cscale(x3, dt));
+          xn = cscale(xn, e1);
         } else {
-          // nBR - 0.5 rBI + c kh2 AI ; nBI + 0.5 rBR - c kh2 AR
-          const double ck = cdisp * (double)(kx * kx + ky * ky);
-          const double2 fr = which == 1 ? cadd(tnd, cscale(x3, ck)) : csub(tnd, cscale(x3, ck));
-          if (eul) xn = cscale(csub(xo, cscale(fr, dt)), e1);
-          else xn = csub(cscale(xo, e2), cscale(cscale(fr, dt2), e1));
+          xn = csub(cscale(xo, e2), cscale(fr, dt2 * e1));
+          if (which == 0 && sp.use_dq) xn = cadd(xn, cscale(x3, dt2 * e2));
+          // Robert-Asselin filter (main_waqg.f90:395-410)
+          xf = cadd(x0, cscale(cadd(csub(xo, cscale(x0, 2.0)), xn), gam));
         }
-        // Robert-Asselin filter (main_waqg.f90:395-410)
-        if (!eul) xf = cadd(x0, cscale(cadd(csub(xo, cscale(x0, 2.0)), xn), gam));
       }
       X[m] = xn;
       Xo[m] = xf;
@@ -305,38 +383,6 @@ k_fx_col_update(Geom g, StepParams sp, int zbase, StateP<double> st, const doubl
         (which == 2 ? st.sig1 : st.sig2)[m] = sv;
       }
     }
-  }
-  if (!qw_prep) return;
-  __syncthreads();
-  // y-inverse transforms of B and i ky B at n+1 (compute_qw,
-  // derivatives.f90:929-957) from this CTA's own stores: planes (BR, i ky BR,
-  // BI, i ky BI) = 0..3, BR and BI to the kept planes when given
-  for (int p = 0; p < 4; ++p) {
-    const double2* X = (p >> 1) == 0 ? st.BR : st.BI;
-    double2 d[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      d[r] = make_double2(0.0, 0.0);
-      if (fx_zero_in<8>(r)) continue;
-      int row; bool cj;
-      col_src(g, kx, c.j + r * NB, row, cj);
-      if (row < 0) continue;
-      double2 x = X[zoff + (long long)row * g.KXP + kx];
-      if (p & 1) { const double ky = (double)g.ky_of_row(row); x = make_double2(-ky * x.y, ky * x.x); }
-      if (cj) x.y = -x.y;
-      d[r] = x;
-    }
-    fxc v[8];
-    int base;
-    c.template run<false>(d, v, base);
-    if (kx > g.K) continue;
-    double2 o[8];
-    fx_doubles<8, true>(v, o, base);
-    double2* dst = (Qb && (p & 1) == 0) ? Qb + q_off(zb, p >> 1, 0, N, g.KXP) : S + scr_off(zb, p, 0, N, g.KXP);
-    dst += (long long)c.j * g.KXP + kx;
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-      dst[(long long)r * NB * g.KXP] = o[r];
   }
 }
 
@@ -355,8 +401,14 @@ k_fx_col_qw(Geom g, StepParams sp, int zbase, const double2* __restrict__ q, dou
   const int mem = sp.mpar ? z / g.nseg : 0;          // ensemble member of this level (stacks)
   const double s = sp.mpar ? sp.mpar[4 * mem + 2] * sp.mpar[4 * mem + 3] : sp.Ro * sp.W2F;
   double2 A[8], B[8];
-  fx_col_plane<N>(c, g, S + scr_off(zb, 0, 0, N, g.KXP), kx, A);
-  fx_col_plane<N>(c, g, S + scr_off(zb, 1, 0, N, g.KXP), kx, B);
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    if (h == 1) {
+#pragma unroll
+      for (int r = 0; r < 8; ++r) A[r] = B[r];
+    }
+    fx_col_plane<N>(c, g, S + scr_off(zb, h, 0, N, g.KXP), kx, B);
+  }
   bool bad = false;       // a non-finite q* (the state has blown up)
   if (kx <= g.K) {
 #pragma unroll
