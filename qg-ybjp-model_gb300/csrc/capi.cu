@@ -165,7 +165,7 @@ int build_tables(const qg_config& c, qg::HostTables& t, std::string& err) {
   t.fac_psi.assign((size_t)nd * n3 * 4, 0.0);
   t.fac_A.assign((size_t)nd * n3 * 4, 0.0);
   std::vector<double> d(n3), dl(n3), du(n3);
-  // FP64 path: {f_i, d'_i, 0, 0} for DGTSV's exact arithmetic;
+  // FP64 path: {f_i, d'_i, 1/d'_i, 0} for DGTSV's arithmetic (div_by);
   // mixed path: {f_i, s/d'_i, u_i/d'_i, 0} with s the RHS scaling of the operator
   const bool exact = c.precision == QG_PREC_FP64;
   for (auto& kv : idx) {
@@ -197,13 +197,13 @@ int build_tables(const qg_config& c, qg::HostTables& t, std::string& err) {
         const double f = dl[i] / dp;
         out[4 * i] = f;
         out[4 * i + 1] = exact ? dp : s / dp;
-        out[4 * i + 2] = exact ? 0.0 : du[i] / dp;
+        out[4 * i + 2] = exact ? 1.0 / dp : du[i] / dp;
         dp = d[i + 1] - f * du[i];
       }
       if (dp == 0.0 || !std::isfinite(dp)) { err = "zero pivot in tridiagonal factorisation"; return QG_ERR_PIVOT; }
       out[4 * (n3 - 1)] = 0.0;
       out[4 * (n3 - 1) + 1] = exact ? dp : s / dp;
-      out[4 * (n3 - 1) + 2] = 0.0;
+      out[4 * (n3 - 1) + 2] = exact ? 1.0 / dp : 0.0;
     }
   }
   return QG_OK;

@@ -222,9 +222,9 @@ class Engine : public EngineBase {
       vbuf = nullptr;
       (void)cudaGetLastError();
     }
-    // mixed path: per-column copies of the solve factors (coalesced reads);
+    // per-column copies of the solve factors (coalesced reads);
     // without them the solves read the per-kh^2 tables
-    if (kSolvePerColumn && sizeof(T) == 4 && vbuf) {
+    if (kSolvePerColumn && vbuf) {
       if (cudaMalloc(&pcfac, (size_t)6 * g.nseg * nret * sizeof(double)) != cudaSuccess) {
         pcfac = nullptr;
         (void)cudaGetLastError();
@@ -724,7 +724,7 @@ class Engine : public EngineBase {
     int rc = ensure_tmp();
     if (rc) return rc;
     if ((rc = upload_compact(qstar, tmpF[0]))) return rc;
-    if ((rc = solve_generic(tmpF[0], nullptr, nullptr, tmpF[1], nullptr, nullptr, 1, 0))) return rc;
+    if ((rc = solve_generic(tmpF[0], nullptr, nullptr, tmpF[1], nullptr, nullptr, 1, 0, nullptr, 0, -1, true))) return rc;
     return download_compact(tmpF[1], psik, 0);
   }
 
@@ -732,7 +732,7 @@ class Engine : public EngineBase {
     int rc = ensure_tmp();
     if (rc) return rc;
     if ((rc = upload_compact(bk, tmpF[0]))) return rc;
-    if ((rc = solve_generic(nullptr, tmpF[0], tmpF[0], nullptr, tmpF[1], tmpF[2], 0, 1))) return rc;
+    if ((rc = solve_generic(nullptr, tmpF[0], nullptr, nullptr, tmpF[1], nullptr, 0, 2, nullptr, 0, -1, true))) return rc;
     if ((rc = download_compact(tmpF[1], ak, 0))) return rc;
     if (ck) return download_compact(tmpF[1], ck, 1);
     return QG_OK;
@@ -978,18 +978,32 @@ class Engine : public EngineBase {
     else return Tiles<T, NN>::CT;
   }
 
+  // whether a grid of n CTAs, per_sm of them resident on an SM, is at most
+  // `waves` waves: k_fx_col_inv then spreads a tile's fields over several CTAs
+  // (a shorter chain per CTA and more of the GPU at work) instead of looping
+  // over them (one table load per tile).  us per launch, looped -> spread:
+  // 64^2 x 64 22.5 -> 14.0, 128^2 x 64 36.7 -> 29.0, 256^2 x 128 (2.6 waves)
+  // 144 -> 147.  (The FP32 kernels are not spread: k_col_update 64^2 x 32 17.9
+  // -> 13.8, but the compiler then fuses other products with additions and the
+  // fields differ in their last bits from those of larger grids.)
+  bool few_ctas(long long n, int waves, int per_sm) const { return n <= (long long)waves * per_sm * nsm; }
+
   // k_col_inv on levels [z0, z0 + zc): mode 0 all six fields into Sb, 1 the
   // first four (BR, BI are kept in Qb), 2 BR and BI into Qb
   template <int NN>
   void launch_col_inv(int z0, int zc, const C* psi, const C* q, const C* br, const C* bi, C* Sb, C* Qb, int mode,
                       cudaStream_t on) {
     // column tiles up to kx = K (the padding columns beyond K are never read)
-    const dim3 gc((g.K + col_ct<NN>()) / col_ct<NN>(), zc);
-    if constexpr (kFx)
-      k_fx_col_inv<NN><<<gc, FxCol<NN>::NT, FxCol<NN>::smem(), on>>>(g, z0, psi, q, br, bi, Sb, tw, Qb,
-                                                                     mode == 2 ? 4 : 0, mode == 1 ? 4 : 6);
-    else
-      k_col_inv<T, NN><<<gc, Tiles<T, NN>::CNT, sm_ci<NN, Tiles<T, NN>::CIP>(Tiles<T, NN>::CINF), on>>>(
+    const int tiles = (g.K + col_ct<NN>()) / col_ct<NN>();
+    if constexpr (kFx) {
+      const int f0 = mode == 2 ? 4 : 0, f1 = mode == 1 ? 4 : 6;
+      const int split = few_ctas((long long)tiles * zc, 1, fx_col_ctas<NN>(QG_FX_COL_CTAS)) ? f1 - f0 : 1;
+      k_fx_col_inv<NN><<<dim3(tiles * split, zc), FxCol<NN>::NT, FxCol<NN>::smem(), on>>>(g, z0, psi, q, br, bi, Sb, tw,
+                                                                                          Qb, f0, f1, split);
+      return;
+    }
+    if constexpr (!kFx)
+      k_col_inv<T, NN><<<dim3(tiles, zc), Tiles<T, NN>::CNT, sm_ci<NN, Tiles<T, NN>::CIP>(Tiles<T, NN>::CINF), on>>>(
           g, z0, psi, q, br, bi, Sb, tw, Qb, mode);
   }
 
@@ -1056,7 +1070,7 @@ class Engine : public EngineBase {
         }
         if (int rc0 = pbeg(QG_K_COL_UPDATE, bs)) return rc0;
         if constexpr (kFx)
-          k_fx_col_update<NN><<<gc, FxCol<NN>::NT, FxCol<NN>::smem(), bs>>>(g, s, z0, sptr, e1, e2, e1w, e2w, Sb, tw,
+          k_fx_col_update<NN><<<dim3(gc.x, gc.y, 3), FxCol<NN>::NT, FxCol<NN>::smem(), bs>>>(g, s, z0, sptr, e1, e2, e1w, e2w, Sb, tw,
                                                                            need_qw ? 1 : 0, Qb);
         else
           k_col_update<T, NN><<<gc, Tiles<T, NN>::CNT, UpdLay<T, NN>::bytes(), bs>>>(g, s, z0, sptr, e1, e2, e1w, e2w, Sb, tw,
@@ -1136,19 +1150,26 @@ class Engine : public EngineBase {
     const int ncl = retained ? nret : (int)g.plane;
     double* const pcf = retained ? pcfac : nullptr;     // the per-column factors follow the retained list
     if (kSolveStore && vbuf) {
-      const int nrec = (do_psi ? 2 : 0) + (do_A ? 4 : 0);   // recurrences per column
-#define QG_SOLVE_ST(TCV, PCV)                                                                              \
-  k_solve_st<T, TCV, PCV><<<dim3((unsigned)((ncl + TCV - 1) / TCV), nsegs), nrec * TCV,                 \
-                            (size_t)g.nseg * 8, on>>>(                                                     \
+      const int nrec = (do_psi ? 2 : 0) + (do_A == 1 ? 4 : do_A);   // recurrences per column
+      // A launch of few columns spreads their recurrences over CTAs of one
+      // warp, so that more SMs' FP64 pipes (2 lanes per clock) work on them,
+      // and reads longer segments ahead
+      const bool few = few_ctas((long long)((ncl + 31) / 32) * nsegs * nrec, 1, 12);
+      const int zs = few ? nrec : 1;
+#define QG_SOLVE_ST(TCV, PCV, SV)                                                                            \
+  k_solve_st<T, TCV, PCV, SV><<<dim3((unsigned)((ncl + TCV - 1) / TCV), nsegs, zs), nrec / zs * TCV,        \
+                                (size_t)g.nseg * 8, on>>>(                                                   \
       g, cfg.dz, cfg.Bu, tab_idx, fac_psi, fac_A, du, qs, br, bi, psi, ar, ai, do_psi, do_A, vbuf, pcf, seg0, cl, ncl)
       if (pcf) {
-        if (solve_tc == 16) QG_SOLVE_ST(16, true);
-        else if (solve_tc == 64) QG_SOLVE_ST(64, true);
-        else QG_SOLVE_ST(32, true);
+        if (few) QG_SOLVE_ST(32, true, kSegFew);
+        else if (solve_tc == 16) QG_SOLVE_ST(16, true, kSegSt);
+        else if (solve_tc == 64) QG_SOLVE_ST(64, true, kSegSt);
+        else QG_SOLVE_ST(32, true, kSegSt);
       } else {
-        if (solve_tc == 16) QG_SOLVE_ST(16, false);
-        else if (solve_tc == 64) QG_SOLVE_ST(64, false);
-        else QG_SOLVE_ST(32, false);
+        if (few) QG_SOLVE_ST(32, false, kSegFew);
+        else if (solve_tc == 16) QG_SOLVE_ST(16, false, kSegSt);
+        else if (solve_tc == 64) QG_SOLVE_ST(64, false, kSegSt);
+        else QG_SOLVE_ST(32, false, kSegSt);
       }
 #undef QG_SOLVE_ST
       QG_LAUNCHED();

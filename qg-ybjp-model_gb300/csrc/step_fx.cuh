@@ -133,8 +133,8 @@ k_fx_row_qw(Geom g, double2* __restrict__ S, const double2* __restrict__ twg, in
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const int zb = it / NG, y = (it % NG) * F::RT + c.rr;
     auto plane = [&](int f) -> double2* { return S + scr_off(zb, f, y, N, g.KXP); };
-    const double2* pr = Qb ? Qb + q_off(zb, 0, y, N, g.KXP) : plane(0);
-    const double2* pi = Qb ? Qb + q_off(zb, 1, y, N, g.KXP) : plane(2);
+    const double2* pr = Qb ? Qb + q_off(zb, 0, y, N, g.KXP) : plane(2);
+    const double2* pi = Qb ? Qb + q_off(zb, 1, y, N, g.KXP) : plane(4);
     // inverse transforms of (BRx, BIx), (BRy, BIy), (BR, BI), then the forward
     // transform of (P1, P2), through one copy of the transform
     fxc a[8], p[8], w[8];
@@ -143,7 +143,7 @@ k_fx_row_qw(Geom g, double2* __restrict__ S, const double2* __restrict__ twg, in
     for (int t = 0; t < 4; ++t) {
       if (t < 3) {
         double2 d[8];
-        fx_pack<N>(t == 1 ? plane(1) : pr, t == 1 ? plane(3) : pi, j, K, d);
+        fx_pack<N>(t == 1 ? plane(3) : pr, t == 1 ? plane(5) : pi, j, K, d);
         if (t == 0) {
           // i kx times the packed spectrum of (BR, BI)
 #pragma unroll
@@ -181,8 +181,8 @@ k_fx_row_qw(Geom g, double2* __restrict__ S, const double2* __restrict__ twg, in
       } else {
         c.template split<3>(w, base, K, [&](int, int k, double2 P1, double2 P2) {
           const double qk = 0.25 * (double)(k * k);
-          plane(0)[k] = make_double2(P1.x - qk * P2.x, P1.y - qk * P2.y);
-          plane(1)[k] = P2;
+          plane(3)[k] = make_double2(P1.x - qk * P2.x, P1.y - qk * P2.y);
+          plane(5)[k] = P2;
         });
       }
     }
@@ -198,21 +198,22 @@ k_fx_row_qw(Geom g, double2* __restrict__ S, const double2* __restrict__ twg, in
 template <int N> __host__ __device__ constexpr int fx_col_ctas(int want) { return imin(32, (want * 128) / FxCol<N>::NT); }
 
 // y-inverse transforms of the fields f in [f0, f1) of (u, v, zeta, q, BR, BI)
-// into the planes f of S; BR, BI into the kept planes Qb when given
+// into the planes f of S; BR, BI into the kept planes Qb when given; a tile's
+// fields over `split` CTAs
 template <int N>
 __global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(QG_FX_COL_CTAS))
 k_fx_col_inv(Geom g, int zbase, const double2* __restrict__ psi, const double2* __restrict__ q,
              const double2* __restrict__ BR, const double2* __restrict__ BI, double2* __restrict__ S,
-             const double2* __restrict__ twg, double2* __restrict__ Qb, int f0, int f1) {
+             const double2* __restrict__ twg, double2* __restrict__ Qb, int f0, int f1, int split) {
   using F = FxCol<N>;
   constexpr int NB = F::NB;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned slots[F::SLOTS];
   const FxColCtx<N> c = fx_col_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
-  const int zb = blockIdx.y, kx = blockIdx.x * F::CT + c.c;
+  const int zb = blockIdx.y, kx = (int)(blockIdx.x / split) * F::CT + c.c;
   const long long zoff = (long long)(zbase + zb) * g.plane;
 #pragma unroll 1
-  for (int f = f0; f < f1; ++f) {
+  for (int f = f0 + (int)blockIdx.x % split; f < f1; f += split) {
     const double2* X = f < 3 ? psi : (f == 3 ? q : (f == 4 ? BR : BI));
     double2 d[8];
 #pragma unroll
@@ -285,25 +286,27 @@ k_fx_col_update(Geom g, StepParams sp, int zbase, StateP<double> st, const doubl
   const double cdisp = sp.disp ? (sp.mpar ? sp.mpar[4 * mem + 1] : sp.cdisp) : 0.0;
   const double gam = sp.gamma, dt2 = 2.0 * dt;
   const bool eul = sp.euler != 0;
-  // H and G of q, BR, BI, then the y-inverse transforms of B and i ky B at n+1
-  // (compute_qw, derivatives.f90:929-957: planes BR, i ky BR, BI, i ky BI =
-  // 0..3, BR and BI to the kept planes when given), through one copy of the
-  // transform
+  // H and G of one of q, BR, BI, then the y-inverse transforms of B and i ky B
+  // at n+1 (compute_qw, derivatives.f90:929-957: planes BR, i ky BR, BI,
+  // i ky BI = 2..5, which this CTA alone has read, BR and BI to the kept
+  // planes when given), through one copy of the transform
   double2 H[8];
-  const int nt = qw_prep ? 10 : 6;
+  // (a CTA per variable: the chain of the ten transforms of a tile bounded
+  // small grids, 65.5 -> 32.8 us at 64^2 x 64; 512^2 x 256 the same)
+  const int which = blockIdx.z, nt = qw_prep && which ? 4 : 2;
 #pragma unroll 1
   for (int t = 0; t < nt; ++t) {
     double2 d[8];
     fxc v[8];
     int base;
-    if (t < 6) {
-      const double2* p = S + scr_off(zb, t ^ 1, 0, N, g.KXP) + (long long)c.j * g.KXP + kx;
+    if (t < 2) {
+      const double2* p = S + scr_off(zb, 2 * which + 1 - t, 0, N, g.KXP) + (long long)c.j * g.KXP + kx;
 #pragma unroll
       for (int r = 0; r < 8; ++r) d[r] = kx <= g.K ? p[(long long)r * NB * g.KXP] : make_double2(0.0, 0.0);
       base = c.template load<true>(d, v);
     } else {
-      if (t == 6) __syncthreads();      // B^{n+1}: this CTA's own stores
-      const double2* X = t < 8 ? st.BR : st.BI;
+      if (t == 2) __syncthreads();      // B^{n+1}: this CTA's own stores
+      const double2* X = which == 1 ? st.BR : st.BI;
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
         d[r] = make_double2(0.0, 0.0);
@@ -320,22 +323,20 @@ k_fx_col_update(Geom g, StepParams sp, int zbase, StateP<double> st, const doubl
     }
     c.core(v, base);
     if (kx > g.K) continue;
-    if (t >= 6) {
+    if (t >= 2) {
       fx_doubles<8, true>(v, d, base);
-      const int p = t - 6;
-      double2* dst = (Qb && (p & 1) == 0) ? Qb + q_off(zb, p >> 1, 0, N, g.KXP) : S + scr_off(zb, p, 0, N, g.KXP);
+      double2* dst = (Qb && t == 2) ? Qb + q_off(zb, which - 1, 0, N, g.KXP) : S + scr_off(zb, 2 * which + t - 2, 0, N, g.KXP);
       dst += (long long)c.j * g.KXP + kx;
 #pragma unroll
       for (int r = 0; r < 8; ++r) dst[(long long)r * NB * g.KXP] = d[r];
       continue;
     }
     fx_doubles<8, false>(v, d, base - 2 * fx_ilog2(N));     // (d[3], d[4] are not used)
-    if ((t & 1) == 0) {
+    if (t == 0) {
 #pragma unroll
       for (int r = 0; r < 8; ++r) H[r] = d[r];
       continue;
     }
-    const int which = t >> 1;
     double2* X = which == 0 ? st.q : (which == 1 ? st.BR : st.BI);
     double2* Xo = which == 0 ? st.qo : (which == 1 ? st.BRo : st.BIo);
     const double2* X3 = which == 0 ? st.dq : (which == 1 ? st.AI : st.AR);
@@ -407,7 +408,7 @@ k_fx_col_qw(Geom g, StepParams sp, int zbase, const double2* __restrict__ q, dou
 #pragma unroll
       for (int r = 0; r < 8; ++r) A[r] = B[r];
     }
-    fx_col_plane<N>(c, g, S + scr_off(zb, h, 0, N, g.KXP), kx, B);
+    fx_col_plane<N>(c, g, S + scr_off(zb, 3 + 2 * h, 0, N, g.KXP), kx, B);
   }
   bool bad = false;       // a non-finite q* (the state has blown up)
   if (kx <= g.K) {
