@@ -191,7 +191,7 @@ class AdjEngine final : public Engine<double> {
       err = "the adjoint needs fixed_flow = 0 and passive_scalar = 0";
       return QG_ERR_UNSUPPORTED;
     }
-    int rc = prep_dense(g.n3);
+    int rc = prep_dense(g.n3, kDensePlanes);
     if (rc) return rc;
     for (auto& p : Sb) if ((rc = grab(&p, spec_bytes(), true))) return rc;
     for (auto& p : Pb) if ((rc = grab(&p, (size_t)totP() * sizeof(double), true))) return rc;
@@ -246,20 +246,20 @@ class AdjEngine final : public Engine<double> {
     const long long tot = (long long)g.n3 * g.plane;
     const C* qs = F[F_Q];
     if (need_qw) {
-      k_compact_to_dense<double><<<grid_for(totS()), 256, 0, st>>>(g, 0, g.n3, F[F_BR], Sb[0], 0, cfg.dz);
+      k_compact_to_dense<double><<<conv_grid(g.n, g.n3), 256, 0, st>>>(g, 0, F[F_BR], Sb[0], 0, Divisor(cfg.dz));
       QG_LAUNCHED();
-      k_compact_to_dense<double><<<grid_for(totS()), 256, 0, st>>>(g, 0, g.n3, F[F_BI], Sb[1], 0, cfg.dz);
+      k_compact_to_dense<double><<<conv_grid(g.n, g.n3), 256, 0, st>>>(g, 0, F[F_BI], Sb[1], 0, Divisor(cfg.dz));
       QG_LAUNCHED();
       if ((rc = compute_qw(reinterpret_cast<const double*>(Sb[0]), reinterpret_cast<const double*>(Sb[1]),
                            reinterpret_cast<double*>(Sb[2]), g.n3)))
         return rc;
-      k_dense_to_compact<double><<<grid_for(tot), 256, 0, st>>>(g, 0, g.n3, Sb[2], Af[A_QW]);
+      k_dense_to_compact<double><<<conv_grid(g.KY, g.n3), 256, 0, st>>>(g, 0, Sb[2], Af[A_QW]);
       QG_LAUNCHED();
       k_adj_sum<<<grid_for(tot), 256, 0, st>>>(g, tot, F[F_Q], Af[A_QW], -1.0, Af[A_QSTAR]);
       QG_LAUNCHED();
       qs = Af[A_QSTAR];
     }
-    return solve_generic(qs, F[F_BR], F[F_BI], F[F_PSI], F[F_AR], F[F_AI], 1, 1);
+    return solve_generic(qs, F[F_BR], F[F_BI], F[F_PSI], F[F_AR], F[F_AI], 1, 1, nullptr, 0, -1, true);
   }
 
   // ---- the objective (reference layout) -------------------------------------
@@ -278,7 +278,7 @@ class AdjEngine final : public Engine<double> {
   }
   // C^T y = w_k F(y) on the retained modes
   int CTf(const double* y, double2* out) {
-    int rc = d_r2c(y, Sb[6], g.n3);
+    int rc = d_r2c(y, g.n, Sb[6], g.n3);
     if (rc) return rc;
     k_ct_weights<<<grid_for(totS()), 256, 0, st>>>(g.n, g.kmax2, totS(), (double)g.n * g.n, Sb[6], 0, out);
     QG_LAUNCHED();
@@ -286,11 +286,11 @@ class AdjEngine final : public Engine<double> {
   }
   // A_solver on a dense field
   int A_inv(const double2* in, double2* out) {
-    k_dense_to_compact<double><<<grid_for((long long)g.n3 * g.plane), 256, 0, st>>>(g, 0, g.n3, in, tmpC[0]);
+    k_dense_to_compact<double><<<conv_grid(g.KY, g.n3), 256, 0, st>>>(g, 0, in, tmpC[0]);
     QG_LAUNCHED();
-    int rc = solve_generic(nullptr, tmpC[0], tmpC[0], nullptr, tmpC[1], tmpC[2], 0, 1);
+    int rc = solve_generic(nullptr, tmpC[0], nullptr, nullptr, tmpC[1], nullptr, 0, 2, nullptr, 0, -1, true);
     if (rc) return rc;
-    k_compact_to_dense<double><<<grid_for(totS()), 256, 0, st>>>(g, 0, g.n3, tmpC[1], out, 0, cfg.dz);
+    k_compact_to_dense<double><<<conv_grid(g.n, g.n3), 256, 0, st>>>(g, 0, tmpC[1], out, 0, Divisor(cfg.dz));
     QG_LAUNCHED();
     return QG_OK;
   }
@@ -308,13 +308,13 @@ class AdjEngine final : public Engine<double> {
     const double k4 = 0.25 / cfg.Bu;
     const int src[4] = {F_BR, F_BI, F_AR, F_AI};
     for (int i = 0; i < 4; ++i) {
-      k_compact_to_dense<double><<<grid_for(totS()), 256, 0, st>>>(g, 0, g.n3, F[src[i]], Sb[i], 0, cfg.dz);
+      k_compact_to_dense<double><<<conv_grid(g.n, g.n3), 256, 0, st>>>(g, 0, F[src[i]], Sb[i], 0, Divisor(cfg.dz));
       QG_LAUNCHED();
     }
     // Sb[4], Sb[5]: LA of the real and imaginary parts
     if ((rc = lin(Sb[4], 0, {term(Sb[0], 1, 0, 0), term(Sb[2], k4, 0, 3)})) ||
-        (rc = lin(Sb[5], 0, {term(Sb[1], 1, 0, 0), term(Sb[3], k4, 0, 3)})) || (rc = d_c2r(Sb[4], Pb[0], g.n3)) ||
-        (rc = d_c2r(Sb[5], Pb[1], g.n3)))
+        (rc = lin(Sb[5], 0, {term(Sb[1], 1, 0, 0), term(Sb[3], k4, 0, 3)})) || (rc = d_c2r(Sb[4], Pb[0], g.n, g.n3)) ||
+        (rc = d_c2r(Sb[5], Pb[1], g.n, g.n3)))
       return rc;
     const int z0 = obj_first_level();
     k_obj_partial<<<kObjBlocks, 256, 0, st>>>(g.n, g.n3, z0, Pb[0], Pb[1], part);
@@ -333,7 +333,7 @@ class AdjEngine final : public Engine<double> {
       if ((rc = CTf(Pb[c], Sb[0])) || (rc = lin(Sb[1], 0, {term(Sb[0], k4, 0, 3)})) || (rc = A_inv(Sb[1], Sb[2])) ||
           (rc = lin(Sb[3], 0, {term(Sb[0], 1, 0, 0), term(Sb[2], 1, 0, 0)})))
         return rc;
-      k_dense_to_compact<double><<<grid_for((long long)g.n3 * g.plane), 256, 0, st>>>(g, 0, g.n3, Sb[3],
+      k_dense_to_compact<double><<<conv_grid(g.KY, g.n3), 256, 0, st>>>(g, 0, Sb[3],
                                                                                     lamA[2 + c]);
       QG_LAUNCHED();
     }
@@ -377,7 +377,8 @@ class AdjEngine final : public Engine<double> {
         QG_LAUNCHED();
       });
     }
-    int rc = solve_generic(Af[A_LPSI], Af[A_LAR], Af[A_LAI], Af[A_W], Af[A_LBRA], Af[A_LBIA], 1, 1);
+    int rc = solve_generic(Af[A_LPSI], Af[A_LAR], Af[A_LAI], Af[A_W], Af[A_LBRA], Af[A_LBIA], 1, 1, nullptr, 0, -1,
+                           true);
     if (rc) return rc;
     const long long tot = (long long)g.n3 * g.plane;
     k_adj_solved<<<grid_for(tot), 256, 0, st>>>(g, tot, lo[0], lo[2], lo[3], Af[A_W], Af[A_LBRA], Af[A_LBIA]);

@@ -3,6 +3,8 @@
 // precision: FP64 only in the tridiagonal solves and the diagnostics) or
 // T = double (FP64 everywhere).
 #pragma once
+#include <cuda.h>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <cmath>
@@ -125,6 +127,19 @@ class Engine : public EngineBase {
       QG_CK(cudaMemcpy(cols_all, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice));
       QG_CK(cudaMalloc(&cols_ret, ret.size() * sizeof(int)));
       QG_CK(cudaMemcpy(cols_ret, ret.data(), ret.size() * sizeof(int), cudaMemcpyHostToDevice));
+    }
+    {
+      std::vector<int> k2(t.ndistinct);
+      for (long long m = 0; m < g.plane; ++m)
+        if (t.tab_idx[m] >= 0) {
+          const int kx = (int)(m % g.KXP), ky = g.ky_of_row((int)(m / g.KXP));
+          k2[t.tab_idx[m]] = kx * kx + ky * ky;
+        }
+      om_nd = t.ndistinct;
+      if (om_nd) {
+        QG_CK(cudaMalloc(&om_kh2, om_nd * sizeof(int)));
+        QG_CK(cudaMemcpy(om_kh2, k2.data(), om_nd * sizeof(int), cudaMemcpyHostToDevice));
+      }
     }
     const size_t fb = std::max<size_t>(1, (size_t)t.ndistinct * g.nseg) * sizeof(double4);
     QG_CK(cudaMalloc(&fac_psi, fb));
@@ -334,7 +349,8 @@ class Engine : public EngineBase {
       // the FP32 field is rounded from that copy on the device, so the input
       // crosses the host link once
       if (!psi64) QG_CK(cudaMalloc(&psi64, (size_t)g.n3 * g.plane * sizeof(double2)));
-      k_dense_to_compact<double><<<grid_for((long long)nlev * g.plane), 256, 0, st>>>(g, level0, nlev, src, psi64,
+      psi64_live = true;
+      k_dense_to_compact<double><<<conv_grid(g.KY, nlev), 256, 0, st>>>(g, level0, src, psi64,
                                                                                         iflag);
       QG_LAUNCHED();
       k_round_compact<T><<<grid_for((long long)nlev * g.plane), 256, 0, st>>>(
@@ -342,7 +358,7 @@ class Engine : public EngineBase {
           F[f] + (size_t)level0 * g.plane);
       QG_LAUNCHED();
     } else {
-      k_dense_to_compact<T><<<grid_for((long long)nlev * g.plane), 256, 0, st>>>(g, level0, nlev, src, F[f], iflag);
+      k_dense_to_compact<T><<<conv_grid(g.KY, nlev), 256, 0, st>>>(g, level0, src, F[f], iflag);
       QG_LAUNCHED();
     }
     QG_CK(cudaStreamSynchronize(st));
@@ -366,8 +382,8 @@ class Engine : public EngineBase {
       int rc = ensure(&stage, &stage_bytes, bytes);
       if (rc) return rc;
     }
-    k_compact_to_dense<T><<<grid_for((long long)nlev * g.n * (g.n / 2 + 1)), 256, 0, st>>>(
-        g, level0, nlev, F[f], dst ? dst : (double2*)stage, mode, cfg.dz);
+    k_compact_to_dense<T><<<conv_grid(g.n, nlev), 256, 0, st>>>(g, level0, F[f], dst ? dst : (double2*)stage, mode,
+                                                                Divisor(cfg.dz));
     QG_LAUNCHED();
     if (!dst) QG_CK(cudaMemcpyAsync(kvar, stage, bytes, cudaMemcpyDefault, st));
     QG_CK(cudaStreamSynchronize(st));
@@ -402,7 +418,7 @@ class Engine : public EngineBase {
     }
     q_valid = false;
     if (apply_sumB) {
-      k_sumB<T><<<(unsigned)((g.plane + 127) / 128), 128, 0, st>>>(g, F[F_BR], F[F_BI], z0, z0 + nz);
+      k_sumB<T><<<dim3((unsigned)((g.plane + 127) / 128), 2), 128, 0, st>>>(g, F[F_BR], F[F_BI], z0, z0 + nz);
       QG_LAUNCHED();
     }
     const size_t lb = (size_t)g.plane * sizeof(C), off = (size_t)z0 * g.plane;
@@ -410,12 +426,12 @@ class Engine : public EngineBase {
       // fixed flow: q = 0 for all times (main_waqg.f90:141-146)
       QG_CK(cudaMemsetAsync(F[F_Q] + off, 0, (size_t)nz * lb, st));
     } else if (q_from_psi) {
-      if (psi64) {
-        k_init_q<T, double><<<grid_for((long long)nz * g.plane), 256, 0, st>>>(g, cfg.dz, cu, cl, psi64, F[F_Q], z0,
-                                                                               z0 + nz);
+      const Divisor dz2(cfg.dz * cfg.dz);
+      const dim3 gi((unsigned)((g.plane + 127) / 128), (g.nseg + kInitLev - 1) / kInitLev * (nz / g.nseg));
+      if (psi64_live) {
+        k_init_q<T, double><<<gi, 128, 0, st>>>(g, cfg.dz, dz2, cu, cl, psi64, F[F_Q], z0);
       } else {
-        k_init_q<T, T><<<grid_for((long long)nz * g.plane), 256, 0, st>>>(g, cfg.dz, cu, cl, F[F_PSI], F[F_Q], z0,
-                                                                          z0 + nz);
+        k_init_q<T, T><<<gi, 128, 0, st>>>(g, cfg.dz, dz2, cu, cl, F[F_PSI], F[F_Q], z0);
       }
       QG_LAUNCHED();
     }
@@ -431,10 +447,9 @@ class Engine : public EngineBase {
     return QG_OK;
   }
 
-  // the FP64 copy of psi that qg_set_state keeps for init_q (mixed path)
-  void release_init_buffers() override {
-    if (psi64) { cudaStreamSynchronize(st); cudaFree(psi64); psi64 = nullptr; }
-  }
+  // the FP64 copy of psi that qg_set_state keeps for init_q (mixed path) is
+  // used up; its memory stays for the handle's next run
+  void release_init_buffers() override { psi64_live = false; }
 
   // ---- the step -------------------------------------------------------------
   int step(int euler) override {
@@ -531,193 +546,163 @@ class Engine : public EngineBase {
   // ---- output path ----------------------------------------------------------
   int dump_real(int which, float* out0, float* out1, int level0, int nlev, double s1, double s2) override {
     if (level0 < 0 || nlev <= 0 || level0 + nlev > g.n3) { err = "bad level range"; return QG_ERR_ARG; }
-    int rc = prep_dense(nlev);
+    int rc = prep_dense(nlev, kDensePlanes);
     if (rc) return rc;
-    const long long tot = (long long)nlev * g.n * (g.n / 2 + 1), np = (long long)nlev * g.n * g.n;
-    float* o32 = reinterpret_cast<float*>(dstage);        // nlev*n*(n+2) doubles hold nlev*n*n floats
+    const size_t bytes = (size_t)nlev * g.n * g.n * sizeof(float);
     const int nf = which == 0 ? 1 : 2;
+    CompactIn<T> in{g, level0, {which == 0 ? F[F_PSI] : F[F_BR], F[F_BI]},
+                    {which == 2 ? F[F_AR] : nullptr, which == 2 ? F[F_AI] : nullptr}, Divisor(cfg.Bu)};
+    F32Out o{{nullptr, nullptr}, s1, s2};
+    float* out[2] = {out0, out1};
     for (int c = 0; c < nf; ++c) {
-      const C* src = which == 0 ? F[F_PSI] : (c == 0 ? F[F_BR] : F[F_BI]);
-      k_compact_to_dense<T><<<grid_for(tot), 256, 0, st>>>(g, level0, nlev, src, D[0], 0, cfg.dz);
-      QG_LAUNCHED();
-      const double2* spec = D[0];
-      if (which == 2) {
-        k_compact_to_dense<T><<<grid_for(tot), 256, 0, st>>>(g, level0, nlev, c == 0 ? F[F_AR] : F[F_AI], D[1], 0,
-                                                            cfg.dz);
-        QG_LAUNCHED();
-        k_dense_la<<<grid_for(tot), 256, 0, st>>>(g.n, g.kmax2, tot, D[0], D[1], cfg.Bu, D[2]);
-        QG_LAUNCHED();
-        spec = D[2];
-      }
-      if ((rc = d_c2r(spec, P[0], nlev))) return rc;
-      k_phys_f32<T><<<grid_for(np), 256, 0, st>>>(np, P[0], s1, s2, o32);
-      QG_LAUNCHED();
-      QG_CK(cudaMemcpyAsync(c == 0 ? out0 : out1, o32, (size_t)np * sizeof(float), cudaMemcpyDefault, st));
-      QG_CK(cudaStreamSynchronize(st));
+      void* v;
+      if ((rc = out_view(out[c], bytes, c, &v))) return rc;
+      o.o[c] = static_cast<float*>(v);
     }
+    if ((rc = d_inv(in, nlev, nf, g.K))) return rc;
+    QG_SWITCH_N(g.n, {
+      using DN = Dense<T, NN>;
+      k_drow_c2r_f32<T, NN><<<dim3(g.n / 2 / DN::RT, nlev, nf), DN::RNT, DN::sm_row(), st>>>(iktxP(), nf, g.K, W, o, tw);
+      QG_LAUNCHED();
+    });
+    for (int c = 0; c < nf; ++c)
+      if ((rc = out_copy(out[c], o.o[c], bytes))) return rc;
+    QG_CK(cudaStreamSynchronize(st));
     return QG_OK;
   }
 
   // ---- omega equation (the vertical-velocity diagnostic) ---------------------
-  // right-hand side from the dense psi in D[0] into D[5]
-  int omega_rhs_dev() {
-    const long long tot = (long long)g.n3 * g.n * (g.n / 2 + 1), pt = (long long)g.n3 * g.n * g.n;
-    k_omega_spec<<<grid_for(tot), 256, 0, st>>>(g.n, g.n3, g.kmax2, cfg.dz, D[0], D[1], D[2], D[3], D[4]);
-    QG_LAUNCHED();
-    int rc;
-    for (int k = 0; k < 4; ++k)
-      if ((rc = d_c2r(D[1 + k], P[k], g.n3))) return rc;
-    k_omega_phys<T><<<grid_for(pt), 256, 0, st>>>(pt, P[0], P[1], P[2], P[3], P[4]);
-    QG_LAUNCHED();
-    return d_r2c(P[4], D[5], g.n3);
+  // right-hand side from psi (the reference's layout, or the resident field
+  // when dense is null) into rhs; retained: the retained modes and zeros, else
+  // every mode
+  int omega_rhs_dev(const double2* dense, double2* rhs, bool retained) {
+    OmegaIn<T> in{g, dense, F[F_PSI], Divisor(cfg.dz)};
+    int rc = d_inv(in, g.n3, 4, g.n / 2);
+    if (rc) return rc;
+    const int KM = retained ? g.K : g.n / 2;
+    if ((rc = d_prod(g.n3, 4, KM, 1, 1, 0, 0))) return rc;
+    return d_fwd<1>(DenseOut{{rhs, nullptr, nullptr}, retained ? 2 : 0, g.kmax2, 0.0, 0.0}, g.n3, 4, 1);
   }
-  // w from the dense right-hand side in `rhs` into D[1]
-  int omega_solve_dev(const double2* rhs) {
-    const long long per = (long long)g.n * (g.n / 2 + 1);
-    if (!om_scr) QG_CK(cudaMalloc(&om_scr, (size_t)3 * (g.n3 > 1 ? g.n3 - 1 : 1) * per * sizeof(double)));
-    k_omega_solve<<<(unsigned)((per + 127) / 128), 128, 0, st>>>(g.n, g.n3, g.kmax2, cfg.dz, om_t1, om_du, om_dl, om_a,
-                                                                 rhs, om_scr, D[1]);
+  // w from the dense right-hand side into w (device arrays)
+  int omega_solve_dev(const double2* rhs, double2* w) {
+    const int m = g.n3 - 1;
+    QG_CK(cudaMemsetAsync(w, 0, dense_bytes(g.n3), st));
+    if (m < 1 || om_nd == 0) return QG_OK;
+    if (!om_fac) {
+      double4* f = nullptr;
+      QG_CK(cudaMalloc(&f, (size_t)om_nd * m * sizeof(double4)));
+      k_omega_fac<<<(om_nd + 127) / 128, 128, 0, st>>>(om_nd, g.n3, cfg.dz, om_kh2, om_t1, om_du, om_dl, om_a, f);
+      om_fac = f;
+      QG_LAUNCHED();
+    }
+    if (!om_scr) QG_CK(cudaMalloc(&om_scr, (size_t)2 * m * nret * sizeof(double)));
+    k_omega_solve<<<dim3((unsigned)((nret + 63) / 64), 2), 64, 0, st>>>(g, cfg.dz, om_du, om_fac, tab_idx, cols_ret, nret,
+                                                                       rhs, om_scr, w);
     QG_LAUNCHED();
     return QG_OK;
   }
   int omega_eqn_rhs(const double* psik, double* rhs) override {
-    int rc = prep_dense(g.n3);
+    const size_t db = dense_bytes(g.n3);
+    int rc = prep_dense(g.n3, kDensePlanes);
     if (rc) return rc;
-    QG_CK(cudaMemcpyAsync(D[0], psik, dense_bytes(g.n3), cudaMemcpyDefault, st));
-    if ((rc = omega_rhs_dev())) return rc;
-    QG_CK(cudaMemcpyAsync(rhs, D[5], dense_bytes(g.n3), cudaMemcpyDefault, st));
+    const void* p;
+    void* o;
+    if ((rc = in_view(psik, db, 0, &p)) || (rc = out_view(rhs, db, 1, &o))) return rc;
+    if ((rc = omega_rhs_dev((const double2*)p, (double2*)o, false)) || (rc = out_copy(rhs, o, db))) return rc;
     QG_CK(cudaStreamSynchronize(st));
     return QG_OK;
   }
   int omega_equation(const double* rhs, double* wk) override {
-    int rc = prep_dense(g.n3);
-    if (rc) return rc;
-    QG_CK(cudaMemcpyAsync(D[0], rhs, dense_bytes(g.n3), cudaMemcpyDefault, st));
-    if ((rc = omega_solve_dev(D[0]))) return rc;
-    QG_CK(cudaMemcpyAsync(wk, D[1], dense_bytes(g.n3), cudaMemcpyDefault, st));
+    const size_t db = dense_bytes(g.n3);
+    int rc;
+    const void* p;
+    void* o;
+    // (w is written while the right-hand side is read: never in place)
+    if ((rc = in_view(rhs, db, 0, &p)) || (rc = out_view(wk, db, 1, &o, p))) return rc;
+    if ((rc = omega_solve_dev((const double2*)p, (double2*)o)) || (rc = out_copy(wk, o, db))) return rc;
     QG_CK(cudaStreamSynchronize(st));
     return QG_OK;
   }
   int omega_from_state(double* wk) override {
-    int rc = prep_dense(g.n3);
+    const size_t db = dense_bytes(g.n3);
+    int rc = prep_dense(g.n3, kDensePlanes);
     if (rc) return rc;
-    k_compact_to_dense<T><<<grid_for((long long)g.n3 * g.n * (g.n / 2 + 1)), 256, 0, st>>>(g, 0, g.n3, F[F_PSI], D[0], 0,
-                                                                                          cfg.dz);
-    QG_LAUNCHED();
-    if ((rc = omega_rhs_dev()) || (rc = omega_solve_dev(D[5]))) return rc;
-    QG_CK(cudaMemcpyAsync(wk, D[1], dense_bytes(g.n3), cudaMemcpyDefault, st));
+    void* o;
+    if ((rc = out_view(wk, db, 1, &o)) || (rc = ensure(&stg[0], &stg_bytes[0], db))) return rc;
+    if ((rc = omega_rhs_dev(nullptr, (double2*)stg[0], true)) || (rc = omega_solve_dev((double2*)stg[0], (double2*)o)) ||
+        (rc = out_copy(wk, o, db)))
+      return rc;
     QG_CK(cudaStreamSynchronize(st));
     return QG_OK;
   }
 
   // ---- routine-level drop-ins ---------------------------------------------
   int fft_r2c(const double* rvar, double* kvar, int nz) override {
-    int rc = prep_dense(nz);
+    int rc = prep_dense(nz, 1);
     if (rc) return rc;
-    const long long np = (long long)nz * g.n * (g.n + 2);
-    QG_CK(cudaMemcpyAsync(dstage, rvar, np * sizeof(double), cudaMemcpyDefault, st));
-    k_phys_unpad<T><<<grid_for((long long)nz * g.n * g.n), 256, 0, st>>>(g.n, (long long)nz * g.n * g.n, dstage, P[0]);
-    QG_LAUNCHED();
-    if ((rc = d_r2c(P[0], D[0], nz))) return rc;
-    QG_CK(cudaMemcpyAsync(kvar, D[0], dense_bytes(nz), cudaMemcpyDefault, st));
+    const size_t rb = (size_t)nz * g.n * (g.n + 2) * sizeof(double), db = dense_bytes(nz);
+    const void* r;
+    void* k;
+    if ((rc = in_view(rvar, rb, 0, &r)) || (rc = out_view(kvar, db, 1, &k))) return rc;
+    if ((rc = d_r2c((const double*)r, g.n + 2, (double2*)k, nz)) || (rc = out_copy(kvar, k, db))) return rc;
     QG_CK(cudaStreamSynchronize(st));
     return QG_OK;
   }
 
   int fft_c2r(const double* kvar, double* rvar, int nz) override {
-    int rc = prep_dense(nz);
+    int rc = prep_dense(nz, 1);
     if (rc) return rc;
-    QG_CK(cudaMemcpyAsync(D[0], kvar, dense_bytes(nz), cudaMemcpyDefault, st));
-    if ((rc = d_c2r(D[0], P[0], nz))) return rc;
-    const long long np = (long long)nz * g.n * (g.n + 2);
-    k_phys_pad<T><<<grid_for(np), 256, 0, st>>>(g.n, np, P[0], dstage);
-    QG_LAUNCHED();
-    QG_CK(cudaMemcpyAsync(rvar, dstage, np * sizeof(double), cudaMemcpyDefault, st));
+    const size_t rb = (size_t)nz * g.n * (g.n + 2) * sizeof(double), db = dense_bytes(nz);
+    const void* k;
+    void* r;
+    if ((rc = in_view(kvar, db, 0, &k)) || (rc = out_view(rvar, rb, 1, &r))) return rc;
+    if ((rc = d_c2r((const double2*)k, (double*)r, g.n + 2, nz)) || (rc = out_copy(rvar, r, rb))) return rc;
+    QG_CK(cudaStreamSynchronize(st));
+    return QG_OK;
+  }
+
+  // the three nonlinear terms: inputs under their operators to (kx, y)
+  // planes, rows to products, columns to outputs
+  int nonlinear(std::initializer_list<const double*> ins, std::initializer_list<std::pair<int, int>> fields,
+                std::initializer_list<double*> outs, int mode, int cross, int nA, int nX, int nz) {
+    int rc = prep_dense(nz, kDensePlanes);
+    if (rc) return rc;
+    const size_t db = dense_bytes(nz);
+    const void* v[kDenseFields];
+    int k = 0;
+    for (const double* p : ins) { if ((rc = in_view(p, db, k, &v[k]))) return rc; ++k; }
+    DenseIn in{};
+    in.kmax2 = g.kmax2;
+    int nf = 0;
+    for (const auto& f : fields) { in.p[nf] = (const double2*)v[f.first]; in.op[nf] = f.second; ++nf; }
+    DenseOut o{{nullptr, nullptr, nullptr}, mode, g.kmax2, cfg.Ro, cfg.W2F};
+    int no = 0;
+    // (staged inputs are read before staged outputs are written)
+    for (double* p : outs) { void* q; if ((rc = out_view(p, db, no, &q))) return rc; o.p[no++] = (double2*)q; }
+    const int np = kDensePlanes;
+    if ((rc = d_inv(in, nz, nf, g.n / 2, np)) || (rc = d_prod(nz, np, g.K, cross, 0, nA, nX))) return rc;
+    if ((rc = mode == 2 ? d_fwd<1>(o, nz, np, no) : d_fwd<2>(o, nz, np, no))) return rc;
+    no = 0;
+    for (double* p : outs) { if ((rc = out_copy(p, o.p[no], db))) return rc; ++no; }
     QG_CK(cudaStreamSynchronize(st));
     return QG_OK;
   }
 
   int convol_waqg(const double* uk, const double* vk, const double* qk, const double* BRk, const double* BIk,
                   double* nqk, double* nBRk, double* nBIk, int nz) override {
-    int rc = prep_dense(nz);
-    if (rc) return rc;
-    const size_t db = dense_bytes(nz);
-    const long long tot = (long long)nz * g.n * (g.n / 2 + 1), pt = (long long)nz * g.n * g.n;
-    QG_CK(cudaMemcpyAsync(D[0], uk, db, cudaMemcpyDefault, st));
-    QG_CK(cudaMemcpyAsync(D[1], vk, db, cudaMemcpyDefault, st));
-    if ((rc = d_c2r(D[0], P[0], nz)) || (rc = d_c2r(D[1], P[1], nz))) return rc;
-    const double* ins[3] = {qk, BRk, BIk};
-    double* outs[3] = {nqk, nBRk, nBIk};
-    for (int k = 0; k < 3; ++k) {
-      QG_CK(cudaMemcpyAsync(D[2], ins[k], db, cudaMemcpyDefault, st));
-      if ((rc = d_c2r(D[2], P[2], nz))) return rc;
-      k_phys<T><<<grid_for(pt), 256, 0, st>>>(pt, 0, P[0], P[2], nullptr, nullptr, P[3]);
-      QG_LAUNCHED();
-      if ((rc = d_r2c(P[3], D[3], nz))) return rc;
-      k_phys<T><<<grid_for(pt), 256, 0, st>>>(pt, 0, P[1], P[2], nullptr, nullptr, P[3]);
-      QG_LAUNCHED();
-      if ((rc = d_r2c(P[3], D[4], nz))) return rc;
-      k_dense_ik<<<grid_for(tot), 256, 0, st>>>(g.n, g.kmax2, tot, D[3], D[4], D[5]);
-      QG_LAUNCHED();
-      QG_CK(cudaMemcpyAsync(outs[k], D[5], db, cudaMemcpyDefault, st));
-      QG_CK(cudaStreamSynchronize(st));
-    }
-    return QG_OK;
+    return nonlinear({uk, vk, qk, BRk, BIk}, {{0, OP_ID}, {1, OP_ID}, {2, OP_ID}, {3, OP_ID}, {4, OP_ID}},
+                     {nqk, nBRk, nBIk}, 1, 0, 2, 3, nz);
   }
 
   int refraction_waqg(const double* BRk, const double* BIk, const double* psik, double* rBRk, double* rBIk,
                       int nz) override {
-    int rc = prep_dense(nz);
-    if (rc) return rc;
-    const size_t db = dense_bytes(nz);
-    const long long tot = (long long)nz * g.n * (g.n / 2 + 1), pt = (long long)nz * g.n * g.n;
-    QG_CK(cudaMemcpyAsync(D[0], psik, db, cudaMemcpyDefault, st));
-    k_dense_op<<<grid_for(tot), 256, 0, st>>>(g.n, g.kmax2, tot, 0, D[0], D[1]);
-    QG_LAUNCHED();
-    if ((rc = d_c2r(D[1], P[0], nz))) return rc;
-    const double* ins[2] = {BRk, BIk};
-    double* outs[2] = {rBRk, rBIk};
-    for (int k = 0; k < 2; ++k) {
-      QG_CK(cudaMemcpyAsync(D[2], ins[k], db, cudaMemcpyDefault, st));
-      if ((rc = d_c2r(D[2], P[1], nz))) return rc;
-      k_phys<T><<<grid_for(pt), 256, 0, st>>>(pt, 0, P[0], P[1], nullptr, nullptr, P[2]);
-      QG_LAUNCHED();
-      if ((rc = d_r2c(P[2], D[3], nz))) return rc;
-      k_dense_mask<<<grid_for(tot), 256, 0, st>>>(g.n, g.kmax2, tot, D[3], D[4]);
-      QG_LAUNCHED();
-      QG_CK(cudaMemcpyAsync(outs[k], D[4], db, cudaMemcpyDefault, st));
-      QG_CK(cudaStreamSynchronize(st));
-    }
-    return QG_OK;
+    return nonlinear({BRk, BIk, psik}, {{2, OP_LAP}, {0, OP_ID}, {1, OP_ID}}, {rBRk, rBIk}, 2, 0, 1, 2, nz);
   }
 
+  // BRy BIx - BRx BIy and BR^2 + BI^2 (derivatives.f90:973, 996)
   int compute_qw(const double* BRk, const double* BIk, double* qwk, int nz) override {
-    int rc = prep_dense(nz);
-    if (rc) return rc;
-    const size_t db = dense_bytes(nz);
-    const long long tot = (long long)nz * g.n * (g.n / 2 + 1), pt = (long long)nz * g.n * g.n;
-    QG_CK(cudaMemcpyAsync(D[0], BRk, db, cudaMemcpyDefault, st));
-    QG_CK(cudaMemcpyAsync(D[1], BIk, db, cudaMemcpyDefault, st));
-    // BRx, BRy, BIx, BIy -> P0..P3
-    const int ops[4] = {1, 2, 1, 2};
-    for (int k = 0; k < 4; ++k) {
-      k_dense_op<<<grid_for(tot), 256, 0, st>>>(g.n, g.kmax2, tot, ops[k], D[k < 2 ? 0 : 1], D[2]);
-      QG_LAUNCHED();
-      if ((rc = d_c2r(D[2], P[k], nz))) return rc;
-    }
-    // qwr = BRy*BIx - BRx*BIy
-    k_phys<T><<<grid_for(pt), 256, 0, st>>>(pt, 2, P[1], P[2], P[0], P[3], P[4]);
-    QG_LAUNCHED();
-    if ((rc = d_r2c(P[4], D[3], nz))) return rc;
-    if ((rc = d_c2r(D[0], P[0], nz)) || (rc = d_c2r(D[1], P[1], nz))) return rc;
-    k_phys<T><<<grid_for(pt), 256, 0, st>>>(pt, 1, P[0], P[1], nullptr, nullptr, P[4]);
-    QG_LAUNCHED();
-    if ((rc = d_r2c(P[4], D[4], nz))) return rc;
-    k_dense_qw<<<grid_for(tot), 256, 0, st>>>(g.n, g.kmax2, tot, D[3], D[4], cfg.Ro, cfg.W2F, D[5]);
-    QG_LAUNCHED();
-    QG_CK(cudaMemcpyAsync(qwk, D[5], db, cudaMemcpyDefault, st));
-    QG_CK(cudaStreamSynchronize(st));
-    return QG_OK;
+    return nonlinear({BRk, BIk}, {{0, OP_IKY}, {1, OP_IKX}, {0, OP_IKX}, {1, OP_IKY}, {0, OP_ID}, {1, OP_ID}}, {qwk}, 3, 2,
+                     0, 0, nz);
   }
 
   int psi_solver(const double* qstar, double* psik) override {
@@ -725,7 +710,9 @@ class Engine : public EngineBase {
     if (rc) return rc;
     if ((rc = upload_compact(qstar, tmpF[0]))) return rc;
     if ((rc = solve_generic(tmpF[0], nullptr, nullptr, tmpF[1], nullptr, nullptr, 1, 0, nullptr, 0, -1, true))) return rc;
-    return download_compact(tmpF[1], psik, 0);
+    if ((rc = download_compact(tmpF[1], psik, 0))) return rc;
+    QG_CK(cudaStreamSynchronize(st));
+    return QG_OK;
   }
 
   int A_solver(const double* bk, double* ak, double* ck) override {
@@ -734,7 +721,8 @@ class Engine : public EngineBase {
     if ((rc = upload_compact(bk, tmpF[0]))) return rc;
     if ((rc = solve_generic(nullptr, tmpF[0], nullptr, nullptr, tmpF[1], nullptr, 0, 2, nullptr, 0, -1, true))) return rc;
     if ((rc = download_compact(tmpF[1], ak, 0))) return rc;
-    if (ck) return download_compact(tmpF[1], ck, 1);
+    if (ck && (rc = download_compact(tmpF[1], ck, 1))) return rc;
+    QG_CK(cudaStreamSynchronize(st));
     return QG_OK;
   }
 
@@ -778,6 +766,9 @@ class Engine : public EngineBase {
   int* iflag = nullptr;
   int nsm = 1, occ_rm = 1, occ_rq = 1;   // SMs; resident CTAs per SM of the persistent row kernels
   double *om_t1 = nullptr, *om_du = nullptr, *om_dl = nullptr, *om_a = nullptr, *om_scr = nullptr;
+  double4* om_fac = nullptr;   // omega operator's factors per distinct kh2 (first use)
+  int* om_kh2 = nullptr;       // the distinct kh2
+  int om_nd = 0;
   C* sig[2] = {};     // regular YBJ: per-level sigma terms
   C* Qp = nullptr;             // kept y-inverse planes of B, [n3][2][n][KXP], or null
   bool q_valid = false;        // Qp holds the transforms of the current B
@@ -785,7 +776,8 @@ class Engine : public EngineBase {
   double* mpar = nullptr;      // their step parameters (StepParams::mpar)
   C* S = nullptr;              // [lanes][Zb][kNScr][n][KXP] scratch planes
   int s_levels = 0;            // levels of scratch allocated
-  double2* psi64 = nullptr;
+  double2* psi64 = nullptr;    // FP64 copy of psi between qg_set_state and qg_init_state
+  bool psi64_live = false;
   int Zb = 1;
   // phase-A batches run on `lanes` streams (lane 0: st), batch b on lane
   // b % lanes with its own scratch slot; they join st before the solves
@@ -796,13 +788,15 @@ class Engine : public EngineBase {
   cudaEvent_t ev_start = nullptr;
   bool need_qw = true;
   void* stage = nullptr; size_t stage_bytes = 0;
-  // dense drop-in buffers
-  int dense_nz = 0;
-  double2* D[6] = {};
-  T* P[5] = {};
+  // (kx, y) planes of the routine-level calls (kDensePlanes per level where
+  // products are formed), and staging copies of the callers' arrays that the
+  // kernels cannot use in place
+  static constexpr int kDensePlanes = 6;
   C* W = nullptr;
-  double* dstage = nullptr;
-  C* tmpF[3] = {};
+  size_t w_planes = 0;
+  void* stg[kDenseFields] = {};
+  size_t stg_bytes[kDenseFields] = {};
+  C* tmpF[2] = {};
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
 
   void release() {
@@ -810,10 +804,9 @@ class Engine : public EngineBase {
     for (auto& x : gexec) if (x) { cudaGraphExecDestroy(x); x = nullptr; }
     for (auto& p : F) if (p) { cudaFree(p); p = nullptr; }
     void* ps[] = {e1, e2, e1w, e2w, tw, tab_idx, cols_all, cols_ret, fac_psi, fac_A, pcfac, vbuf, du, cu, cl, r2, diag_part, diag_out, dwz, fwz, S, stage,
-                  W, dstage, psi64, om_t1, om_du, om_dl, om_a, om_scr, sig[0], sig[1], mpar, Qp};
+                  W, psi64, om_t1, om_du, om_dl, om_a, om_scr, om_fac, om_kh2, sig[0], sig[1], mpar, Qp};
     for (void* p : ps) if (p) cudaFree(p);
-    for (auto& p : D) if (p) cudaFree(p);
-    for (auto& p : P) if (p) cudaFree(p);
+    for (auto& p : stg) if (p) cudaFree(p);
     for (auto& p : tmpF) if (p) cudaFree(p);
     if (diag_host) cudaFreeHost(diag_host);
     if (wflag_h) cudaFreeHost(wflag_h);
@@ -846,6 +839,8 @@ class Engine : public EngineBase {
     long long b = (n + 255) / 256;
     return (unsigned)std::max<long long>(1, std::min<long long>(b, 152LL * 16));
   }
+
+  static dim3 conv_grid(int rows, int nlev) { return dim3((rows + kConvRows - 1) / kConvRows, nlev); }
 
   int map_field(int field) const {
     switch (field) {
@@ -912,9 +907,14 @@ class Engine : public EngineBase {
       // per-function attribute shared by every handle: set it for the deepest supported column
       QG_CK(cudaFuncSetAttribute(k_solve<T>, (cudaFuncAttribute)mx, (int)solve_smem(kMaxN3)));
       using DN = Dense<T, NN>;
-      QG_CK(cudaFuncSetAttribute(k_dcol_inv<T, NN>, (cudaFuncAttribute)mx, (int)DN::sm_col()));
-      QG_CK(cudaFuncSetAttribute(k_dcol_fwd<T, NN>, (cudaFuncAttribute)mx, (int)DN::sm_col()));
-      QG_CK(cudaFuncSetAttribute(k_drow_c2r<T, NN>, (cudaFuncAttribute)mx, (int)DN::sm_row()));
+      QG_CK(cudaFuncSetAttribute(k_dcol_inv<T, NN, DenseIn>, (cudaFuncAttribute)mx, (int)DN::sm_col()));
+      QG_CK(cudaFuncSetAttribute(k_dcol_inv<T, NN, CompactIn<T>>, (cudaFuncAttribute)mx, (int)DN::sm_col()));
+      QG_CK(cudaFuncSetAttribute(k_dcol_inv<T, NN, OmegaIn<T>>, (cudaFuncAttribute)mx, (int)DN::sm_col()));
+      QG_CK(cudaFuncSetAttribute(k_dcol_fwd<T, NN, 1>, (cudaFuncAttribute)mx, (int)DN::sm_col(1)));
+      QG_CK(cudaFuncSetAttribute(k_dcol_fwd<T, NN, 2>, (cudaFuncAttribute)mx, (int)DN::sm_col(2)));
+      QG_CK(cudaFuncSetAttribute(k_drow_c2r_pad<T, NN>, (cudaFuncAttribute)mx, (int)DN::sm_row()));
+      QG_CK(cudaFuncSetAttribute(k_drow_c2r_f32<T, NN>, (cudaFuncAttribute)mx, (int)DN::sm_row()));
+      QG_CK(cudaFuncSetAttribute(k_drow_prod<T, NN>, (cudaFuncAttribute)mx, (int)DProd<T, NN>::smem()));
       QG_CK(cudaFuncSetAttribute(k_drow_r2c<T, NN>, (cudaFuncAttribute)mx, (int)DN::sm_row()));
     });
     return QG_OK;
@@ -1219,42 +1219,114 @@ class Engine : public EngineBase {
   size_t dense_bytes(int nz) const { return (size_t)nz * g.n * (g.n / 2 + 1) * sizeof(double2); }
   int iktxP() const { return dense_kxp(g.n); }
 
-  int prep_dense(int nz) {
+  int prep_dense(int nz, int planes) {
     if (nz <= 0) { err = "nz must be positive"; return QG_ERR_ARG; }
-    if (nz <= dense_nz) return QG_OK;
+    const size_t need = (size_t)nz * planes;
+    if (need <= w_planes) return QG_OK;
     QG_CK(cudaStreamSynchronize(st));
-    for (auto& p : D) if (p) { cudaFree(p); p = nullptr; }
-    for (auto& p : P) if (p) { cudaFree(p); p = nullptr; }
-    if (W) { cudaFree(W); W = nullptr; }
-    if (dstage) { cudaFree(dstage); dstage = nullptr; }
-    for (auto& p : D) QG_CK(cudaMalloc(&p, dense_bytes(nz)));
-    for (auto& p : P) QG_CK(cudaMalloc(&p, (size_t)nz * g.n * g.n * sizeof(T)));
-    QG_CK(cudaMalloc(&W, (size_t)nz * g.n * iktxP() * sizeof(C)));
-    QG_CK(cudaMalloc(&dstage, (size_t)nz * g.n * (g.n + 2) * sizeof(double)));
-    dense_nz = nz;
+    if (W) { cudaFree(W); W = nullptr; w_planes = 0; }
+    QG_CK(cudaMalloc(&W, need * g.n * iktxP() * sizeof(C)));
+    w_planes = need;
     return QG_OK;
   }
 
-  int d_c2r(const double2* spec, T* phys, int nz) {
+  // Whether kernels on this device may use [p, p + bytes) in place: 16-byte
+  // aligned memory of this device, inside one allocation.  Anything else goes
+  // through a staging copy, whose cudaMemcpy accepts or refuses it as it does
+  // any pointer.
+  bool in_place(const void* p, size_t bytes) const {
+    if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { (void)cudaGetLastError(); return false; }
+    if (at.type != cudaMemoryTypeDevice || at.device != cfg.device) return false;
+    using Range = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static const Range range = []() -> Range {
+      void* f = nullptr;
+      cudaDriverEntryPointQueryResult q;
+      if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+          q != cudaDriverEntryPointSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+      }
+      return reinterpret_cast<Range>(f);
+    }();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    const CUdeviceptr a = reinterpret_cast<CUdeviceptr>(p);
+    return range && range(&base, &size, a) == CUDA_SUCCESS && a - base + bytes <= size;
+  }
+  // a device view of an input (copied into staging slot `slot` if need be)
+  int in_view(const void* p, size_t bytes, int slot, const void** v) {
+    if (in_place(p, bytes)) { *v = p; return QG_OK; }
+    if (int rc = ensure(&stg[slot], &stg_bytes[slot], bytes)) return rc;
+    QG_CK(cudaMemcpyAsync(stg[slot], p, bytes, cudaMemcpyDefault, st));
+    *v = stg[slot];
+    return QG_OK;
+  }
+  // where kernels write an output: the caller's array, or staging slot `slot`
+  // (also where the array overlaps `keep`, an input of the same size that is
+  // read while the output is written); out_copy then brings it to the caller
+  int out_view(void* p, size_t bytes, int slot, void** v, const void* keep = nullptr) {
+    const char *a = (const char*)p, *k = (const char*)keep;
+    if (in_place(p, bytes) && !(keep && a < k + bytes && k < a + bytes)) { *v = p; return QG_OK; }
+    if (int rc = ensure(&stg[slot], &stg_bytes[slot], bytes)) return rc;
+    *v = stg[slot];
+    return QG_OK;
+  }
+  int out_copy(void* p, const void* v, size_t bytes) {
+    if (v != p) QG_CK(cudaMemcpyAsync(p, v, bytes, cudaMemcpyDefault, st));
+    return QG_OK;
+  }
+
+  // y-inverse transforms of nf fields of src at kx <= KM into planes 0 .. nf-1
+  // (np per level)
+  template <class Src> int d_inv(const Src& src, int nz, int nf, int KM, int np = 0) {
     QG_SWITCH_N(g.n, {
       using DN = Dense<T, NN>;
-      k_dcol_inv<T, NN><<<dim3(iktxP() / DN::CT, nz), DN::CNT, DN::sm_col(), st>>>(iktxP(), spec, W, tw);
+      k_dcol_inv<T, NN, Src><<<dim3((KM + DN::CT) / DN::CT, nz, nf), DN::CNT, DN::sm_col(), st>>>(iktxP(), np ? np : nf, src,
+                                                                                               W, tw);
       QG_LAUNCHED();
-      k_drow_c2r<T, NN><<<dim3(g.n / 2 / DN::RT, nz), DN::RNT, DN::sm_row(), st>>>(iktxP(), W, phys, tw);
+    });
+    return QG_OK;
+  }
+  int d_prod(int nz, int np, int KM, int cross, int scale, int nA, int nX) {
+    QG_SWITCH_N(g.n, {
+      using DN = Dense<T, NN>;
+      k_drow_prod<T, NN><<<dim3(g.n / 2 / DN::RT, nz), DN::RNT, DProd<T, NN>::smem(), st>>>(iktxP(), np, KM, cross, scale, nA,
+                                                                                         nX, W, tw);
+      QG_LAUNCHED();
+    });
+    return QG_OK;
+  }
+  template <int NF> int d_fwd(const DenseOut& o, int nz, int np, int no) {
+    QG_SWITCH_N(g.n, {
+      using DN = Dense<T, NN>;
+      k_dcol_fwd<T, NN, NF><<<dim3(iktxP() / DN::CT, nz, no), DN::CNT, DN::sm_col(NF), st>>>(iktxP(), np, W, o, tw);
       QG_LAUNCHED();
     });
     return QG_OK;
   }
 
-  int d_r2c(const T* phys, double2* spec, int nz) {
+  // c2r and r2c of nz levels; physical rows of ld doubles (n or n + 2)
+  int d_c2r(const double2* spec, double* phys, int ld, int nz) {
+    DenseIn in{};
+    in.p[0] = spec;
+    in.op[0] = OP_ID;
+    if (int rc = d_inv(in, nz, 1, g.n / 2)) return rc;
     QG_SWITCH_N(g.n, {
       using DN = Dense<T, NN>;
-      k_drow_r2c<T, NN><<<dim3(g.n / 2 / DN::RT, nz), DN::RNT, DN::sm_row(), st>>>(iktxP(), phys, W, tw);
-      QG_LAUNCHED();
-      k_dcol_fwd<T, NN><<<dim3(iktxP() / DN::CT, nz), DN::CNT, DN::sm_col(), st>>>(iktxP(), W, spec, tw);
+      k_drow_c2r_pad<T, NN><<<dim3(g.n / 2 / DN::RT, nz), DN::RNT, DN::sm_row(), st>>>(iktxP(), W, phys, ld, tw);
       QG_LAUNCHED();
     });
     return QG_OK;
+  }
+  int d_r2c(const double* phys, int ld, double2* spec, int nz) {
+    QG_SWITCH_N(g.n, {
+      using DN = Dense<T, NN>;
+      k_drow_r2c<T, NN><<<dim3(g.n / 2 / DN::RT, nz), DN::RNT, DN::sm_row(), st>>>(iktxP(), phys, ld, W, tw);
+      QG_LAUNCHED();
+    });
+    return d_fwd<1>(DenseOut{{spec, nullptr, nullptr}, 0, g.kmax2, 0.0, 0.0}, nz, 1, 1);
   }
 
   int ensure_tmp() {
@@ -1264,25 +1336,20 @@ class Engine : public EngineBase {
   }
 
   int upload_compact(const double* kvar, C* dst) {
-    const size_t bytes = dense_bytes(g.n3);
-    int rc = ensure(&stage, &stage_bytes, bytes);
-    if (rc) return rc;
-    QG_CK(cudaMemcpyAsync(stage, kvar, bytes, cudaMemcpyDefault, st));
-    k_dense_to_compact<T><<<grid_for((long long)g.n3 * g.plane), 256, 0, st>>>(g, 0, g.n3, (const double2*)stage, dst);
+    const void* v;
+    if (int rc = in_view(kvar, dense_bytes(g.n3), 0, &v)) return rc;
+    k_dense_to_compact<T><<<conv_grid(g.KY, g.n3), 256, 0, st>>>(g, 0, (const double2*)v, dst);
     QG_LAUNCHED();
     return QG_OK;
   }
 
   int download_compact(const C* src, double* kvar, int mode) {
     const size_t bytes = dense_bytes(g.n3);
-    int rc = ensure(&stage, &stage_bytes, bytes);
-    if (rc) return rc;
-    k_compact_to_dense<T><<<grid_for((long long)g.n3 * g.n * (g.n / 2 + 1)), 256, 0, st>>>(g, 0, g.n3, src,
-                                                                                           (double2*)stage, mode, cfg.dz);
+    void* v;
+    if (int rc = out_view(kvar, bytes, 0, &v)) return rc;
+    k_compact_to_dense<T><<<conv_grid(g.n, g.n3), 256, 0, st>>>(g, 0, src, (double2*)v, mode, Divisor(cfg.dz));
     QG_LAUNCHED();
-    QG_CK(cudaMemcpyAsync(kvar, stage, bytes, cudaMemcpyDefault, st));
-    QG_CK(cudaStreamSynchronize(st));
-    return QG_OK;
+    return out_copy(kvar, v, bytes);
   }
 };
 

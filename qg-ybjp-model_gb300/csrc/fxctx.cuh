@@ -177,10 +177,10 @@ template <int N, int T = 128> struct FxRowCtx {
     fx_core<N>(v, base, buf, tw, j, [](int i) { return fx_idx(i); }, [&]() { sync(); },
                [&](unsigned m) { return fx_row_reduce<NB, true>(m, slots + 2 * FxRow<N, T>::RT * FxRow<N, T>::W, rr); });
   }
-  // inverse transform of the packed spectrum d (zeros at |k| > K) into
+  // inverse transform of the packed spectrum d (PRUNED: zeros at |k| > K) into
   // integers of 61 bits: v.y the first (real) row, v.x the second
-  __device__ __forceinline__ void inverse(double2 (&d)[8], fxc (&v)[8], int& base) {
-    base = fx_ints<8, false, true>(d, v, reduce<false>(fx_maxp<8, true>(d)));
+  template <bool PRUNED = true> __device__ __forceinline__ void inverse(double2 (&d)[8], fxc (&v)[8], int& base) {
+    base = fx_ints<8, false, PRUNED>(d, v, reduce<false>(fx_maxp<8, PRUNED>(d)));
     core(v, base);
     fx_norm<8, 61>(v, reduce<true>(fx_bits<8>(v)), base);
   }
@@ -223,11 +223,11 @@ template <int N, int T = 128> struct FxRowCtx {
       if (j + q * NB <= KM) put(q, j + q * NB, o[2 * q], o[2 * q + 1]);
   }
   // forward transform of the integers v (two packed rows) and its split
-  template <class Put> __device__ __forceinline__ void forward(fxc (&v)[8], int base, int K, Put put) {
+  template <int Q = 3, class Put> __device__ __forceinline__ void forward(fxc (&v)[8], int base, int K, Put put) {
     const unsigned o = reduce<true>(fx_bits<8>(v));
     fx_norm<8, 59>(v, o, base);
     core(v, base);
-    split<3>(v, base, K, put);
+    split<Q>(v, base, K, put);
   }
 };
 

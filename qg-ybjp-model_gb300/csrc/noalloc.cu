@@ -74,7 +74,7 @@ int setup_device(int dev, DeviceSetup** out) {
     NA_CK(cudaMemcpyToSymbol(g_noalloc_tw, tw.data(), sizeof(double2) * kTwEntries));
     const int mx = cudaFuncAttributeMaxDynamicSharedMemorySize;
 #define NA_ATTR(NN)                                                                                        \
-    NA_CK(cudaFuncSetAttribute(qg::k_dcol_inv<double, NN>, (cudaFuncAttribute)mx,                          \
+    NA_CK(cudaFuncSetAttribute(qg::k_dcol_inv<double, NN, qg::DenseIn>, (cudaFuncAttribute)mx,                          \
                                (int)qg::Dense<double, NN>::sm_col()));                                     \
     NA_CK(cudaFuncSetAttribute(qg::k_drow_c2r_pad<double, NN>, (cudaFuncAttribute)mx,                      \
                                (int)qg::Dense<double, NN>::sm_row()));
@@ -130,11 +130,13 @@ int launch_chunks(const double2* in, double* out, int nz, cudaStream_t st, const
   const double2* tw = s.tw + tw_offset(N);
   for (int z0 = 0; z0 < nz; z0 += chunk) {
     const int zc = nz - z0 < chunk ? nz - z0 : chunk;
-    qg::k_dcol_inv<double, N><<<dim3(ip / DN::CT, zc), DN::CNT, DN::sm_col(), st>>>(
-        ip, in + (size_t)z0 * N * (N / 2 + 1), s.scratch, tw);
+    qg::DenseIn src{};
+    src.p[0] = in + (size_t)z0 * N * (N / 2 + 1);
+    src.op[0] = qg::OP_ID;
+    qg::k_dcol_inv<double, N, qg::DenseIn><<<dim3(ip / DN::CT, zc), DN::CNT, DN::sm_col(), st>>>(ip, 1, src, s.scratch, tw);
     NA_LAUNCH_CK();
     qg::k_drow_c2r_pad<double, N><<<dim3(N / 2 / DN::RT, zc), DN::RNT, DN::sm_row(), st>>>(
-        ip, s.scratch, out + (size_t)z0 * N * (N + 2), tw);
+        ip, s.scratch, out + (size_t)z0 * N * (N + 2), N + 2, tw);
     NA_LAUNCH_CK();
   }
   return QG_OK;
