@@ -193,7 +193,8 @@ __device__ __forceinline__ void adj_col_inverse(const FxColCtx<N>& c, const Geom
 }
 
 // the transposed products' kernels keep one transform per thread in flight,
-// as the step's (step_fx.cuh)
+// as the step's (step_fx.cuh); the column kernels' independent fields are
+// spread over gridDim.z CTAs where a grid would leave SMs idle
 template <int N>
 __global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(QG_FX_COL_CTAS))
 k_adj_col_inv(Geom g, AdjP p, int zbase, AdjIn L, const double* __restrict__ e1t, const double* __restrict__ e2t,
@@ -208,7 +209,7 @@ k_adj_col_inv(Geom g, AdjP p, int zbase, AdjIn L, const double* __restrict__ e1t
   const double inv2n2 = 0.5 / ((double)N * (double)N);
   // l and -i ky l of the adjoint tendencies of q, BR, BI
 #pragma unroll 1
-  for (int f = 0; f < 6; ++f) {
+  for (int f = blockIdx.z; f < 6; f += gridDim.z) {
     const int w = f >> 1;
     adj_col_inverse<N>(c, g, kx, SA + scr_off(zb, f, 0, N, g.KXP), [&](int row, int ky) {
       const long long mt = (long long)row * g.KXP + kx;
@@ -228,8 +229,11 @@ k_adj_col_inv(Geom g, AdjP p, int zbase, AdjIn L, const double* __restrict__ e1t
 template <int N> struct AdjRow {
   static constexpr size_t smem() { return FxRow<N>::smem() + (size_t)3 * FxRow<N>::RT * N * sizeof(double2); }
 };
+#ifndef QG_ADJ_ROW_CTAS
+#define QG_ADJ_ROW_CTAS 2
+#endif
 template <int N>
-__global__ void __launch_bounds__(FxRow<N>::NT, fx_row_ctas<N>(2))
+__global__ void __launch_bounds__(FxRow<N>::NT, fx_row_ctas<N>(QG_ADJ_ROW_CTAS))
 k_adj_row(Geom g, AdjP p, const double2* __restrict__ SF, double2* __restrict__ SA, const double2* __restrict__ twg) {
   using F = FxRow<N>;
   constexpr int NB = F::NB;
@@ -350,9 +354,11 @@ k_adj_col_fwd(Geom g, AdjP p, int zbase, AdjIn L, AdjOut O, const double* __rest
   const int zb = blockIdx.y, kx = blockIdx.x * F::CT + c.c;
   const long long zoff = (long long)(zbase + zb) * g.plane;
   // psi -> (u, v, zeta) = (-i ky, i kx, -kh^2) psi: transposes i ky, -i kx, -kh^2
+  // (spread over gridDim.z = 4 CTAs: u, v, zeta; q; BR; BI)
+  const int f0 = blockIdx.z ? 2 + blockIdx.z : 0, f1 = gridDim.z == 1 ? 6 : (blockIdx.z ? f0 + 1 : 3);
   double2 a[8];
 #pragma unroll 1
-  for (int f = 0; f < 6; ++f) {
+  for (int f = f0; f < f1; ++f) {
     adj_col_plane<N>(c, g, SA + scr_off(zb, f, 0, N, g.KXP), kx, [&](int r, long long mt, int ky, double2 h) {
       const long long m = zoff + mt;
       if (f == 0) {
@@ -393,7 +399,7 @@ k_adj_qw_col_inv(Geom g, int zbase, const double2* __restrict__ BR, const double
   const long long zoff = (long long)(zbase + zb) * g.plane;
   const double inv2n2 = 0.5 / ((double)N * (double)N);
 #pragma unroll 1
-  for (int f = 0; f < 6; ++f) {
+  for (int f = blockIdx.z; f < 6; f += gridDim.z) {
     const double2* X = f < 2 ? BR : (f < 4 ? BI : w);
     adj_col_inverse<N>(c, g, kx, SF + scr_off(zb, f, 0, N, g.KXP), [&](int row, int ky) {
       double2 x = X[zoff + (long long)row * g.KXP + kx];
@@ -473,9 +479,11 @@ k_adj_qw_col_fwd(Geom g, int zbase, double2* __restrict__ lBR, double2* __restri
   const FxColCtx<N> c = fx_col_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
   const int zb = blockIdx.y, kx = blockIdx.x * F::CT + c.c;
   const long long zoff = (long long)(zbase + zb) * g.plane;
+  // (spread over gridDim.z = 2 CTAs: BR; BI)
+  const int f0 = 2 * blockIdx.z, f1 = gridDim.z == 1 ? 4 : f0 + 2;
   double2 a[8];
 #pragma unroll 1
-  for (int f = 0; f < 4; ++f) {
+  for (int f = f0; f < f1; ++f) {
     double2* lB = f < 2 ? lBR : lBI;
     adj_col_plane<N>(c, g, SF + scr_off(zb, f, 0, N, g.KXP), kx, [&](int r, long long mt, int ky, double2 h) {
       if ((f & 1) == 0) { a[r] = h; return; }

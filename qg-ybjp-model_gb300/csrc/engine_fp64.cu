@@ -367,13 +367,15 @@ class AdjEngine final : public Engine<double> {
         using FC = FxCol<NN>;
         using FR = FxRow<NN>;
         const dim3 gc((g.K + FC::CT) / FC::CT, zc), gr(g.n / FR::RT, zc);
+        const bool few = few_ctas((long long)gc.x * gc.y, 1, fx_col_ctas<NN>(QG_FX_COL_CTAS));
+        auto over = [&](unsigned k) { return dim3(gc.x, gc.y, few ? k : 1); };
         launch_col_inv<NN>(z0, zc, psi, q, BR, BI, S, nullptr, 0, st);
         QG_LAUNCHED();
-        k_adj_col_inv<NN><<<gc, FC::NT, FC::smem(), st>>>(g, p, z0, L, e1, e2, e1w, e2w, SA, tw);
+        k_adj_col_inv<NN><<<over(6), FC::NT, FC::smem(), st>>>(g, p, z0, L, e1, e2, e1w, e2w, SA, tw);
         QG_LAUNCHED();
         k_adj_row<NN><<<gr, FR::NT, AdjRow<NN>::smem(), st>>>(g, p, S, SA, tw);
         QG_LAUNCHED();
-        k_adj_col_fwd<NN><<<gc, FC::NT, FC::smem(), st>>>(g, p, z0, L, O, e1, e2, e1w, e2w, SA, tw);
+        k_adj_col_fwd<NN><<<over(4), FC::NT, FC::smem(), st>>>(g, p, z0, L, O, e1, e2, e1w, e2w, SA, tw);
         QG_LAUNCHED();
       });
     }
@@ -389,11 +391,13 @@ class AdjEngine final : public Engine<double> {
         using FC = FxCol<NN>;
         using FR = FxRow<NN>;
         const dim3 gc((g.K + FC::CT) / FC::CT, zc), gr(g.n / FR::RT, zc);
-        k_adj_qw_col_inv<NN><<<gc, FC::NT, FC::smem(), st>>>(g, z0, BR, BI, Af[A_W], S, tw);
+        const bool few = few_ctas((long long)gc.x * gc.y, 1, fx_col_ctas<NN>(QG_FX_COL_CTAS));
+        auto over = [&](unsigned k) { return dim3(gc.x, gc.y, few ? k : 1); };
+        k_adj_qw_col_inv<NN><<<over(6), FC::NT, FC::smem(), st>>>(g, z0, BR, BI, Af[A_W], S, tw);
         QG_LAUNCHED();
         k_adj_qw_row<NN><<<gr, FR::NT, FR::smem(), st>>>(g, p, S, tw);
         QG_LAUNCHED();
-        k_adj_qw_col_fwd<NN><<<gc, FC::NT, FC::smem(), st>>>(g, z0, lo[2], lo[3], S, tw);
+        k_adj_qw_col_fwd<NN><<<over(2), FC::NT, FC::smem(), st>>>(g, z0, lo[2], lo[3], S, tw);
         QG_LAUNCHED();
       });
     }
