@@ -229,11 +229,8 @@ k_adj_col_inv(Geom g, AdjP p, int zbase, AdjIn L, const double* __restrict__ e1t
 template <int N> struct AdjRow {
   static constexpr size_t smem() { return FxRow<N>::smem() + (size_t)3 * FxRow<N>::RT * N * sizeof(double2); }
 };
-#ifndef QG_ADJ_ROW_CTAS
-#define QG_ADJ_ROW_CTAS 2
-#endif
 template <int N>
-__global__ void __launch_bounds__(FxRow<N>::NT, fx_row_ctas<N>(QG_ADJ_ROW_CTAS))
+__global__ void __launch_bounds__(FxRow<N>::NT, fx_row_ctas<N>(2))
 k_adj_row(Geom g, AdjP p, const double2* __restrict__ SF, double2* __restrict__ SA, const double2* __restrict__ twg) {
   using F = FxRow<N>;
   constexpr int NB = F::NB;

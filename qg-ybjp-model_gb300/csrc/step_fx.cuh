@@ -117,11 +117,13 @@ k_fx_row_main(Geom g, StepParams sp, double2* __restrict__ S, const double2* __r
 // ===========================================================================
 // Rows of compute_qw (k_row_qw's planes and results)
 // ===========================================================================
-#ifndef QG_FX_QW_CTAS
-#define QG_FX_QW_CTAS 4
-#endif
+// CTAs per SM that its register budget targets: three leave it 168 registers
+// (us per launch, 4 -> 3: 128^2 x 64 55.2 -> 51.1, 256^2 x 128 399 -> 387),
+// but at N = 512, two warps per row, the fourth CTA pays (3274, with three
+// 3293; five 3543)
+template <int N> __host__ __device__ constexpr int fx_qw_ctas() { return fx_row_ctas<N>(N >= 512 ? 4 : 3); }
 template <int N>
-__global__ void __launch_bounds__(FxRow<N>::NT, fx_row_ctas<N>(QG_FX_QW_CTAS))
+__global__ void __launch_bounds__(FxRow<N>::NT, fx_qw_ctas<N>())
 k_fx_row_qw(Geom g, double2* __restrict__ S, const double2* __restrict__ twg, int nitems, const double2* __restrict__ Qb) {
   using F = FxRow<N>;
   constexpr int NB = F::NB;
