@@ -72,15 +72,16 @@ __device__ __forceinline__ long long fx_mulhi(long long a, long long b) {
 // too).  at places element i in the transform's shared buffer, sync orders
 // the transform's threads, red ORs a word over them (and orders them).
 // At entry the threads are past their last access to the buffer; the slots
-// of a thread's outputs are its own to write afterwards.
+// of a thread's outputs are its own to write afterwards.  ROWS: two packed
+// rows, whose spectra split() separates (fx_top).
 // ===========================================================================
-template <int N, int NS, class P, class Sync, class Red>
+template <int N, int NS, bool ROWS, class P, class Sync, class Red>
 __device__ __forceinline__ void fx_core_pass(fxc (&v)[8], int& base, fxc* __restrict__ buf, const int4* __restrict__ tw,
                                              int j, P at, Sync sync, Red red) {
   constexpr int R = fx_radix(N, NS), NB = N / 8, PER = 8 / R;
   constexpr bool last = NS * R == N, renorm = fx_renorm<N>();
   int s = 0;
-  if constexpr (renorm) s = fx_room(red(fx_bits<8>(v)));    // (orders the earlier pass's stores)
+  if constexpr (renorm) s = fx_room<fx_top<N, ROWS>(NS)>(red(fx_bits<8>(v)));    // (orders the earlier pass's stores)
   else sync();
 #pragma unroll
   for (int p = 0; p < PER; ++p)
@@ -106,17 +107,17 @@ __device__ __forceinline__ void fx_core_pass(fxc (&v)[8], int& base, fxc* __rest
 #pragma unroll
       for (int r = 0; r < R; ++r) buf[at(b + r * NS)] = v[p * R + r];
     }
-    fx_core_pass<N, NS * R>(v, base, buf, tw, j, at, sync, red);
+    fx_core_pass<N, NS * R, ROWS>(v, base, buf, tw, j, at, sync, red);
   }
 }
-template <int N, class P, class Sync, class Red>
+template <int N, bool ROWS, class P, class Sync, class Red>
 __device__ __forceinline__ void fx_core(fxc (&v)[8], int& base, fxc* __restrict__ buf, const int4* __restrict__ tw, int j,
                                         P at, Sync sync, Red red) {
   fx_dft8(v);
 #pragma unroll
   for (int r = 0; r < 8; ++r) buf[at(j * 8 + r)] = v[r];
   base += fx_shift_total<N>();
-  fx_core_pass<N, 8>(v, base, buf, tw, j, at, sync, red);
+  fx_core_pass<N, 8, ROWS>(v, base, buf, tw, j, at, sync, red);
 }
 
 // ===========================================================================
@@ -174,7 +175,7 @@ template <int N, int T = 128> struct FxRowCtx {
     return fx_row_reduce<NB, OR>(m, slots + set, rr);
   }
   __device__ __forceinline__ void core(fxc (&v)[8], int& base) const {
-    fx_core<N>(v, base, buf, tw, j, [](int i) { return fx_idx(i); }, [&]() { sync(); },
+    fx_core<N, true>(v, base, buf, tw, j, [](int i) { return fx_idx(i); }, [&]() { sync(); },
                [&](unsigned m) { return fx_row_reduce<NB, true>(m, slots + 2 * FxRow<N, T>::RT * FxRow<N, T>::W, rr); });
   }
   // inverse transform of the packed spectrum d (PRUNED: zeros at |k| > K) into
@@ -302,7 +303,7 @@ template <int N> struct FxColCtx {
     return fx_ints<8, FWD, PRUNED>(d, v, reduce<false>(fx_maxp<8, PRUNED>(d), 0));
   }
   __device__ __forceinline__ void core(fxc (&v)[8], int& base) const {
-    fx_core<N>(v, base, buf, tw, j, [&](int i) { return fx_idx(i) * F::CT + c; }, []() { __syncthreads(); },
+    fx_core<N, false>(v, base, buf, tw, j, [&](int i) { return fx_idx(i) * F::CT + c; }, []() { __syncthreads(); },
                [&](unsigned m) { return reduce<true>(m, 1); });
   }
   template <bool FWD, bool PRUNED = !FWD> __device__ __forceinline__ void run(double2 (&d)[8], fxc (&v)[8], int& base) const {

@@ -237,9 +237,39 @@ template <int R> __device__ __forceinline__ unsigned fx_bits(const fxc* v) {
   }
   return o;
 }
-// left shift that brings components with these bits below 2^61 (the sums of
-// two outputs of a transform then stay below 2^63)
-__device__ __forceinline__ int fx_room(unsigned o) { return max(__clz((int)o) - 3, 0); }
+// Growth.  A transform's inputs have components below 2^59: a modulus below
+// 2^59.5, or 2^59 for each of two real rows packed as one complex input.  A
+// pass of radix R lets either grow by R / 2^shift at most.  Every output has
+// to stay below 2^63 in modulus; where the rows are then separated (ROWS), the
+// sum of two outputs, twice one row's spectrum, has to as well.  Lengths that
+// renormalise set the modulus back before each later pass, to components
+// below 2^fx_top: 2^61, and 2^60 before a last pass that grows the rows by
+// more than the sums leave room for (n = 1024, whose radix 8 follows a radix
+// 2: there rows beside a zero or much smaller row reached 2^63.5).
+// Twice the base-2 logarithms:
+__host__ __device__ constexpr int fx_grow2(int r, int shift) { return 2 * (fx_log2(r) - shift); }
+template <int N, bool ROWS> __host__ __device__ constexpr int fx_top(int ns) {
+  return ROWS && ns * fx_radix(N, ns) == N && 2 * 61 + 1 + fx_grow2(fx_radix(N, ns), fx_shift<N>(ns)) > 2 * 62 ? 60 : 61;
+}
+template <int N> __host__ __device__ constexpr bool fx_growth_ok() {
+  int mod = 2 * 59 + 1 + 2 * 3, row = 2 * 59 + 2 * 3;     // after the first pass
+  for (int s = 8; s < N; s *= fx_radix(N, s)) {
+    if (fx_renorm<N>()) {                          // (left shifts only)
+      const int top = 2 * fx_top<N, true>(s) + 1;
+      mod = mod > top ? mod : top;
+      row = row > top ? row : top;
+    }
+    const int g = fx_grow2(fx_radix(N, s), fx_shift<N>(s));
+    mod += g;
+    row += g;
+    if (mod >= 2 * 63 || 2 * 61 + 1 + g >= 2 * 63) return false;
+  }
+  return row <= 2 * 62;
+}
+static_assert(fx_growth_ok<16>() && fx_growth_ok<32>() && fx_growth_ok<64>() && fx_growth_ok<128>() && fx_growth_ok<256>() &&
+              fx_growth_ok<512>() && fx_growth_ok<1024>(), "the integers stay in 64 bits");
+// left shift that brings components with these bits below 2^TOP
+template <int TOP> __device__ __forceinline__ int fx_room(unsigned o) { return max(__clz((int)o) - (64 - TOP), 0); }
 template <int R> __device__ __forceinline__ void fx_shl(fxc* v, int s) {
 #pragma unroll
   for (int r = 0; r < R; ++r) { v[r].x <<= s; v[r].y <<= s; }
