@@ -149,20 +149,16 @@ __device__ __forceinline__ double2 rt_scale(double2 v, int kx, int ky, double in
   return (kx == 0 && ky == 0) ? make_double2(2.0 * v.x * inv2n2, 0.0) : cscale(v, inv2n2);
 }
 
-// packed spectrum X + iY of two half spectra get(kk, X, Y) at k = j + r NB
-template <int N, class Get> __device__ __forceinline__ void adj_pack(int j, int K, double2 (&d)[8], Get get) {
+// two half spectra get(kk, X, Y) as fx_half's
+template <int N, class Get> __device__ __forceinline__ void adj_half(int j, int K, double2 (&a)[8], double2 (&b)[8], Get get) {
 #pragma unroll
   for (int r = 0; r < 8; ++r) {
-    d[r] = make_double2(0.0, 0.0);
+    a[r] = b[r] = make_double2(0.0, 0.0);
     if (fx_zero_in<8>(r)) continue;
     const int k = j + r * (N / 8), kk = r < 4 ? k : N - k;
-    if (kk > K) continue;
-    double2 X, Y;
-    get(kk, X, Y);
-    if (k == 0) d[r] = make_double2(X.x, Y.x);           // imaginary parts at kx = 0 are ignored
-    else if (r < 4) d[r] = make_double2(X.x - Y.y, X.y + Y.x);
-    else d[r] = make_double2(X.x + Y.y, Y.x - X.y);
+    if (kk <= K) get(kk, a[r], b[r]);
   }
+  if (j == 0) a[0].y = b[0].y = 0.0;
 }
 
 // y-inverse transforms of one plane of a column tile: get(row, ky) is the
@@ -235,7 +231,7 @@ k_adj_row(Geom g, AdjP p, const double2* __restrict__ SF, double2* __restrict__ 
   using F = FxRow<N>;
   constexpr int NB = F::NB;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ unsigned slots[F::SLOTS];
+  __shared__ uint2 slots[F::SLOTS];
   FxRowCtx<N> c = fx_row_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
   // point (x = j + r NB) of pair q at park[(q * 8 + r) * NT]
   double2* park = reinterpret_cast<double2*>(smem_raw) + fx_tw_count<N>() + F::RT * F::LD + threadIdx.x;
@@ -253,13 +249,13 @@ k_adj_row(Geom g, AdjP p, const double2* __restrict__ SF, double2* __restrict__ 
     const double2 *A = q < 3 ? sf(2 * q) : (q < 6 ? sa(2 * (q - 3)) : sa(4));
     const double2 *B = q < 3 ? sf(2 * q + 1) : (q < 6 ? sa(2 * (q - 3) + 1) : sa(2));
     const double sb = q < 3 ? 1.0 : (q < 6 ? adv : -hr);
-    double2 d[8], o[8];
-    adj_pack<N>(j, K, d, [&](int kk, double2& a, double2& b) {
+    double2 X[8], Y[8], o[8];
+    adj_half<N>(j, K, X, Y, [&](int kk, double2& a, double2& b) {
       a = A[kk];
       b = cscale(B[kk], sb);
       if (q >= 3) a = q < 6 ? cscale(cmul_mi(a), adv * (double)kk) : cscale(a, hr);
     });
-    c.inverse_d(d, o);
+    c.inverse_d(X, Y, o);
     if (q < 3) {
 #pragma unroll
       for (int r = 0; r < 8; ++r) park[(q * 8 + r) * F::NT] = o[r];
@@ -416,52 +412,54 @@ k_adj_qw_row(Geom g, AdjP p, double2* __restrict__ SF, const double2* __restrict
   using F = FxRow<N>;
   constexpr int NB = F::NB;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ unsigned slots[F::SLOTS];
+  __shared__ uint2 slots[F::SLOTS];
   FxRowCtx<N> c = fx_row_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
   const int zb = blockIdx.y, y = blockIdx.x * F::RT + c.rr, K = g.K, j = c.j;
   auto sf = [&](int f) { return SF + scr_off(zb, f, y, N, g.KXP); };
   const double s = p.s;
   fxc l[8], b[8], v[8];
-  int el, eb;
-  double2 d[8];
+  int2 el, eb;
+  double2 X[8], Y[8];
   {
     const double2 *W1 = sf(4), *W2 = sf(5);
-    adj_pack<N>(j, K, d, [&](int kk, double2& X, double2& Y) {
+    adj_half<N>(j, K, X, Y, [&](int kk, double2& x, double2& y2) {
       const double2 w1 = W1[kk], w2 = W2[kk];
-      X = cscale(w1, -s);
-      Y = cscale(cadd(cscale(w1, (double)kk * (double)kk), w2), 0.25 * s);
+      x = cscale(w1, -s);
+      y2 = cscale(cadd(cscale(w1, (double)kk * (double)kk), w2), 0.25 * s);
     });
-    c.inverse(d, l, el);           // l.y: lP1, l.x: lP2
+    c.inverse(X, Y, l, el);        // l.y: lP1, l.x: lP2
   }
+  auto bases = [&](int e, int ex, int ey) { return make_int2(fx_prod_base(e, ex), fx_prod_base(e, ey)); };
   // (a_R, a_I) = lP1 (-BIy, BRy)
-  fx_pack<N>(sf(1), sf(3), j, K, d);
-  c.inverse(d, b, eb);
+  fx_half<N>(sf(1), sf(3), j, K, X, Y);
+  c.inverse(X, Y, b, eb);
 #pragma unroll
   for (int r = 0; r < 8; ++r) { v[r].x = -fx_mulhi(l[r].y, b[r].x); v[r].y = fx_mulhi(l[r].y, b[r].y); }
   double2 aR[3], aI[3];
 #pragma unroll
   for (int q = 0; q < 3; ++q) aR[q] = aI[q] = make_double2(0.0, 0.0);
-  c.forward(v, el + eb - 1023 + 64, K, [&](int q, int, double2 X, double2 Y) { aR[q] = X; aI[q] = Y; });
+  c.forward(v, bases(el.y, eb.x, eb.y), K, [&](int q, int, double2 R, double2 I) { aR[q] = R; aI[q] = I; });
   // (b_R, b_I) = lP1 (BIx, -BRx)
-  fx_pack<N>(sf(0), sf(2), j, K, d);
+  fx_half<N>(sf(0), sf(2), j, K, X, Y);
 #pragma unroll
   for (int r = 0; r < 8; ++r) {
-    const double k = (double)(j + r * NB - (r < 4 ? 0 : N));
-    d[r] = make_double2(-k * d[r].y, k * d[r].x);
+    const double k = (double)(r < 4 ? j + r * NB : N - (j + r * NB));
+    X[r] = make_double2(-k * X[r].y, k * X[r].x);
+    Y[r] = make_double2(-k * Y[r].y, k * Y[r].x);
   }
-  c.inverse(d, b, eb);
+  c.inverse(X, Y, b, eb);
 #pragma unroll
   for (int r = 0; r < 8; ++r) { v[r].x = fx_mulhi(l[r].y, b[r].x); v[r].y = -fx_mulhi(l[r].y, b[r].y); }
-  c.forward(v, el + eb - 1023 + 64, K, [&](int, int k, double2 X, double2 Y) { sf(1)[k] = X; sf(3)[k] = Y; });
+  c.forward(v, bases(el.y, eb.x, eb.y), K, [&](int, int k, double2 R, double2 I) { sf(1)[k] = R; sf(3)[k] = I; });
   // (c_R, c_I) = 2 lP2 (BR, BI)
-  fx_pack<N>(sf(0), sf(2), j, K, d);
-  c.inverse(d, b, eb);
+  fx_half<N>(sf(0), sf(2), j, K, X, Y);
+  c.inverse(X, Y, b, eb);
 #pragma unroll
   for (int r = 0; r < 8; ++r) { v[r].x = fx_mulhi(l[r].x, b[r].y); v[r].y = fx_mulhi(l[r].x, b[r].x); }
-  c.forward(v, el + eb - 1023 + 64 + 1, K, [&](int q, int k, double2 X, double2 Y) {
+  c.forward(v, bases(el.x + 1, eb.y, eb.x), K, [&](int q, int k, double2 R, double2 I) {
     const double kx = (double)k;
-    sf(0)[k] = cadd(cscale(cmul_mi(aR[q]), kx), X);
-    sf(2)[k] = cadd(cscale(cmul_mi(aI[q]), kx), Y);
+    sf(0)[k] = cadd(cscale(cmul_mi(aR[q]), kx), R);
+    sf(2)[k] = cadd(cscale(cmul_mi(aI[q]), kx), I);
   });
 }
 

@@ -217,6 +217,19 @@ __device__ __forceinline__ cplx<T> pack_full(const cplx<T>* X, const cplx<T>* Y,
   return k < n / 2 ? mk<T>(a.x - b.y, a.y + b.x) : mk<T>(a.x + b.y, b.x - a.y);
 }
 
+// the half spectra X, Y of two rows with kx in [0, n/2] as fx_half's, zeros
+// past kx = KM; real at kx = 0 and n/2
+template <int N>
+__device__ __forceinline__ void half_full(const double2* X, const double2* Y, int j, int KM, double2 (&a)[8], double2 (&b)[8]) {
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    a[r] = b[r] = make_double2(0.0, 0.0);
+    const int k = j + r * (N / 8), kk = r < 4 ? k : N - k;
+    if (kk <= KM) { a[r] = X[kk]; b[r] = Y[kk]; }
+  }
+  if (j == 0) a[0].y = b[0].y = a[4].y = b[4].y = 0.0;
+}
+
 // one CTA: RT pairs of rows of level z; W: the level's plane; put(y, x, value)
 // stores the outputs
 template <typename T, int N, class Put>
@@ -225,20 +238,15 @@ __device__ __forceinline__ void drow_c2r(int iktxP, int KM, const cplx<T>* __res
   using D = Dense<T, N>;
   if constexpr (D::FX) {
     constexpr int NB = N / 8;
-    __shared__ unsigned slots[FxRow<N>::SLOTS];
+    __shared__ uint2 slots[FxRow<N>::SLOTS];
     FxRowCtx<N> c = fx_row_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
     const bool live = c.rr < D::RT;
     const int y = 2 * (p0 + c.rr);
     const double2* X = W + (long long)y * iktxP;
-    double2 d[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-      d[r] = live ? pack_full<T>(X, X + iktxP, c.j + r * NB, N, KM) : make_double2(0.0, 0.0);
-    fxc v[8];
-    int base = fx_ints<8, false, false>(d, v, c.template reduce<false>(fx_maxp<8, false>(d)));
-    c.core(v, base);
+    double2 a[8], b[8], d[8];
+    half_full<N>(X, X + iktxP, c.j, live ? KM : -1, a, b);
+    c.template inverse_d<false>(a, b, d);
     if (!live) return;
-    fx_doubles<8, true>(v, d, base);
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
       put(y, c.j + r * NB, d[r].x);
@@ -321,7 +329,7 @@ k_drow_r2c(int iktxP, const double* __restrict__ phys, int ld, cplx<T>* __restri
   W += dense_plane(z, 1, 0, N, iktxP);
   if constexpr (D::FX) {
     constexpr int NB = N / 8;
-    __shared__ unsigned slots[FxRow<N>::SLOTS];
+    __shared__ uint2 slots[FxRow<N>::SLOTS];
     FxRowCtx<N> c = fx_row_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
     const bool live = c.rr < D::RT;
     const int y = 2 * (p0 + c.rr);
@@ -331,11 +339,8 @@ k_drow_r2c(int iktxP, const double* __restrict__ phys, int ld, cplx<T>* __restri
       const double* q = a + y * ld + c.j + r * NB;
       d[r] = live ? make_double2(q[0], q[ld]) : make_double2(0.0, 0.0);
     }
-    fxc v[8];
-    int base = fx_ints<8, true, false>(d, v, c.template reduce<false>(fx_maxp<8, false>(d)));
-    c.core(v, base);
     double2* o = W + (long long)y * iktxP;
-    c.template split<5>(v, base, N / 2, [&](int, int k, double2 X, double2 Y) {
+    c.template forward_d<5>(d, N / 2, [&](int, int k, double2 X, double2 Y) {
       if (!live) return;
       o[k] = X;
       o[iktxP + k] = Y;
@@ -386,23 +391,21 @@ k_drow_prod(int iktxP, int np, int KM, int cross, int scale, int nA, int nX, cpl
   const int nt = cross == 2 ? 6 : (cross == 1 ? 4 : nA + nX);
   if constexpr (D::FX) {
     constexpr int NB = N / 8;
-    __shared__ unsigned slots[FxRow<N>::SLOTS];
+    __shared__ uint2 slots[FxRow<N>::SLOTS];
     FxRowCtx<N> c = fx_row_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
     fxc* park = reinterpret_cast<fxc*>(smem_raw) + fx_tw_count<N>() + FxRow<N>::RT * FxRow<N>::LD + threadIdx.x;   // [2][8][RNT]
     const bool live = c.rr < D::RT;
     const int y = 2 * (p0 + c.rr);
     auto plane = [&](int f) { return W + dense_plane(z, np, f, N, iktxP) + (long long)y * iktxP; };
     fxc x[8], p[8];
-    int ex = 0, e0 = 0, e1 = 0, ep = 0;
+    int2 ex = make_int2(0, 0), e0 = ex, e1 = ex, ep = ex;
 #pragma unroll 1
     for (int t = 0; t < nt; ++t) {
       {
-        double2 d[8];
+        double2 a[8], b[8];
         const double2* X = plane(t);
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-          d[r] = live ? pack_full<T>(X, X + iktxP, c.j + r * NB, N, N / 2) : make_double2(0.0, 0.0);
-        c.template inverse<false>(d, x, ex);
+        half_full<N>(X, X + iktxP, c.j, live ? N / 2 : -1, a, b);
+        c.template inverse<false>(a, b, x, ex);
       }
       const bool keep = cross ? (t == 0 || t == 2) : t < nA;
       if (keep) {
@@ -417,7 +420,10 @@ k_drow_prod(int iktxP, int np, int KM, int cross, int scale, int nA, int nX, cpl
       for (int h = 0; h < nh; ++h) {
         fxc w[8];
         const bool sq = t >= 4 && cross;
-        int base = (sq ? ex : (h ? e1 : e0)) + ex - 1023 + 64 + (cross && !sq ? scale : 0);
+        // (w.x: the first row, whose fields are the parts y)
+        const int2 ea = sq ? ex : (h ? e1 : e0);
+        const int up = cross && !sq ? scale : 0;
+        int2 base = make_int2(fx_prod_base(ea.y, ex.y) + up, fx_prod_base(ea.x, ex.x) + up);
         const fxc* q = park + h * 8 * D::RNT;
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
@@ -432,14 +438,13 @@ k_drow_prod(int iktxP, int np, int KM, int cross, int scale, int nA, int nX, cpl
             for (int r = 0; r < 8; ++r) p[r] = w[r];
             continue;
           }
-          // p -+ w, both to the larger exponent
-          const int s1 = min(max(base - ep, 0), 63), s2 = min(max(ep - base, 0), 63);
-          base = max(base, ep);
+          // p -+ w
+          const FxAlign ax(ep.x, base.x), ay(ep.y, base.y);
+          base = make_int2(ax.e, ay.e);
 #pragma unroll
           for (int r = 0; r < 8; ++r) {
-            const long long wx = w[r].x >> s2, wy = w[r].y >> s2;
-            w[r].x = (p[r].x >> s1) + (sq ? wx : -wx);
-            w[r].y = (p[r].y >> s1) + (sq ? wy : -wy);
+            w[r].x = sq ? ax.add(p[r].x, w[r].x) : ax.sub(p[r].x, w[r].x);
+            w[r].y = sq ? ay.add(p[r].y, w[r].y) : ay.sub(p[r].y, w[r].y);
           }
         }
         double2* o = plane(cross ? (sq ? 1 : 0) : (t - nA) * nA + h);

@@ -883,7 +883,7 @@ class Engine : public EngineBase {
     const int mx = cudaFuncAttributeMaxDynamicSharedMemorySize;
     QG_SWITCH_N(g.n, {
       if constexpr (kFx) {
-        const int sc = (int)FxCol<NN>::smem(), sr = (int)FxRow<NN>::smem();
+        const int sc = (int)FxCol<NN>::smem(), sr = (int)FxQw<NN>::smem();
         QG_CK(cudaFuncSetAttribute(k_fx_col_inv<NN>, (cudaFuncAttribute)mx, sc));
         QG_CK(cudaFuncSetAttribute(k_fx_col_update<NN>, (cudaFuncAttribute)mx, sc));
         QG_CK(cudaFuncSetAttribute(k_fx_col_qw<NN>, (cudaFuncAttribute)mx, sc));
@@ -1089,7 +1089,7 @@ class Engine : public EngineBase {
           if (int rc0 = pbeg(QG_K_ROW_QW, bs)) return rc0;
           if constexpr (kFx) {
             const int items = zc * (NN / FxRow<NN>::RT);
-            k_fx_row_qw<NN><<<std::min(items, std::max(1, nsm * occ_rq / L)), FxRow<NN>::NT, FxRow<NN>::smem(), bs>>>(
+            k_fx_row_qw<NN><<<std::min(items, std::max(1, nsm * occ_rq / L)), FxRow<NN>::NT, FxQw<NN>::smem(), bs>>>(
                 g, Sb, tw, items, Qb);
           } else if constexpr (Tiles<T, NN>::QPRE) {
             const int items = zc * (NN / Tiles<T, NN>::QRT);

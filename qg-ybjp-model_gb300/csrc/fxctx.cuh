@@ -9,18 +9,26 @@ namespace qg {
 // 3N/8): r = 3, 4 are zero for every butterfly
 template <int R> __host__ __device__ constexpr bool fx_zero_in(int r) { return R == 8 && (r == 3 || r == 4); }
 
+// v 2^512 (exact), unless all of it is zero
+template <int R, bool PRUNED> __device__ __forceinline__ void fx_raise(double2* v) {
+  unsigned o = 0;
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (!(PRUNED && fx_zero_in<R>(r)))
+      o |= fx_mag(v[r].x) | fx_mag(v[r].y) | (unsigned)__double2loint(v[r].x) | (unsigned)__double2loint(v[r].y);
+  if (!o) return;
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (!(PRUNED && fx_zero_in<R>(r))) { v[r].x *= 0x1p512; v[r].y *= 0x1p512; }
+}
 // doubles d[R] -> integers below 2^59 (the largest magnitude bits of the whole
 // transform in mag); parts exchanged for the inverse.  Returns the base.
 template <int R, bool FWD, bool PRUNED>
 __device__ __forceinline__ int fx_ints(double2* d, fxc* v, unsigned mag) {
-  int be = (int)(mag >> 20);
-  const int base = be >= 2047 ? kFxNan : max(be, 1) - 58;
-  if (be < kFxTiny) {
-    be = max(be, 1) + 512;
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (!(PRUNED && fx_zero_in<R>(r))) { d[r].x *= 0x1p512; d[r].y *= 0x1p512; }
-  }
+  int be;
+  bool tiny;
+  const int base = fx_base<59>(mag, be, tiny);
+  if (tiny) fx_raise<R, PRUNED>(d);
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     if (PRUNED && fx_zero_in<R>(r)) { v[r].x = v[r].y = 0; continue; }
@@ -42,19 +50,35 @@ template <int R, bool PRUNED> __device__ __forceinline__ unsigned fx_maxp(const 
 // elements in every pass for N >= 64, checked in colfft.cuh)
 __host__ __device__ __forceinline__ constexpr int fx_idx(int i) { return i + (i >> 3); }
 
-// scale v so that its magnitudes, whose high words' bits are in o, fill TOP
-// bits; base follows
-template <int R, int TOP> __device__ __forceinline__ void fx_norm(fxc* v, unsigned o, int& base) {
+// scale one part of v to TOP bits (its magnitudes' high words' bits are in o),
+// to the nearest, base follows; magnitudes below 2^32 gain TOP - 32 bits
+template <int R, int TOP, bool Y> __device__ __forceinline__ void fx_norm1(fxc* v, unsigned o, int& base) {
   const int s = __clz((int)o) - (64 - TOP);
   base -= s;
   if (s >= 0) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) { v[r].x <<= s; v[r].y <<= s; }
+    for (int r = 0; r < R; ++r) (Y ? v[r].y : v[r].x) <<= s;
   } else {
+    const long long h = 1LL << (-s - 1);
 #pragma unroll
-    for (int r = 0; r < R; ++r) { v[r].x >>= -s; v[r].y >>= -s; }
+    for (int r = 0; r < R; ++r) { long long& x = Y ? v[r].y : v[r].x; x = (x + h) >> -s; }
   }
 }
+template <int R, int TOP> __device__ __forceinline__ void fx_norm(fxc* v, uint2 o, int2& base) {
+  fx_norm1<R, TOP, false>(v, o.x, base.x);
+  fx_norm1<R, TOP, true>(v, o.y, base.y);
+}
+// a +- b of the bases ea, eb: integers of the larger one, e, to the nearest
+struct FxAlign {
+  int e, sa, sb;
+  long long ha, hb;
+  __device__ __forceinline__ FxAlign(int ea, int eb)
+      : e(max(ea, eb)), sa(min(e - ea, 62)), sb(min(e - eb, 62)), ha((1LL << sa) >> 1), hb((1LL << sb) >> 1) {}
+  __device__ __forceinline__ long long add(long long a, long long b) const { return ((a + ha) >> sa) + ((b + hb) >> sb); }
+  __device__ __forceinline__ long long sub(long long a, long long b) const { return ((a + ha) >> sa) - ((b + hb) >> sb); }
+};
+// base of a b / 2^64
+__device__ __forceinline__ int fx_prod_base(int ea, int eb) { return ea + eb - 1023 + 64; }
 
 // a b / 2^64 (|a|, |b| < 2^62)
 __device__ __forceinline__ long long fx_mulhi(long long a, long long b) {
@@ -73,13 +97,15 @@ __device__ __forceinline__ long long fx_mulhi(long long a, long long b) {
 // the transform's threads, red ORs a word over them (and orders them).
 // At entry the threads are past their last access to the buffer; the slots
 // of a thread's outputs are its own to write afterwards.  ROWS: two packed
-// rows, whose spectra split() separates (fx_top).
+// rows, whose spectra split() separates (fx_top).  FIT: the second pass takes
+// back the room that the first one's growth left, as every pass does where
+// fx_renorm() holds; the word that this takes rides on the pass's barrier.
 // ===========================================================================
-template <int N, int NS, bool ROWS, class P, class Sync, class Red>
+template <int N, int NS, bool ROWS, bool FIT, class P, class Sync, class Red>
 __device__ __forceinline__ void fx_core_pass(fxc (&v)[8], int& base, fxc* __restrict__ buf, const int4* __restrict__ tw,
                                              int j, P at, Sync sync, Red red) {
   constexpr int R = fx_radix(N, NS), NB = N / 8, PER = 8 / R;
-  constexpr bool last = NS * R == N, renorm = fx_renorm<N>();
+  constexpr bool last = NS * R == N, renorm = fx_renorm<N>() || (FIT && NS == 8);
   int s = 0;
   if constexpr (renorm) s = fx_room<fx_top<N, ROWS>(NS)>(red(fx_bits<8>(v)));    // (orders the earlier pass's stores)
   else sync();
@@ -107,17 +133,17 @@ __device__ __forceinline__ void fx_core_pass(fxc (&v)[8], int& base, fxc* __rest
 #pragma unroll
       for (int r = 0; r < R; ++r) buf[at(b + r * NS)] = v[p * R + r];
     }
-    fx_core_pass<N, NS * R, ROWS>(v, base, buf, tw, j, at, sync, red);
+    fx_core_pass<N, NS * R, ROWS, FIT>(v, base, buf, tw, j, at, sync, red);
   }
 }
-template <int N, bool ROWS, class P, class Sync, class Red>
+template <int N, bool ROWS, bool FIT, class P, class Sync, class Red>
 __device__ __forceinline__ void fx_core(fxc (&v)[8], int& base, fxc* __restrict__ buf, const int4* __restrict__ tw, int j,
                                         P at, Sync sync, Red red) {
   fx_dft8(v);
 #pragma unroll
   for (int r = 0; r < 8; ++r) buf[at(j * 8 + r)] = v[r];
   base += fx_shift_total<N>();
-  fx_core_pass<N, 8, ROWS>(v, base, buf, tw, j, at, sync, red);
+  fx_core_pass<N, 8, ROWS, FIT>(v, base, buf, tw, j, at, sync, red);
 }
 
 // ===========================================================================
@@ -129,7 +155,7 @@ template <int N, int T = 128> struct FxRow {
   static constexpr int RT = T / NB < N ? T / NB : N;      // rows per CTA of T threads
   static constexpr int NT = RT * NB;                      // threads per CTA
   static constexpr int W = NB > 32 ? NB / 32 : 1;         // warps per row
-  static constexpr int SLOTS = 3 * RT * W;
+  static constexpr int SLOTS = 3 * RT * W;             // (pairs)
   static constexpr size_t smem() { return (size_t)(fx_tw_count<N>() + RT * LD) * sizeof(double2); }
 };
 
@@ -137,72 +163,127 @@ template <int NB> __device__ __forceinline__ void fx_row_sync(int rr) {
   if constexpr (NB <= 32) __syncwarp();
   else asm volatile("bar.sync %0, %1;" ::"r"(1 + rr), "n"(NB) : "memory");
 }
-// maximum or bitwise OR of m over the row's threads; orders them too
-template <int NB, bool OR> __device__ __forceinline__ unsigned fx_row_reduce(unsigned m, unsigned* slots, int rr) {
+// maximum or bitwise OR of m's parts over the row's threads; orders them too
+template <int NB, bool OR> __device__ __forceinline__ uint2 fx_row_reduce(uint2 m, uint2* slots, int rr) {
   if constexpr (NB >= 32) {
-    m = OR ? __reduce_or_sync(0xffffffffu, m) : __reduce_max_sync(0xffffffffu, m);
+    m.x = OR ? __reduce_or_sync(0xffffffffu, m.x) : __reduce_max_sync(0xffffffffu, m.x);
+    m.y = OR ? __reduce_or_sync(0xffffffffu, m.y) : __reduce_max_sync(0xffffffffu, m.y);
   } else {
 #pragma unroll
     for (int o = 1; o < NB; o <<= 1) {
-      const unsigned x = __shfl_xor_sync(0xffffffffu, m, o);
-      m = OR ? (m | x) : max(m, x);
+      const unsigned x = __shfl_xor_sync(0xffffffffu, m.x, o), y = __shfl_xor_sync(0xffffffffu, m.y, o);
+      m.x = OR ? (m.x | x) : max(m.x, x);
+      m.y = OR ? (m.y | y) : max(m.y, y);
     }
   }
   if constexpr (NB <= 32) {
     __syncwarp();
   } else {
     constexpr int W = NB / 32;
-    unsigned* s = slots + rr * W;
+    uint2* s = slots + rr * W;
     if ((threadIdx.x & 31) == 0) s[(threadIdx.x >> 5) % W] = m;
     fx_row_sync<NB>(rr);
 #pragma unroll
-    for (int i = 0; i < W; ++i) m = OR ? (m | s[i]) : max(m, s[i]);
+    for (int i = 0; i < W; ++i) {
+      m.x = OR ? (m.x | s[i].x) : max(m.x, s[i].x);
+      m.y = OR ? (m.y | s[i].y) : max(m.y, s[i].y);
+    }
   }
   return m;
 }
 
-// The thread's view of its row: transforms of eight values per thread.
+// The thread's view of its row pair: transforms of eight values per thread.
+// Two real rows are packed as one complex row, and each has a scale of its own
+// (a base per part), as two transforms would.  With one scale for both, a row
+// 2^-m of its neighbour lost m of its bits, beside a uniform neighbour too,
+// which a floating-point transform does not mix into it.  Scales of their own
+// cost 6 % of k_fx_row_main and 7-13 % of k_fx_row_qw (512^2 x 256: 6400 ->
+// 6840 and 3260 -> 3480 us).
 template <int N, int T = 128> struct FxRowCtx {
   static constexpr int NB = N / 8;
   fxc* buf;
   const int4* tw;
-  unsigned* slots;     // three sets of [RT][W]
+  uint2* slots;        // three sets of [RT][W]
   int rr, j;
   int set = 0;         // reductions alternate between two sets: one follows another without a further barrier
   __device__ __forceinline__ void sync() const { fx_row_sync<NB>(rr); }
-  template <bool OR> __device__ __forceinline__ unsigned reduce(unsigned m) {
+  template <bool OR> __device__ __forceinline__ uint2 reduce(uint2 m) {
     set ^= FxRow<N, T>::RT * FxRow<N, T>::W;
     return fx_row_reduce<NB, OR>(m, slots + set, rr);
   }
-  __device__ __forceinline__ void core(fxc (&v)[8], int& base) const {
-    fx_core<N, true>(v, base, buf, tw, j, [](int i) { return fx_idx(i); }, [&]() { sync(); },
-               [&](unsigned m) { return fx_row_reduce<NB, true>(m, slots + 2 * FxRow<N, T>::RT * FxRow<N, T>::W, rr); });
+  template <bool FIT> __device__ __forceinline__ void core(fxc (&v)[8], int2& base) const {
+    int up = 0;
+    fx_core<N, true, FIT>(v, up, buf, tw, j, [](int i) { return fx_idx(i); }, [&]() { sync(); }, [&](unsigned m) {
+      return fx_row_reduce<NB, true>(make_uint2(m, 0u), slots + 2 * FxRow<N, T>::RT * FxRow<N, T>::W, rr).x;
+    });
+    base.x += up;
+    base.y += up;
   }
-  // inverse transform of the packed spectrum d (PRUNED: zeros at |k| > K) into
-  // integers of 61 bits: v.y the first (real) row, v.x the second
-  template <bool PRUNED = true> __device__ __forceinline__ void inverse(double2 (&d)[8], fxc (&v)[8], int& base) {
-    base = fx_ints<8, false, PRUNED>(d, v, reduce<false>(fx_maxp<8, PRUNED>(d)));
-    core(v, base);
-    fx_norm<8, 61>(v, reduce<true>(fx_bits<8>(v)), base);
+  // integers of the packed spectrum of two rows, parts exchanged for the
+  // inverse (v.y, base.y: the first row), from the half spectra a, b at
+  // kk = j + r NB, or N - j - r NB for r >= 4 (PRUNED: zeros at |k| > K), real
+  // at kk = 0 and N/2.  58 bits for each row, so that their sums stay below
+  // 2^59 (packed as doubles, the smaller values of a row would be rounded
+  // against the other row's); core<true> takes the room back.
+  template <bool PRUNED> __device__ __forceinline__ int2 ints_inverse(double2 (&a)[8], double2 (&b)[8], fxc (&v)[8]) {
+    const uint2 m = reduce<false>(make_uint2(fx_maxp<8, PRUNED>(a), fx_maxp<8, PRUNED>(b)));
+    int ea, eb;
+    bool ta, tb;
+    int2 base;
+    base.y = fx_base<58>(m.x, ea, ta);
+    base.x = fx_base<58>(m.y, eb, tb);
+    if (ta) fx_raise<8, PRUNED>(a);
+    if (tb) fx_raise<8, PRUNED>(b);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      if (PRUNED && fx_zero_in<8>(r)) { v[r].x = v[r].y = 0; continue; }
+      fxc x, y;
+      x.x = fx_in1<58>(a[r].x, ea); x.y = fx_in1<58>(a[r].y, ea);
+      y.x = fx_in1<58>(b[r].x, eb); y.y = fx_in1<58>(b[r].y, eb);
+      if (r < 4) { v[r].y = x.x - y.y; v[r].x = x.y + y.x; }
+      else { v[r].y = x.x + y.y; v[r].x = y.x - x.y; }
+    }
+    return base;
   }
-  // inverse transform of the packed spectrum d into doubles: o.x the first
-  // row, o.y the second
-  __device__ __forceinline__ void inverse_d(double2 (&d)[8], double2 (&o)[8]) {
+  // inverse transform of the packed spectrum into integers of 61 bits: v.y the
+  // first row, v.x the second
+  template <bool PRUNED = true> __device__ __forceinline__ void inverse(double2 (&a)[8], double2 (&b)[8], fxc (&v)[8], int2& base) {
+    base = ints_inverse<PRUNED>(a, b, v);
+    core<true>(v, base);
+    fx_norm<8, 61>(v, reduce<true>(fx_bits2<8>(v)), base);
+  }
+  // ... into doubles: o.x the first row, o.y the second
+  template <bool PRUNED = true> __device__ __forceinline__ void inverse_d(double2 (&a)[8], double2 (&b)[8], double2 (&o)[8]) {
     fxc v[8];
-    int base = fx_ints<8, false, true>(d, v, reduce<false>(fx_maxp<8, true>(d)));
-    core(v, base);
+    int2 base = ints_inverse<PRUNED>(a, b, v);
+    core<true>(v, base);
     fx_doubles<8, true>(v, o, base);
   }
-  // forward transform of the packed rows d and its split
-  template <class Put> __device__ __forceinline__ void forward_d(double2 (&d)[8], int K, Put put) {
+  // forward transform of the packed rows d (x the first, y the second) and its split
+  template <int Q = 3, class Put> __device__ __forceinline__ void forward_d(double2 (&d)[8], int K, Put put) {
+    uint2 m = make_uint2(0u, 0u);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) { m.x = max(m.x, fx_mag(d[r].x)); m.y = max(m.y, fx_mag(d[r].y)); }
+    m = reduce<false>(m);
+    int ex, ey;
+    bool tx, ty;
+    int2 base;
+    base.x = fx_base<59>(m.x, ex, tx);
+    base.y = fx_base<59>(m.y, ey, ty);
     fxc v[8];
-    int base = fx_ints<8, true, false>(d, v, reduce<false>(fx_maxp<8, false>(d)));
-    core(v, base);
-    split<3>(v, base, K, put);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      if (tx) d[r].x *= 0x1p512;
+      if (ty) d[r].y *= 0x1p512;
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) { v[r].x = fx_in1(d[r].x, ex); v[r].y = fx_in1(d[r].y, ey); }
+    core<false>(v, base);
+    split<Q>(v, base, K, put);
   }
   // the spectra of the two packed rows from their transform's outputs v, at
   // k = j + q NB <= KM, q < Q: put(q, k, X, Y)
-  template <int Q, class Put> __device__ __forceinline__ void split(const fxc (&v)[8], int base, int KM, Put put) const {
+  template <int Q, class Put> __device__ __forceinline__ void split(const fxc (&v)[8], int2 base, int KM, Put put) const {
 #pragma unroll
     for (int r = 0; r < 8; ++r)
       if (Q > 3 || !fx_zero_in<8>(r)) buf[fx_idx(j + r * NB)] = v[r];
@@ -211,29 +292,29 @@ template <int N, int T = 128> struct FxRowCtx {
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
       // X = (F[k] + conj F[N-k]) / 2, Y = (F[k] - conj F[N-k]) / (2 i): the
-      // sums stay below 2^63 (each row's spectrum is at most 2^62)
+      // sums stay below 2^63 (each row's spectrum is at most 2^62: fx_growth_ok)
       const int k = j + q * NB;
       const fxc a = v[q], b = buf[fx_idx(k == 0 ? 0 : N - k)];
-      s[2 * q].x = a.x + b.x; s[2 * q].y = a.y - b.y;
-      s[2 * q + 1].x = a.y + b.y; s[2 * q + 1].y = b.x - a.x;
+      s[q].x = a.x + b.x; s[q].y = a.y - b.y;
+      s[Q + q].x = a.y + b.y; s[Q + q].y = b.x - a.x;
     }
     double2 o[2 * Q];
-    fx_doubles<2 * Q, false>(s, o, base - 1);
+    fx_doubles<Q, false>(s, o, base.x - 1);
+    fx_doubles<Q, false>(s + Q, o + Q, base.y - 1);
 #pragma unroll
     for (int q = 0; q < Q; ++q)
-      if (j + q * NB <= KM) put(q, j + q * NB, o[2 * q], o[2 * q + 1]);
+      if (j + q * NB <= KM) put(q, j + q * NB, o[q], o[Q + q]);
   }
   // forward transform of the integers v (two packed rows) and its split
-  template <int Q = 3, class Put> __device__ __forceinline__ void forward(fxc (&v)[8], int base, int K, Put put) {
-    const unsigned o = reduce<true>(fx_bits<8>(v));
-    fx_norm<8, 59>(v, o, base);
-    core(v, base);
+  template <int Q = 3, class Put> __device__ __forceinline__ void forward(fxc (&v)[8], int2 base, int K, Put put) {
+    fx_norm<8, 59>(v, reduce<true>(fx_bits2<8>(v)), base);
+    core<false>(v, base);
     split<Q>(v, base, K, put);
   }
 };
 
 template <int N, int T = 128>
-__device__ __forceinline__ FxRowCtx<N, T> fx_row_ctx(double2* smem, unsigned* slots, const double2* twg) {
+__device__ __forceinline__ FxRowCtx<N, T> fx_row_ctx(double2* smem, uint2* slots, const double2* twg) {
   using F = FxRow<N, T>;
   fx_load_tw<N>(smem, twg, F::NT);
   __syncthreads();
@@ -246,25 +327,20 @@ __device__ __forceinline__ FxRowCtx<N, T> fx_row_ctx(double2* smem, unsigned* sl
   return c;
 }
 
-// packed spectrum X + iY of two half spectra at k = j + r NB
+// the half spectra X, Y of two rows at kk = k (r < 4) or N - k, k = j + r NB,
+// zeros past K (ints_inverse); the imaginary parts at kk = 0 are ignored, as a
+// c2r does
 template <int N>
-__device__ __forceinline__ void fx_pack(const double2* __restrict__ X, const double2* __restrict__ Y, int j, int K,
-                                        double2 (&d)[8]) {
-  constexpr int NB = N / 8;
-  double2 a[8], b[8];
+__device__ __forceinline__ void fx_half(const double2* __restrict__ X, const double2* __restrict__ Y, int j, int K,
+                                        double2 (&a)[8], double2 (&b)[8]) {
 #pragma unroll
   for (int r = 0; r < 8; ++r) {
     a[r] = b[r] = make_double2(0.0, 0.0);
     if (fx_zero_in<8>(r)) continue;
-    const int k = j + r * NB, kk = r < 4 ? k : N - k;
+    const int k = j + r * (N / 8), kk = r < 4 ? k : N - k;
     if (kk <= K) { a[r] = X[kk]; b[r] = Y[kk]; }
   }
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    if (r < 4) d[r] = make_double2(a[r].x - b[r].y, a[r].y + b[r].x);
-    else d[r] = make_double2(a[r].x + b[r].y, b[r].x - a[r].y);
-  }
-  if (j == 0) d[0] = make_double2(a[0].x, b[0].x);     // imaginary parts at kx = 0 are ignored, as a c2r does
+  if (j == 0) a[0].y = b[0].y = 0.0;
 }
 
 // ===========================================================================
@@ -303,7 +379,7 @@ template <int N> struct FxColCtx {
     return fx_ints<8, FWD, PRUNED>(d, v, reduce<false>(fx_maxp<8, PRUNED>(d), 0));
   }
   __device__ __forceinline__ void core(fxc (&v)[8], int& base) const {
-    fx_core<N, false>(v, base, buf, tw, j, [&](int i) { return fx_idx(i) * F::CT + c; }, []() { __syncthreads(); },
+    fx_core<N, false, false>(v, base, buf, tw, j, [&](int i) { return fx_idx(i) * F::CT + c; }, []() { __syncthreads(); },
                [&](unsigned m) { return reduce<true>(m, 1); });
   }
   template <bool FWD, bool PRUNED = !FWD> __device__ __forceinline__ void run(double2 (&d)[8], fxc (&v)[8], int& base) const {

@@ -175,15 +175,28 @@ __device__ __forceinline__ unsigned fx_mag(double x) { return (unsigned)__double
 // transforms whose largest biased exponent is below this are scaled by 2^512
 // first (exact), so that subnormal inputs need no case of their own
 constexpr int kFxTiny = 64;
-// x 2^(59-E) truncated, be >= kFxTiny the largest biased exponent (E = be - 1022)
-__device__ __forceinline__ long long fx_in1(double x, int be) {
+// Exponents: an integer m stands for m 2^(base-1023).  kFxNan: a transform
+// with a non-finite input (bases are sums of a few of these).
+constexpr int kFxNan = 1 << 20;
+// x 2^(BITS-E) truncated, be >= kFxTiny the largest biased exponent (E = be - 1022)
+template <int BITS = 59> __device__ __forceinline__ long long fx_in1(double x, int be) {
   const int hi = __double2hiint(x);
   const unsigned lo = (unsigned)__double2loint(x);
   const int d = min(be - ((hi >> 20) & 0x7ff), 63);
-  unsigned long long m = ((unsigned long long)((hi & 0xfffff) | 0x100000) << 32 | lo) << 6;
+  unsigned long long m = ((unsigned long long)((hi & 0xfffff) | 0x100000) << 32 | lo) << (BITS - 53);
   m >>= d;
   const long long s = (long long)(hi >> 31);
   return ((long long)m ^ s) - s;
+}
+// the base of integers of BITS bits whose largest magnitude bits are mag; be:
+// the exponent that fx_in1 takes, and whether its inputs are scaled by 2^512
+// first
+template <int BITS> __device__ __forceinline__ int fx_base(unsigned mag, int& be, bool& tiny) {
+  be = (int)(mag >> 20);
+  const int base = be >= 2047 ? kFxNan : max(be, 1) - (BITS - 1);
+  tiny = be < kFxTiny;
+  if (tiny) be = max(be, 1) + 512;
+  return base;
 }
 // m 2^(base-1075-...) to the nearest double: base is the biased exponent of
 // the integer's bit 0, 1 <= base and base + 63 <= 2046
@@ -196,9 +209,6 @@ __device__ __forceinline__ double fx_out1(long long m, int base) {
   r = a ? r : 0ull;
   return __longlong_as_double((long long)(r | ((unsigned long long)s & 0x8000000000000000ull)));
 }
-// Exponents: an integer m stands for m 2^(base-1023).  kFxNan: a transform
-// with a non-finite input (bases are sums of a few of these).
-constexpr int kFxNan = 1 << 20;
 __device__ __forceinline__ bool fx_is_nan(int base) { return base > (1 << 18); }
 // whether every integer's double is a normal number (or zero)
 __device__ __forceinline__ bool fx_fast(int base) { return base >= 1 && base + 63 <= 2046; }
@@ -207,35 +217,49 @@ __device__ __forceinline__ double fx_pow2(int e) { return __hiloint2double((e + 
 // o <- o 2^(base-1023) for normal o in [1, 2^63] or 0, at scales where the
 // result may be subnormal, zero, infinite or NaN: three exact powers of two,
 // of which only the last can round
-template <int M> __device__ __forceinline__ void fx_rescale(double2* o, int base) {
-  const int e = min(max(base - 1023, -2400), 2400), t = e / 3;
-  const double a = fx_is_nan(base) ? __longlong_as_double(0x7ff8000000000000ll) : fx_pow2(t), b = fx_pow2(t),
-               c = fx_pow2(e - 2 * t);
-#pragma unroll
-  for (int r = 0; r < M; ++r) { o[r].x = ((o[r].x * a) * b) * c; o[r].y = ((o[r].y * a) * b) * c; }
-}
-// doubles of the integers v 2^(base-1023), M complex values; SWAP exchanges
-// the parts.  One branch for all of them: a rescaling per value was predicated
-// into every conversion and made the kernels 25-50 % slower.
-template <int M, bool SWAP> __device__ __forceinline__ void fx_doubles(const fxc* v, double2* o, int base) {
-  const bool fast = fx_fast(base);
-  const int b = fast ? base : 1023;
+struct FxScale {
+  double a, b, c;
+  __device__ __forceinline__ explicit FxScale(int base) {
+    const int e = min(max(base - 1023, -2400), 2400), t = e / 3;
+    a = fx_is_nan(base) ? __longlong_as_double(0x7ff8000000000000ll) : fx_pow2(t);
+    b = fx_pow2(t);
+    c = fx_pow2(e - 2 * t);
+  }
+  __device__ __forceinline__ double operator()(double o) const { return ((o * a) * b) * c; }
+};
+// doubles of the integers v, M complex values with parts x 2^(base.x-1023),
+// y 2^(base.y-1023); SWAP exchanges the parts.  One branch for all of them: a
+// rescaling per value was predicated into every conversion and made the
+// kernels 25-50 % slower.
+template <int M, bool SWAP> __device__ __forceinline__ void fx_doubles(const fxc* v, double2* o, int2 base) {
+  const bool fast = fx_fast(base.x) && fx_fast(base.y);
+  const int bx = fast ? base.x : 1023, by = fast ? base.y : 1023;
 #pragma unroll
   for (int r = 0; r < M; ++r) {
-    const double x = fx_out1(v[r].x, b), y = fx_out1(v[r].y, b);
+    const double x = fx_out1(v[r].x, bx), y = fx_out1(v[r].y, by);
     o[r] = SWAP ? make_double2(y, x) : make_double2(x, y);
   }
-  if (!fast) fx_rescale<M>(o, base);
-}
-// bits set in any of the magnitudes' high words (x ^ sign)
-template <int R> __device__ __forceinline__ unsigned fx_bits(const fxc* v) {
-  unsigned o = 0;
+  if (!fast) {
+    const FxScale sx(SWAP ? base.y : base.x), sy(SWAP ? base.x : base.y);
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int a = (int)(v[r].x >> 32), b = (int)(v[r].y >> 32);
-    o |= (unsigned)(a ^ (a >> 31)) | (unsigned)(b ^ (b >> 31));
+    for (int r = 0; r < M; ++r) { o[r].x = sx(o[r].x); o[r].y = sy(o[r].y); }
   }
+}
+template <int M, bool SWAP> __device__ __forceinline__ void fx_doubles(const fxc* v, double2* o, int base) {
+  fx_doubles<M, SWAP>(v, o, make_int2(base, base));
+}
+// bits set in any of the magnitudes' high words (x ^ sign): of the parts x, of
+// the parts y, of both
+__device__ __forceinline__ unsigned fx_hibits(long long x) { const int a = (int)(x >> 32); return (unsigned)(a ^ (a >> 31)); }
+template <int R> __device__ __forceinline__ uint2 fx_bits2(const fxc* v) {
+  uint2 o = make_uint2(0u, 0u);
+#pragma unroll
+  for (int r = 0; r < R; ++r) { o.x |= fx_hibits(v[r].x); o.y |= fx_hibits(v[r].y); }
   return o;
+}
+template <int R> __device__ __forceinline__ unsigned fx_bits(const fxc* v) {
+  const uint2 o = fx_bits2<R>(v);
+  return o.x | o.y;
 }
 // Growth.  A transform's inputs have components below 2^59: a modulus below
 // 2^59.5, or 2^59 for each of two real rows packed as one complex input.  A
@@ -251,10 +275,10 @@ __host__ __device__ constexpr int fx_grow2(int r, int shift) { return 2 * (fx_lo
 template <int N, bool ROWS> __host__ __device__ constexpr int fx_top(int ns) {
   return ROWS && ns * fx_radix(N, ns) == N && 2 * 61 + 1 + fx_grow2(fx_radix(N, ns), fx_shift<N>(ns)) > 2 * 62 ? 60 : 61;
 }
-template <int N> __host__ __device__ constexpr bool fx_growth_ok() {
+template <int N> __host__ __device__ constexpr bool fx_growth_ok(bool fit) {
   int mod = 2 * 59 + 1 + 2 * 3, row = 2 * 59 + 2 * 3;     // after the first pass
   for (int s = 8; s < N; s *= fx_radix(N, s)) {
-    if (fx_renorm<N>()) {                          // (left shifts only)
+    if (fx_renorm<N>() || (fit && s == 8)) {      // (left shifts only)
       const int top = 2 * fx_top<N, true>(s) + 1;
       mod = mod > top ? mod : top;
       row = row > top ? row : top;
@@ -266,6 +290,7 @@ template <int N> __host__ __device__ constexpr bool fx_growth_ok() {
   }
   return row <= 2 * 62;
 }
+template <int N> __host__ __device__ constexpr bool fx_growth_ok() { return fx_growth_ok<N>(false) && fx_growth_ok<N>(true); }
 static_assert(fx_growth_ok<16>() && fx_growth_ok<32>() && fx_growth_ok<64>() && fx_growth_ok<128>() && fx_growth_ok<256>() &&
               fx_growth_ok<512>() && fx_growth_ok<1024>(), "the integers stay in 64 bits");
 // left shift that brings components with these bits below 2^TOP

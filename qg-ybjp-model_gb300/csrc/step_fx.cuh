@@ -40,7 +40,7 @@ k_fx_row_main(Geom g, StepParams sp, double2* __restrict__ S, const double2* __r
               const double2* __restrict__ Qb) {
   using F = typename FxMain<N>::F;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ unsigned slots[F::SLOTS];
+  __shared__ uint2 slots[F::SLOTS];
   FxRowCtx<N, kFxMainT> c = fx_row_ctx<N, kFxMainT>(reinterpret_cast<double2*>(smem_raw), slots, twg);
   fxc* zq = reinterpret_cast<fxc*>(smem_raw) + fx_tw_count<N>() + F::RT * F::LD + threadIdx.x;   // point r at zq[r * NT]
   fxc* bb = zq + 8 * F::NT;
@@ -55,15 +55,15 @@ k_fx_row_main(Geom g, StepParams sp, double2* __restrict__ S, const double2* __r
     // per use the kernel's code outgrew the instruction cache, with one copy
     // for both directions the loop's selects cost as much
     fxc uv[8];
-    int ezq = 0, ebb = 0, euv = 0;
+    int2 ezq = make_int2(0, 0), ebb = ezq, euv = ezq;      // (.y: zeta, BR, u; .x: q, BI, v)
 #pragma unroll 1
     for (int t = 0; t < 3; ++t) {
       const double2 *X = plane(0), *Y = plane(1);
       if (t == 0) { X = plane(2); Y = plane(3); }
       else if (t == 1) { X = Qb ? Qb + q_off(zb, 0, y, N, g.KXP) : plane(4); Y = Qb ? Qb + q_off(zb, 1, y, N, g.KXP) : plane(5); }
-      double2 d[8];
-      fx_pack<N>(X, Y, j, K, d);
-      c.inverse(d, uv, euv);
+      double2 a[8], b[8];
+      fx_half<N>(X, Y, j, K, a, b);
+      c.inverse(a, b, uv, euv);
       if (t < 2) {
         if (t == 0) ezq = euv;
         else ebb = euv;
@@ -78,9 +78,10 @@ k_fx_row_main(Geom g, StepParams sp, double2* __restrict__ S, const double2* __r
 #pragma unroll 1
     for (int f = sp.refr ? -1 : 0; f < 3; ++f) {
       fxc w[8];
-      int base;
+      int2 base;
       if (f < 0) {
-        base = ezq + ebb - 1023 + 63;      // (one exponent less: half of the spectra enters planes 2 and 4)
+        // (one exponent less: half of the spectra enters planes 2 and 4)
+        base = make_int2(fx_prod_base(ezq.y, ebb.y) - 1, fx_prod_base(ezq.y, ebb.x) - 1);
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
           const long long z = zq[r * F::NT].y;
@@ -89,7 +90,8 @@ k_fx_row_main(Geom g, StepParams sp, double2* __restrict__ S, const double2* __r
           w[r].y = fx_mulhi(z, b.x);
         }
       } else {
-        base = euv + (f == 0 ? ezq : ebb) - 1023 + 64;
+        const int ex = f == 0 ? ezq.x : (f == 1 ? ebb.y : ebb.x);
+        base = make_int2(fx_prod_base(euv.y, ex), fx_prod_base(euv.x, ex));
         const long long* px = f == 0 ? &zq->x : (f == 1 ? &bb->y : &bb->x);
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
@@ -117,10 +119,16 @@ k_fx_row_main(Geom g, StepParams sp, double2* __restrict__ S, const double2* __r
 // ===========================================================================
 // Rows of compute_qw (k_row_qw's planes and results)
 // ===========================================================================
+// (BRx, BIx) are parked in shared memory, each thread its own eight points: in
+// registers beside two rows' spectra they spilled (us per launch, registers ->
+// shared: 128^2 x 64 57 -> 53, 256^2 x 128 460 -> 432, 512^2 x 256 3730 -> 3490)
+template <int N> struct FxQw {
+  using F = FxRow<N>;
+  static constexpr size_t smem() { return F::smem() + (size_t)F::RT * N * sizeof(fxc); }
+};
 // CTAs per SM that its register budget targets: three leave it 168 registers
-// (us per launch, 4 -> 3: 128^2 x 64 55.2 -> 51.1, 256^2 x 128 399 -> 387),
-// but at N = 512, two warps per row, the fourth CTA pays (3274, with three
-// 3293; five 3543)
+// (us per launch, four -> three: 64^2 x 64 20.4 -> 18.3, 128^2 x 64 59 -> 53,
+// 256^2 x 128 the same); at N = 512, two warps per row, the fourth CTA paid
 template <int N> __host__ __device__ constexpr int fx_qw_ctas() { return fx_row_ctas<N>(N >= 512 ? 4 : 3); }
 template <int N>
 __global__ void __launch_bounds__(FxRow<N>::NT, fx_qw_ctas<N>())
@@ -128,8 +136,9 @@ k_fx_row_qw(Geom g, double2* __restrict__ S, const double2* __restrict__ twg, in
   using F = FxRow<N>;
   constexpr int NB = F::NB;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ unsigned slots[F::SLOTS];
+  __shared__ uint2 slots[F::SLOTS];
   FxRowCtx<N> c = fx_row_ctx<N>(reinterpret_cast<double2*>(smem_raw), slots, twg);
+  fxc* park = reinterpret_cast<fxc*>(smem_raw) + fx_tw_count<N>() + F::RT * F::LD + threadIdx.x;   // point r at park[r * NT]
   const int K = g.K, j = c.j;
   constexpr int NG = N / F::RT;
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
@@ -139,47 +148,52 @@ k_fx_row_qw(Geom g, double2* __restrict__ S, const double2* __restrict__ twg, in
     const double2* pi = Qb ? Qb + q_off(zb, 1, y, N, g.KXP) : plane(4);
     // inverse transforms of (BRx, BIx), (BRy, BIy), (BR, BI), then the forward
     // transform of (P1, P2), through one copy of the transform
-    fxc a[8], p[8], w[8];
-    int ea = 0, e1 = 0, base = 0;
+    fxc w[8];
+    long long p[8];
+    int2 ea = make_int2(0, 0), base = ea;     // (.y: BRx, BRy, BR; .x: BIx, BIy, BI; then P2 and P1)
+    int ep = 0;
 #pragma unroll 1
     for (int t = 0; t < 4; ++t) {
       if (t < 3) {
-        double2 d[8];
-        fx_pack<N>(t == 1 ? plane(3) : pr, t == 1 ? plane(5) : pi, j, K, d);
+        double2 X[8], Y[8];
+        fx_half<N>(t == 1 ? plane(3) : pr, t == 1 ? plane(5) : pi, j, K, X, Y);
         if (t == 0) {
-          // i kx times the packed spectrum of (BR, BI)
+          // i kx times both
 #pragma unroll
           for (int r = 0; r < 8; ++r) {
-            const double k = (double)(j + r * NB - (r < 4 ? 0 : N));
-            d[r] = make_double2(-k * d[r].y, k * d[r].x);
+            const double k = (double)(r < 4 ? j + r * NB : N - (j + r * NB));
+            X[r] = make_double2(-k * X[r].y, k * X[r].x);
+            Y[r] = make_double2(-k * Y[r].y, k * Y[r].x);
           }
         }
-        base = fx_ints<8, false, true>(d, w, c.template reduce<false>(fx_maxp<8, true>(d)));
+        base = c.template ints_inverse<true>(X, Y, w);
       } else {
-        fx_norm<8, 59>(w, c.template reduce<true>(fx_bits<8>(w)), base);
+        fx_norm<8, 59>(w, c.template reduce<true>(fx_bits2<8>(w)), base);
       }
-      c.core(w, base);
-      if (t < 3) fx_norm<8, 61>(w, c.template reduce<true>(fx_bits<8>(w)), base);
+      c.template core<true>(w, base);
+      if (t < 3) fx_norm<8, 61>(w, c.template reduce<true>(fx_bits2<8>(w)), base);
       if (t == 0) {
 #pragma unroll
-        for (int r = 0; r < 8; ++r) a[r] = w[r];
+        for (int r = 0; r < 8; ++r) park[r * F::NT] = w[r];
         ea = base;
       } else if (t == 1) {
         // P1 = BRy BIx - BRx BIy (derivatives.f90:973)
-#pragma unroll
-        for (int r = 0; r < 8; ++r) p[r].x = fx_mulhi(w[r].y, a[r].x) - fx_mulhi(a[r].y, w[r].x);
-        e1 = ea + base - 1023 + 64;
-      } else if (t == 2) {
-        // P2 = BR^2 + BI^2 (derivatives.f90:996), then both to the larger exponent
-        const int e2 = 2 * base - 1023 + 64;
-        const int s1 = min(max(e2 - e1, 0), 63), s2 = min(max(e1 - e2, 0), 63);
+        const FxAlign al(fx_prod_base(base.y, ea.x), fx_prod_base(ea.y, base.x));
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
-          const long long P2 = fx_mulhi(w[r].y, w[r].y) + fx_mulhi(w[r].x, w[r].x);
-          w[r].x = p[r].x >> s1;
-          w[r].y = P2 >> s2;
+          const fxc a = park[r * F::NT];
+          p[r] = al.sub(fx_mulhi(w[r].y, a.x), fx_mulhi(a.y, w[r].x));
         }
-        base = max(e1, e2);
+        ep = al.e;
+      } else if (t == 2) {
+        // P2 = BR^2 + BI^2 (derivatives.f90:996)
+        const FxAlign al(fx_prod_base(base.y, base.y), fx_prod_base(base.x, base.x));
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          w[r].y = al.add(fx_mulhi(w[r].y, w[r].y), fx_mulhi(w[r].x, w[r].x));
+          w[r].x = p[r];
+        }
+        base = make_int2(ep, al.e);
       } else {
         c.template split<3>(w, base, K, [&](int, int k, double2 P1, double2 P2) {
           const double qk = 0.25 * (double)(k * k);
