@@ -349,7 +349,8 @@ class Engine : public EngineBase {
       // the FP32 field is rounded from that copy on the device, so the input
       // crosses the host link once
       if (!psi64) QG_CK(cudaMalloc(&psi64, (size_t)g.n3 * g.plane * sizeof(double2)));
-      psi64_live = true;
+      psi64_live.resize(g.n3, 0);
+      std::fill_n(psi64_live.begin() + level0, nlev, 1);
       k_dense_to_compact<double><<<conv_grid(g.KY, nlev), 256, 0, st>>>(g, level0, src, psi64,
                                                                                         iflag);
       QG_LAUNCHED();
@@ -426,9 +427,20 @@ class Engine : public EngineBase {
       // fixed flow: q = 0 for all times (main_waqg.f90:141-146)
       QG_CK(cudaMemsetAsync(F[F_Q] + off, 0, (size_t)nz * lb, st));
     } else if (q_from_psi) {
+      // from the FP64 copy where the host set psi since the last
+      // initialisation or step; levels it did not set join it from the
+      // resident psi
+      const bool copy = !psi64_live.empty() && std::count(psi64_live.begin() + z0, psi64_live.begin() + z0 + nz, 1) > 0;
+      for (int a = z0, b; copy && a < z0 + nz; a = b) {
+        for (b = a + 1; b < z0 + nz && psi64_live[b] == psi64_live[a]; ++b) {}
+        if (psi64_live[a]) continue;
+        const long long m = (long long)(b - a) * g.plane;
+        k_widen_compact<T><<<grid_for(m), 256, 0, st>>>(m, F[F_PSI] + (size_t)a * g.plane, psi64 + (size_t)a * g.plane);
+        QG_LAUNCHED();
+      }
       const Divisor dz2(cfg.dz * cfg.dz);
       const dim3 gi((unsigned)((g.plane + 127) / 128), (g.nseg + kInitLev - 1) / kInitLev * (nz / g.nseg));
-      if (psi64_live) {
+      if (copy) {
         k_init_q<T, double><<<gi, 128, 0, st>>>(g, cfg.dz, dz2, cu, cl, psi64, F[F_Q], z0);
       } else {
         k_init_q<T, T><<<gi, 128, 0, st>>>(g, cfg.dz, dz2, cu, cl, F[F_PSI], F[F_Q], z0);
@@ -449,7 +461,7 @@ class Engine : public EngineBase {
 
   // the FP64 copy of psi that qg_set_state keeps for init_q (mixed path) is
   // used up; its memory stays for the handle's next run
-  void release_init_buffers() override { psi64_live = false; }
+  void release_init_buffers() override { std::fill(psi64_live.begin(), psi64_live.end(), 0); }
 
   // ---- the step -------------------------------------------------------------
   int step(int euler) override {
@@ -777,7 +789,7 @@ class Engine : public EngineBase {
   C* S = nullptr;              // [lanes][Zb][kNScr][n][KXP] scratch planes
   int s_levels = 0;            // levels of scratch allocated
   double2* psi64 = nullptr;    // FP64 copy of psi between qg_set_state and qg_init_state
-  bool psi64_live = false;
+  std::vector<unsigned char> psi64_live;   // levels whose psi was set since the last initialisation or step
   int Zb = 1;
   // phase-A batches run on `lanes` streams (lane 0: st), batch b on lane
   // b % lanes with its own scratch slot; they join st before the solves
@@ -1185,6 +1197,7 @@ class Engine : public EngineBase {
   // they do not hold the transforms of the current B (new handle,
   // qg_set_state of BR or BI, initialisation), are computed from B.
   int prepare() override {
+    release_init_buffers();     // the step replaces psi
     if (!Qp || q_valid) return QG_OK;
     for (int z0 = 0; z0 < g.n3; z0 += Zb) {
       const int zc = std::min(Zb, g.n3 - z0);
