@@ -220,10 +220,6 @@ class Engine : public EngineBase {
     sp.ybj = cfg.ybj_plus ? 1 : 0;
     sp.mpar = mpar;
     need_qw = (!cfg.fixed_flow && !cfg.no_feedback);
-    // kept y-inverse planes of B (YBJ+ runs whose update transforms B^{n+1} for q^w)
-    if (kReuseB && need_qw && cfg.ybj_plus) {
-      QG_CK(cudaMalloc(&Qp, (size_t)g.n3 * kNQ * g.n * g.KXP * sizeof(C)));
-    }
     int r0 = set_smem_attrs();
     if (r0) return r0;
     if (cfg.solve_columns != 0 && cfg.solve_columns != 16 && cfg.solve_columns != 32 && cfg.solve_columns != 64) {
@@ -248,6 +244,13 @@ class Engine : public EngineBase {
                                                                          cols_ret, nret);
         QG_LAUNCHED();
       }
+    }
+    // kept y-inverse planes of B (YBJ+ runs whose update transforms B^{n+1}
+    // for q^w); without them k_col_inv transforms B again in every step
+    if (kReuseB && need_qw && cfg.ybj_plus &&
+        cudaMalloc(&Qp, (size_t)g.n3 * kNQ * g.n * g.KXP * sizeof(C)) != cudaSuccess) {
+      Qp = nullptr;
+      (void)cudaGetLastError();
     }
     QG_CK(cudaStreamSynchronize(st));
     return QG_OK;
