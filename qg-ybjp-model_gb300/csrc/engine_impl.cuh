@@ -275,7 +275,7 @@ class Engine : public EngineBase {
     if (nl * nz > s_levels) {
       cudaFree(S);
       S = nullptr;
-      QG_CK(cudaMalloc(&S, (size_t)nl * nz * per_level));
+      QG_CK(dev_alloc(&S, (size_t)nl * nz * per_level));
       s_levels = nl * nz;
     }
     Zb = nz;
@@ -463,7 +463,8 @@ class Engine : public EngineBase {
   }
 
   // the FP64 copy of psi that qg_set_state keeps for init_q (mixed path) is
-  // used up; its memory stays for the handle's next run
+  // used up; its memory stays for the handle's next run, or for what needs it
+  // (dev_alloc)
   void release_init_buffers() override { std::fill(psi64_live.begin(), psi64_live.end(), 0); }
 
   // ---- the step -------------------------------------------------------------
@@ -524,8 +525,8 @@ class Engine : public EngineBase {
       QG_CK(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
       QG_CK(cudaStreamCreateWithPriority(&std_, cudaStreamNonBlocking, prio_low));
       QG_CK(cudaEventCreateWithFlags(&ev_state, cudaEventDisableTiming));
-      QG_CK(cudaMalloc(&diag_part_a, diag_part_n * kNDiag * sizeof(double)));
-      QG_CK(cudaMalloc(&diag_out_a, kNDiag * sizeof(double)));
+      QG_CK(dev_alloc(&diag_part_a, diag_part_n * kNDiag * sizeof(double)));
+      QG_CK(dev_alloc(&diag_out_a, kNDiag * sizeof(double)));
       QG_CK(cudaMallocHost(&diag_host_a, kNDiag * sizeof(double)));
     }
     if (diag_pending) { err = "the previous asynchronous diagnostics were not collected"; return QG_ERR_ARG; }
@@ -605,12 +606,12 @@ class Engine : public EngineBase {
     if (m < 1 || om_nd == 0) return QG_OK;
     if (!om_fac) {
       double4* f = nullptr;
-      QG_CK(cudaMalloc(&f, (size_t)om_nd * m * sizeof(double4)));
+      QG_CK(dev_alloc(&f, (size_t)om_nd * m * sizeof(double4)));
       k_omega_fac<<<(om_nd + 127) / 128, 128, 0, st>>>(om_nd, g.n3, cfg.dz, om_kh2, om_t1, om_du, om_dl, om_a, f);
       om_fac = f;
       QG_LAUNCHED();
     }
-    if (!om_scr) QG_CK(cudaMalloc(&om_scr, (size_t)2 * m * nret * sizeof(double)));
+    if (!om_scr) QG_CK(dev_alloc(&om_scr, (size_t)2 * m * nret * sizeof(double)));
     k_omega_solve<<<dim3((unsigned)((nret + 63) / 64), 2), 64, 0, st>>>(g, cfg.dz, om_du, om_fac, tab_idx, cols_ret, nret,
                                                                        rhs, om_scr, w);
     QG_LAUNCHED();
@@ -868,10 +869,21 @@ class Engine : public EngineBase {
     }
   }
 
+  // cudaMalloc of what a handle allocates after qg_create: gives the FP64 copy
+  // of psi back, if it holds nothing, before it fails
+  template <typename P> cudaError_t dev_alloc(P** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation || !psi64 || std::count(psi64_live.begin(), psi64_live.end(), 1)) return e;
+    (void)cudaGetLastError();
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess || (e = cudaFree(psi64)) != cudaSuccess) return e;
+    psi64 = nullptr;
+    return cudaMalloc(p, bytes);
+  }
+
   int ensure(void** p, size_t* have, size_t need) {
     if (*have >= need) return QG_OK;
     if (*p) { QG_CK(cudaStreamSynchronize(st)); cudaFree(*p); *p = nullptr; *have = 0; }
-    QG_CK(cudaMalloc(p, need));
+    QG_CK(dev_alloc(p, need));
     *have = need;
     return QG_OK;
   }
@@ -1241,7 +1253,7 @@ class Engine : public EngineBase {
     if (need <= w_planes) return QG_OK;
     QG_CK(cudaStreamSynchronize(st));
     if (W) { cudaFree(W); W = nullptr; w_planes = 0; }
-    QG_CK(cudaMalloc(&W, need * g.n * iktxP() * sizeof(C)));
+    QG_CK(dev_alloc(&W, need * g.n * iktxP() * sizeof(C)));
     w_planes = need;
     return QG_OK;
   }
@@ -1347,7 +1359,7 @@ class Engine : public EngineBase {
 
   int ensure_tmp() {
     const size_t fbytes = (size_t)g.n3 * g.plane * sizeof(C);
-    for (auto& p : tmpF) if (!p) { QG_CK(cudaMalloc(&p, fbytes)); QG_CK(cudaMemsetAsync(p, 0, fbytes, st)); }
+    for (auto& p : tmpF) if (!p) { QG_CK(dev_alloc(&p, fbytes)); QG_CK(cudaMemsetAsync(p, 0, fbytes, st)); }
     return QG_OK;
   }
 

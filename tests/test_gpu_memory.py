@@ -1,9 +1,12 @@
-"""Device memory that a handle can do without: it is created and runs where that part does not fit, with the same results."""
+"""Device memory that a handle can do without: it is created and runs where that part does not fit, with the same results, and gives
+back what it keeps unused before a later call fails."""
 from __future__ import annotations
 
+import numpy as np
 import pytest
 
 from qgybj import Simulation
+from qgybj._lib import check, lib, ptr
 from qgybj.config import CONFIGS, dealias_mask, make_initial_condition, model_parameters, scaled
 from tests.helpers import rel_l2
 
@@ -68,3 +71,28 @@ def test_a_handle_without_the_memory_it_can_do_without(precision, size, tol):
     with sim:
         got = run(sim)
     assert all(rel_l2(a, b) <= tol for a, b in zip(got, want))
+
+
+def test_the_unused_copy_of_psi_makes_room():
+    import torch
+    n, n3 = 512, 64
+    rc = scaled(CONFIGS["c1"], n, n3)
+    ic = make_initial_condition(rc)
+    params = model_parameters(rc, ic.delt)
+    out = torch.empty((n3, n, n), dtype=torch.float32, device="cuda")
+    psi = torch.from_numpy(ic.psi).cuda()
+    torch.cuda.synchronize()
+    with Simulation(params, "mixed") as sim:
+        def dump():
+            check(lib().qg_dump_psi(sim.h, ptr(out), 0, n3, 1.0, 1.0), sim.h)
+            return out.cpu().numpy()
+        sim.set_state("psi", psi)
+        sim.init_state(True, True)
+        planes = 6 * n3 * n * ((n // 2 + 1 + 7) // 8 * 8) * 8        # of the transforms, 415 MB
+        copy = n3 * 341 * 176 * 16                                    # of the FP64 psi, 61 MB
+        with _Leave(planes - copy // 2):
+            a = dump()
+        # and it comes back with the next psi
+        sim.set_state("psi", psi)
+        sim.init_state(True, True)
+        assert np.array_equal(a, dump())
