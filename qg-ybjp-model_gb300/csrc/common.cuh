@@ -61,7 +61,8 @@ struct StepParams {
   int disp;           // 0 when no_dispersion == 1 or passive_scalar == 1
   int use_dq;         // inviscid == 0 && nuz != 0
   int euler;          // forward Euler first step
-  int ybj;            // 1: YBJ+ (A from A_solver_ybj_plus); 0: regular YBJ (A from the vertical integral of B)
+  int ybj;            // 0: regular YBJ, whose A (from the vertical integral of B) takes sigma terms; 1: no such terms
+                      // (YBJ+, or passive_scalar == 1, where A is not computed)
   // a stack of ensemble members (Geom::nseg levels each): per member
   // {delt, 0.5/(Bu Ro), Ro, W2F} at mpar[4 m .. 4 m + 3], and the integrating
   // factor tables of member m at + m * plane; nullptr for one run

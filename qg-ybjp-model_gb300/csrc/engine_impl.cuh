@@ -217,7 +217,7 @@ class Engine : public EngineBase {
     sp.disp = (cfg.no_dispersion || cfg.passive_scalar) ? 0 : 1;
     sp.use_dq = (cfg.inviscid == 0 && cfg.nuz != 0.0) ? 1 : 0;
     sp.euler = 0;
-    sp.ybj = cfg.ybj_plus ? 1 : 0;
+    sp.ybj = cfg.ybj_plus || cfg.passive_scalar ? 1 : 0;
     sp.mpar = mpar;
     need_qw = (!cfg.fixed_flow && !cfg.no_feedback);
     int r0 = set_smem_attrs();
