@@ -396,8 +396,10 @@ class Engine : public EngineBase {
 
   // Device address through which kernels may access p: device memory as is,
   // page-locked host memory through its mapping; nullptr for anything else
-  // (pageable or managed memory is staged through a copy instead).
+  // (pageable or managed memory, an address that is not 16-byte aligned),
+  // which is staged through a copy instead.
   static const void* device_view(const void* p) {
+    if (reinterpret_cast<uintptr_t>(p) & 15) return nullptr;
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
     if (at.type == cudaMemoryTypeDevice) return p;
