@@ -246,10 +246,8 @@ class AdjEngine final : public Engine<double> {
     const long long tot = (long long)g.n3 * g.plane;
     const C* qs = F[F_Q];
     if (need_qw) {
-      k_compact_to_dense<double><<<conv_grid(g.n, g.n3), 256, 0, st>>>(g, 0, F[F_BR], Sb[0], 0, Divisor(cfg.dz));
-      QG_LAUNCHED();
-      k_compact_to_dense<double><<<conv_grid(g.n, g.n3), 256, 0, st>>>(g, 0, F[F_BI], Sb[1], 0, Divisor(cfg.dz));
-      QG_LAUNCHED();
+      if ((rc = to_dense(F[F_BR], Sb[0], 0, 0, g.n3))) return rc;
+      if ((rc = to_dense(F[F_BI], Sb[1], 0, 0, g.n3))) return rc;
       if ((rc = compute_qw(reinterpret_cast<const double*>(Sb[0]), reinterpret_cast<const double*>(Sb[1]),
                            reinterpret_cast<double*>(Sb[2]), g.n3)))
         return rc;
@@ -290,8 +288,7 @@ class AdjEngine final : public Engine<double> {
     QG_LAUNCHED();
     int rc = solve_generic(nullptr, tmpC[0], nullptr, nullptr, tmpC[1], nullptr, 0, 2, nullptr, 0, -1, true);
     if (rc) return rc;
-    k_compact_to_dense<double><<<conv_grid(g.n, g.n3), 256, 0, st>>>(g, 0, tmpC[1], out, 0, Divisor(cfg.dz));
-    QG_LAUNCHED();
+    if ((rc = to_dense(tmpC[1], out, 0, 0, g.n3))) return rc;
     return QG_OK;
   }
 
@@ -308,8 +305,7 @@ class AdjEngine final : public Engine<double> {
     const double k4 = 0.25 / cfg.Bu;
     const int src[4] = {F_BR, F_BI, F_AR, F_AI};
     for (int i = 0; i < 4; ++i) {
-      k_compact_to_dense<double><<<conv_grid(g.n, g.n3), 256, 0, st>>>(g, 0, F[src[i]], Sb[i], 0, Divisor(cfg.dz));
-      QG_LAUNCHED();
+      if ((rc = to_dense(F[src[i]], Sb[i], 0, 0, g.n3))) return rc;
     }
     // Sb[4], Sb[5]: LA of the real and imaginary parts
     if ((rc = lin(Sb[4], 0, {term(Sb[0], 1, 0, 0), term(Sb[2], k4, 0, 3)})) ||

@@ -386,9 +386,7 @@ class Engine : public EngineBase {
       int rc = ensure(&stage, &stage_bytes, bytes);
       if (rc) return rc;
     }
-    k_compact_to_dense<T><<<conv_grid(g.n, nlev), 256, 0, st>>>(g, level0, F[f], dst ? dst : (double2*)stage, mode,
-                                                                Divisor(cfg.dz));
-    QG_LAUNCHED();
+    if (int rc = to_dense(F[f], dst ? dst : (double2*)stage, mode, level0, nlev)) return rc;
     if (!dst) QG_CK(cudaMemcpyAsync(kvar, stage, bytes, cudaMemcpyDefault, st));
     QG_CK(cudaStreamSynchronize(st));
     return QG_OK;
@@ -859,6 +857,15 @@ class Engine : public EngineBase {
   }
 
   static dim3 conv_grid(int rows, int nlev) { return dim3((rows + kConvRows - 1) / kConvRows, nlev); }
+  // levels [level0, level0 + nlev) of a resident field (mode 1: their vertical
+  // differences) in the reference's layout
+  int to_dense(const C* f, double2* dense, int mode, int level0, int nlev) {
+    const int iktx = g.n / 2 + 1;
+    k_compact_to_dense<T><<<dim3((g.n * iktx + kDenseRun - 1) / kDenseRun, nlev), 256, 0, st>>>(
+        g, level0, f, dense, mode, Divisor(cfg.dz), (unsigned)((0x100000000ull + iktx - 1) / iktx));
+    QG_LAUNCHED();
+    return QG_OK;
+  }
 
   int map_field(int field) const {
     switch (field) {
@@ -1377,8 +1384,7 @@ class Engine : public EngineBase {
     const size_t bytes = dense_bytes(g.n3);
     void* v;
     if (int rc = out_view(kvar, bytes, 0, &v)) return rc;
-    k_compact_to_dense<T><<<conv_grid(g.n, g.n3), 256, 0, st>>>(g, 0, src, (double2*)v, mode, Divisor(cfg.dz));
-    QG_LAUNCHED();
+    if (int rc = to_dense(src, (double2*)v, mode, 0, g.n3)) return rc;
     return out_copy(kvar, v, bytes);
   }
 };
