@@ -101,6 +101,7 @@ class AdjEngine final : public Engine<double> {
       QG_LAUNCHED();
       if ((rc = download_compact(lamB[0], outs[k], 0))) return rc;
     }
+    QG_CK(cudaStreamSynchronize(st));
     return QG_OK;
   }
 
