@@ -81,7 +81,8 @@ typedef struct qg_config {
   const double* r_2ut;     /* [n3] N^2 at za(iz), or NULL (= Bu/a_ell_ut); diagnostics */
   int levels_per_batch;    /* z levels per phase-A batch; 0 = choose automatically     */
   int use_graphs;          /* 1 = replay the step as a CUDA graph (default), 0 = launch */
-  int solve_columns;       /* columns per CTA of the column solves: 16, 32 or 64; 0 = 32 */
+  int solve_columns;       /* columns per CTA of the column solves: 16, 32 or 64; 0 = 32 *
+                            * (solves of few columns always take a warp per recurrence)  */
 } qg_config;
 
 typedef struct qg_handle qg_handle;

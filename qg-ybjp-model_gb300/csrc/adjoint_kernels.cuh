@@ -192,7 +192,7 @@ __device__ __forceinline__ void adj_col_inverse(const FxColCtx<N>& c, const Geom
 // as the step's (step_fx.cuh); the column kernels' independent fields are
 // spread over gridDim.z CTAs where a grid would leave SMs idle
 template <int N>
-__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(QG_FX_COL_CTAS))
+__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(kFxColCtas))
 k_adj_col_inv(Geom g, AdjP p, int zbase, AdjIn L, const double* __restrict__ e1t, const double* __restrict__ e2t,
               const double* __restrict__ e1wt, const double* __restrict__ e2wt, double2* __restrict__ SA,
               const double2* __restrict__ twg) {
@@ -336,7 +336,7 @@ __device__ __forceinline__ void adj_col_plane(const FxColCtx<N>& c, const Geom& 
 }
 
 template <int N>
-__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(QG_FX_COL_CTAS))
+__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(kFxColCtas))
 k_adj_col_fwd(Geom g, AdjP p, int zbase, AdjIn L, AdjOut O, const double* __restrict__ e1t,
               const double* __restrict__ e2t, const double* __restrict__ e1wt, const double* __restrict__ e2wt,
               const double2* __restrict__ SA, const double2* __restrict__ twg) {
@@ -381,7 +381,7 @@ k_adj_col_fwd(Geom g, AdjP p, int zbase, AdjIn L, AdjOut O, const double* __rest
 // y-inverse FFTs for the q^w transpose: BR, i ky BR, BI, i ky BI, w', ky^2 w'
 // with w' = w/(2N^2) ((0,0): Re w/N^2), into SF
 template <int N>
-__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(QG_FX_COL_CTAS))
+__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(kFxColCtas))
 k_adj_qw_col_inv(Geom g, int zbase, const double2* __restrict__ BR, const double2* __restrict__ BI,
                  const double2* __restrict__ w, double2* __restrict__ SF, const double2* __restrict__ twg) {
   using F = FxCol<N>;
@@ -407,7 +407,7 @@ k_adj_qw_col_inv(Geom g, int zbase, const double2* __restrict__ BR, const double
 // q^w = s R(P1) - s kh^2/4 R(P2); writes (G_R, H_R, G_I, H_I) with
 // lB = w_k [F_y(G) - i ky F_y(H)], G = -i kx F_x(a) + F_x(c), H = F_x(b)
 template <int N>
-__global__ void __launch_bounds__(FxRow<N>::NT, fx_row_ctas<N>(QG_FX_ROW_CTAS))
+__global__ void __launch_bounds__(FxRow<N>::NT, fx_row_ctas<N>(kFxRowCtas))
 k_adj_qw_row(Geom g, AdjP p, double2* __restrict__ SF, const double2* __restrict__ twg) {
   using F = FxRow<N>;
   constexpr int NB = F::NB;
@@ -465,7 +465,7 @@ k_adj_qw_row(Geom g, AdjP p, double2* __restrict__ SF, const double2* __restrict
 
 // final adds: lq += w, lB += A_solver(lA) (+ q^w transpose when with_qw)
 template <int N>
-__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(QG_FX_COL_CTAS))
+__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(kFxColCtas))
 k_adj_qw_col_fwd(Geom g, int zbase, double2* __restrict__ lBR, double2* __restrict__ lBI, const double2* __restrict__ SF,
                  const double2* __restrict__ twg) {
   using F = FxCol<N>;

@@ -370,7 +370,7 @@ __device__ __forceinline__ void row_last_fwd512(const cplx<T>* __restrict__ tr, 
   else { b[0] = t[0]; b[1] = t[1]; b[2] = t[2]; }
 }
 
-// the half spectra at k from a = F[k], b = F[N-k] (unpack_spec's arithmetic)
+// the half spectra at k from a = F[k], b = F[N-k] (unpack_pad's arithmetic)
 template <typename T>
 __device__ __forceinline__ void split_pair(cplx<T> a, cplx<T> b, cplx<T>& X, cplx<T>& Y) {
   X = mk<T>((a.x + b.x) * (T)0.5, (a.y - b.y) * (T)0.5);

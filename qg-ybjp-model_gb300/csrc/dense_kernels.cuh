@@ -10,12 +10,8 @@ namespace qg {
 
 // dense spectral: double2 [nz][n][iktx]; W: cplx<T> [nz][n(y)][iktxP]; phys: T [nz][n][n]
 
-#ifndef QG_DENSE_COL_CTAS
-#define QG_DENSE_COL_CTAS 6
-#endif
-#ifndef QG_DENSE_ROW_CTAS
-#define QG_DENSE_ROW_CTAS 4
-#endif
+// CTAs per SM (of 128 threads) that the fixed-point kernels' register budgets target
+constexpr int kDenseColCtas = 6, kDenseRowCtas = 4;
 
 // small integers (|k| < 2^24) as doubles, off the FP64 pipe
 __device__ __forceinline__ double int_to64(int k) { return f32_to_f64((float)k); }
@@ -29,9 +25,8 @@ template <typename T, int N> struct Dense {
   static constexpr int NB = FX ? N / 8 : N / radix_of(N);
   static constexpr int RT = FX ? imin(FxRow<N>::RT, N / 2) : imin(N / 2, imax(1, 256 / NB));
   static constexpr int RNT = FX ? FxRow<N>::NT : RT * NB;
-  // CTAs per SM that the fixed-point kernels' register budgets target
-  static constexpr int CMINB = FX ? imin(32, (QG_DENSE_COL_CTAS * 128) / CNT) : 1;
-  static constexpr int RMINB = FX ? imin(32, imax(1, (QG_DENSE_ROW_CTAS * 128) / RNT)) : 1;
+  static constexpr int CMINB = FX ? imin(32, (kDenseColCtas * 128) / CNT) : 1;
+  static constexpr int RMINB = FX ? imin(32, imax(1, (kDenseRowCtas * 128) / RNT)) : 1;
   static constexpr int LD = FX ? FxRow<N>::LD : PadLD<N>::value;
   static constexpr size_t sm_col(int nf = 1) { return FX ? FxCol<N>::smem() : (size_t)(N + nf * ColLay<N, CT>::FS) * sizeof(cplx<T>); }
   static constexpr size_t sm_row() { return FX ? FxRow<N>::smem() : (size_t)(N + RT * LD) * sizeof(cplx<T>); }

@@ -364,7 +364,7 @@ class AdjEngine final : public Engine<double> {
         using FC = FxCol<NN>;
         using FR = FxRow<NN>;
         const dim3 gc((g.K + FC::CT) / FC::CT, zc), gr(g.n / FR::RT, zc);
-        const bool few = few_ctas((long long)gc.x * gc.y, 1, fx_col_ctas<NN>(QG_FX_COL_CTAS));
+        const bool few = few_ctas((long long)gc.x * gc.y, 1, fx_col_ctas<NN>(kFxColCtas));
         auto over = [&](unsigned k) { return dim3(gc.x, gc.y, few ? k : 1); };
         launch_col_inv<NN>(z0, zc, psi, q, BR, BI, S, nullptr, 0, st);
         QG_LAUNCHED();
@@ -388,7 +388,7 @@ class AdjEngine final : public Engine<double> {
         using FC = FxCol<NN>;
         using FR = FxRow<NN>;
         const dim3 gc((g.K + FC::CT) / FC::CT, zc), gr(g.n / FR::RT, zc);
-        const bool few = few_ctas((long long)gc.x * gc.y, 1, fx_col_ctas<NN>(QG_FX_COL_CTAS));
+        const bool few = few_ctas((long long)gc.x * gc.y, 1, fx_col_ctas<NN>(kFxColCtas));
         auto over = [&](unsigned k) { return dim3(gc.x, gc.y, few ? k : 1); };
         k_adj_qw_col_inv<NN><<<over(6), FC::NT, FC::smem(), st>>>(g, z0, BR, BI, Af[A_W], S, tw);
         QG_LAUNCHED();

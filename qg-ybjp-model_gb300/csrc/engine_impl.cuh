@@ -1019,9 +1019,9 @@ class Engine : public EngineBase {
   // (a shorter chain per CTA and more of the GPU at work) instead of looping
   // over them (one table load per tile).  us per launch, looped -> spread:
   // 64^2 x 64 22.5 -> 14.0, 128^2 x 64 36.7 -> 29.0, 256^2 x 128 (2.6 waves)
-  // 144 -> 147.  (The FP32 kernels are not spread: k_col_update 64^2 x 32 17.9
-  // -> 13.8, but the compiler then fuses other products with additions and the
-  // fields differ in their last bits from those of larger grids.)
+  // 144 -> 147.  (The FP32 kernels are not spread: the compiler then fuses
+  // other products with additions, and the fields differ in their last bits
+  // from those of larger grids.)
   bool few_ctas(long long n, int waves, int per_sm) const { return n <= (long long)waves * per_sm * nsm; }
 
   // k_col_inv on levels [z0, z0 + zc): mode 0 all six fields into Sb, 1 the
@@ -1033,7 +1033,7 @@ class Engine : public EngineBase {
     const int tiles = (g.K + col_ct<NN>()) / col_ct<NN>();
     if constexpr (kFx) {
       const int f0 = mode == 2 ? 4 : 0, f1 = mode == 1 ? 4 : 6;
-      const int split = few_ctas((long long)tiles * zc, 1, fx_col_ctas<NN>(QG_FX_COL_CTAS)) ? f1 - f0 : 1;
+      const int split = few_ctas((long long)tiles * zc, 1, fx_col_ctas<NN>(kFxColCtas)) ? f1 - f0 : 1;
       k_fx_col_inv<NN><<<dim3(tiles * split, zc), FxCol<NN>::NT, FxCol<NN>::smem(), on>>>(g, z0, psi, q, br, bi, Sb, tw,
                                                                                           Qb, f0, f1, split);
       return;
@@ -1189,7 +1189,11 @@ class Engine : public EngineBase {
       const int nrec = (do_psi ? 2 : 0) + (do_A == 1 ? 4 : do_A);   // recurrences per column
       // A launch of few columns spreads their recurrences over CTAs of one
       // warp, so that more SMs' FP64 pipes (2 lanes per clock) work on them,
-      // and reads longer segments ahead
+      // and reads longer segments ahead (whatever solve_tc is).  us per solve,
+      // otherwise -> so, by warps per SM: 0.9 (FP64 64^2 x 64) 42.9 -> 34.7, 3.6
+      // (128^2 x 64) 45.0 -> 38.8, 4.6 (psi_solver 256^2 x 128) 123 -> 118, 13.9
+      // (256^2 x 128) 147 -> 189; mixed 64^2 x 32 18.3 -> 16.3, 256^2 x 128 80 ->
+      // 139
       const bool few = few_ctas((long long)((ncl + 31) / 32) * nsegs * nrec, 1, 12);
       const int zs = few ? nrec : 1;
 #define QG_SOLVE_ST(TCV, PCV, SV)                                                                            \

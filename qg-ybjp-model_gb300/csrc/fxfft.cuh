@@ -7,20 +7,26 @@
 // 290 integer ones (about 160 clocks), so the FP64 path transforms integers:
 //
 //   * Each transform finds the largest exponent among its inputs (|x| < 2^E)
-//     and scales every input to an integer m = x 2^(59-E) (values below
-//     2^(E-59) lose bits there, where a double keeps them; against the
-//     transform's largest input that is 64 times finer than FP64's own
-//     rounding).
+//     and scales every input to an integer m = x 2^(59-E), truncated towards
+//     zero (values below 2^(E-6) lose bits there, where a double keeps them;
+//     against the transform's largest input that is 64 times finer than FP64's
+//     own rounding).  Two real rows packed as one complex input have an
+//     exponent each (FxRowCtx).
 //   * A radix-R pass lets the modulus grow by at most R, so the integers stay
 //     below 2^62.5 when every later pass divides its inputs by the earlier
 //     pass's radix.  The division is part of the twiddle factor, w = W 2^(64-s)
 //     and x w taken as the high word of the product; the untwiddled input is
-//     shifted.  All roundings are to nearest at 2^-62 of the growth bound.
+//     shifted.  The passes round to nearest, or to one unit where a product's
+//     low x low part is left out, at 2^-62 of the growth bound.
 //   * The outputs are normalised back to doubles, rounded to nearest.
-// The rounding noise relative to the output's rms is at most about 2^-55.5
-// even for an input with a single nonzero value per transform (the worst
-// ratio of bound to rms), where an FP64 transform of the same length is at
-// 2^-53; measured errors against 113-bit transforms are in the tests.
+// The noise relative to the output's rms is largest for an input with a single
+// nonzero value, which the divisions leave at 2^59 / 8^2 = 2^53 after the
+// passes of n = 512: eight inputs of the last butterfly rounded at half a unit,
+// sqrt(8/12) 2^-53 = 2^-53.3 and the earlier passes' beside it, measured
+// 2^-52.7 (2^-53.9 at n = 256, 2^-55.8 at 64; white spectra 2^-57), where an
+// FP64 transform is at 2^-52.1.  Longer transforms, and the inverse rows, take
+// back the unused room (fx_renorm, FIT): 2^-54.3 there for such an input, up to
+// 2^-52.6 for k^-4 spectra.  The tests compare with 113-bit transforms.
 // A transform with a NaN or infinity among its inputs returns NaN; tiny and
 // huge scales (subnormal inputs, overflowing outputs) take exact slow paths.
 //
@@ -36,15 +42,6 @@ struct __align__(16) fxc { long long x, y; };
 // radix of the pass with stride ns of a length-n transform: radix 8 first
 // (eight values per thread throughout), then as radix_of
 __host__ __device__ constexpr int fx_radix(int n, int ns) { return ns == 1 ? 8 : (n < 64 ? n / 8 : radix_of(n / ns)); }
-// stride of the last pass
-template <int N> struct FxLast {
-  static constexpr int calc() {
-    int ns = 1;
-    while (ns * fx_radix(N, ns) < N) ns *= fx_radix(N, ns);
-    return ns;
-  }
-  static constexpr int value = calc();
-};
 // offset of the pass ns in the per-pass twiddle table
 template <int N> __host__ __device__ constexpr int fx_tw_off(int ns) {
   int off = 0;
@@ -68,15 +65,10 @@ template <int N> __host__ __device__ constexpr int fx_shift_total() {
 
 __host__ __device__ constexpr int fx_ilog2(int n) { int m = 0; while ((1 << m) < n) ++m; return m; }
 // transforms this long take back the room that a peaked spectrum leaves
-// unused below the growth bound, before each later pass
+// unused below the growth bound, before each later pass: without it the
+// divisions of n = 1024 would leave a single value's output at 2^51, above
+// FP64's noise
 template <int N> __host__ __device__ constexpr bool fx_renorm() { return N >= 1024; }
-
-// radix of the pass before the one with stride ns > 1
-template <int N> __host__ __device__ constexpr int fx_prev_radix(int ns) {
-  int s = 1, r = 1;
-  while (s < ns) { r = fx_radix(N, s); s *= r; }
-  return r;
-}
 
 // (x + i y) * w with w = (c.hi, c.lo, s.hi, s.lo), c = c.hi 2^32 + c.lo with a
 // signed low word: the high 64 bits of the products, without low x low.  The

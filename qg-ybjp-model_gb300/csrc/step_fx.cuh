@@ -15,10 +15,9 @@
 
 namespace qg {
 
-// CTAs per SM (of 128 threads) that the register budgets target
-#ifndef QG_FX_ROW_CTAS
-#define QG_FX_ROW_CTAS 4
-#endif
+// CTAs per SM (of 128 threads) that the register budgets of the row and column
+// kernels target
+constexpr int kFxRowCtas = 4, kFxColCtas = 7;
 template <int N, int T = 128> __host__ __device__ constexpr int fx_row_ctas(int want) {
   return imin(32, imax(1, (want * 128) / FxRow<N, T>::NT));
 }
@@ -35,7 +34,7 @@ template <int N> struct FxMain {
   static constexpr size_t smem() { return (size_t)(fx_tw_count<N>() + F::RT * F::LD + 2 * F::RT * N) * sizeof(double2); }
 };
 template <int N>
-__global__ void __launch_bounds__(FxMain<N>::F::NT, fx_row_ctas<N, kFxMainT>(QG_FX_ROW_CTAS))
+__global__ void __launch_bounds__(FxMain<N>::F::NT, fx_row_ctas<N, kFxMainT>(kFxRowCtas))
 k_fx_row_main(Geom g, StepParams sp, double2* __restrict__ S, const double2* __restrict__ twg, int nitems,
               const double2* __restrict__ Qb) {
   using F = typename FxMain<N>::F;
@@ -126,9 +125,10 @@ template <int N> struct FxQw {
   using F = FxRow<N>;
   static constexpr size_t smem() { return F::smem() + (size_t)F::RT * N * sizeof(fxc); }
 };
-// CTAs per SM that its register budget targets: three leave it 168 registers
-// (us per launch, four -> three: 64^2 x 64 20.4 -> 18.3, 128^2 x 64 59 -> 53,
-// 256^2 x 128 the same); at N = 512, two warps per row, the fourth CTA paid
+// CTAs per SM that its register budget targets: three leave it 168 registers.
+// us per launch, four -> three: 64^2 x 64 20.4 -> 18.3, 128^2 x 64 59 -> 53,
+// 256^2 x 16 61 -> 55 (x 128 426 -> 432), 16^2 and 32^2 the same; 512^2 x 128
+// 1730 -> 1750, 1024^2 x 16 1028 -> 1020 (two and four warps per row)
 template <int N> __host__ __device__ constexpr int fx_qw_ctas() { return fx_row_ctas<N>(N >= 512 ? 4 : 3); }
 template <int N>
 __global__ void __launch_bounds__(FxRow<N>::NT, fx_qw_ctas<N>())
@@ -208,16 +208,13 @@ k_fx_row_qw(Geom g, double2* __restrict__ S, const double2* __restrict__ twg, in
 // ===========================================================================
 // Columns
 // ===========================================================================
-#ifndef QG_FX_COL_CTAS
-#define QG_FX_COL_CTAS 7
-#endif
 template <int N> __host__ __device__ constexpr int fx_col_ctas(int want) { return imin(32, (want * 128) / FxCol<N>::NT); }
 
 // y-inverse transforms of the fields f in [f0, f1) of (u, v, zeta, q, BR, BI)
 // into the planes f of S; BR, BI into the kept planes Qb when given; a tile's
 // fields over `split` CTAs
 template <int N>
-__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(QG_FX_COL_CTAS))
+__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(kFxColCtas))
 k_fx_col_inv(Geom g, int zbase, const double2* __restrict__ psi, const double2* __restrict__ q,
              const double2* __restrict__ BR, const double2* __restrict__ BI, double2* __restrict__ S,
              const double2* __restrict__ twg, double2* __restrict__ Qb, int f0, int f1, int split) {
@@ -282,7 +279,7 @@ __device__ __forceinline__ void fx_col_plane(const FxColCtx<N>& c, const Geom& g
 // y-forward transforms, time update, y-inverse transforms of B^{n+1} and
 // i ky B^{n+1} (k_col_update)
 template <int N>
-__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(QG_FX_COL_CTAS))
+__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(kFxColCtas))
 k_fx_col_update(Geom g, StepParams sp, int zbase, StateP<double> st, const double* __restrict__ e1t,
                 const double* __restrict__ e2t, const double* __restrict__ e1wt, const double* __restrict__ e2wt,
                 double2* __restrict__ S, const double2* __restrict__ twg, int qw_prep, double2* __restrict__ Qb) {
@@ -405,7 +402,7 @@ k_fx_col_update(Geom g, StepParams sp, int zbase, StateP<double> st, const doubl
 
 // y-forward transforms of the q^w planes, q* = q - q^w (k_col_qw)
 template <int N>
-__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(QG_FX_COL_CTAS))
+__global__ void __launch_bounds__(FxCol<N>::NT, fx_col_ctas<N>(kFxColCtas))
 k_fx_col_qw(Geom g, StepParams sp, int zbase, const double2* __restrict__ q, double2* __restrict__ qstar,
             const double2* __restrict__ S, const double2* __restrict__ twg, int* __restrict__ nflag) {
   using F = FxCol<N>;

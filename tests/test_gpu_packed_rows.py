@@ -13,6 +13,7 @@ from oracle import qgybj_oracle as orc
 from qgybj import Simulation
 from qgybj.config import CONFIGS, dealias_mask, scaled
 from tests.helpers import oracle_for, random_masked, rel_l2
+from tests.test_gpu_fixed_point import _realit, _spectrum
 
 pytestmark = pytest.mark.gpu
 TOL = 2.0 ** -51.8
@@ -102,3 +103,20 @@ def test_step_with_a_uniform_wave_and_a_small_imaginary_part(n, n3):
     exp = model.step_euler(st).BR.copy()
     got[:, 0, 0] = exp[:, 0, 0] = 0.0
     assert rel_l2(got, exp) <= 1e-12
+
+
+@pytest.mark.parametrize("kind", ["one", "gauss", "tiny", "huge"])
+@pytest.mark.parametrize("n", [512, 1024])
+def test_peaked_and_scaled_spectra_at_long_lengths(n, kind):
+    """A few modes, columns down to subnormal values, and the ends of the exponents' range, against 64-bit-mantissa transforms (or
+    longer) at the lengths whose divisions leave the fewest bits."""
+    k = _spectrum(kind, n)
+    with np.errstate(over="ignore", under="ignore"), _sim(n) as sim:
+        ex = sfft.irfft2(_realit(k, n).astype(np.clongdouble), s=(n, n), norm="forward")
+        floor = float(n * np.longdouble(5e-324) / np.linalg.norm((ex / np.abs(ex).max()).astype(float)) / np.abs(ex).max())
+        assert _err(sim.fft_c2r(k)[..., :n], ex) <= TOL + (floor if kind == "tiny" else 0)
+        r = np.zeros((1, n, n + 2))
+        r[..., :n] = ex.astype(float)
+        fx = sfft.rfft2(r[..., :n].astype(np.longdouble), norm="forward")
+        floor = float(n * np.longdouble(5e-324) / np.linalg.norm((fx / np.abs(fx).max()).astype(complex)) / np.abs(fx).max())
+        assert _err(sim.fft_r2c(r), fx) <= TOL + (floor if kind == "tiny" else 0)
