@@ -196,9 +196,9 @@ template <int NB, bool OR> __device__ __forceinline__ uint2 fx_row_reduce(uint2 
 // Two real rows are packed as one complex row, and each has a scale of its own
 // (a base per part), as two transforms would.  With one scale for both, a row
 // 2^-m of its neighbour lost m of its bits, beside a uniform neighbour too,
-// which a floating-point transform does not mix into it.  Scales of their own
-// cost 6 % of k_fx_row_main and 7-13 % of k_fx_row_qw (512^2 x 256: 6400 ->
-// 6840 and 3260 -> 3480 us).
+// which a floating-point transform does not mix into it.  us per launch, one
+// scale -> two: k_fx_row_main 512^2 x 256 6400 -> 6480, 256^2 x 128 725 -> 753,
+// 128^2 x 64 98 -> 98; k_fx_row_qw 3260 -> 3470, 381 -> 428, 51 -> 53.
 template <int N, int T = 128> struct FxRowCtx {
   static constexpr int NB = N / 8;
   fxc* buf;
