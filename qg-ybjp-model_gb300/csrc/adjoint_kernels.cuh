@@ -435,8 +435,10 @@ k_adj_qw_row(Geom g, AdjP p, double2* __restrict__ SF, const double2* __restrict
   c.inverse(X, Y, b, eb);
 #pragma unroll
   for (int r = 0; r < 8; ++r) { v[r].x = -fx_mulhi(l[r].y, b[r].x); v[r].y = fx_mulhi(l[r].y, b[r].y); }
-  // (they wait in the planes of w, read above)
-  c.forward(v, bases(el.y, eb.x, eb.y), K, [&](int, int k, double2 R, double2 I) { sf(4)[k] = R; sf(5)[k] = I; });
+  double2 aR[3], aI[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) aR[q] = aI[q] = make_double2(0.0, 0.0);
+  c.forward(v, bases(el.y, eb.x, eb.y), K, [&](int q, int, double2 R, double2 I) { aR[q] = R; aI[q] = I; });
   // (b_R, b_I) = lP1 (BIx, -BRx)
   fx_half<N>(sf(0), sf(2), j, K, X, Y);
 #pragma unroll
@@ -454,10 +456,10 @@ k_adj_qw_row(Geom g, AdjP p, double2* __restrict__ SF, const double2* __restrict
   c.inverse(X, Y, b, eb);
 #pragma unroll
   for (int r = 0; r < 8; ++r) { v[r].x = fx_mulhi(l[r].x, b[r].y); v[r].y = fx_mulhi(l[r].x, b[r].x); }
-  c.forward(v, bases(el.x + 1, eb.y, eb.x), K, [&](int, int k, double2 R, double2 I) {
+  c.forward(v, bases(el.x + 1, eb.y, eb.x), K, [&](int q, int k, double2 R, double2 I) {
     const double kx = (double)k;
-    sf(0)[k] = cadd(cscale(cmul_mi(sf(4)[k]), kx), R);
-    sf(2)[k] = cadd(cscale(cmul_mi(sf(5)[k]), kx), I);
+    sf(0)[k] = cadd(cscale(cmul_mi(aR[q]), kx), R);
+    sf(2)[k] = cadd(cscale(cmul_mi(aI[q]), kx), I);
   });
 }
 
