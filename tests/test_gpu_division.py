@@ -16,7 +16,7 @@ CSRC = ROOT / "qg-ybjp-model_gb300" / "csrc"
 
 
 @pytest.fixture(scope="module")
-def checker(tmp_path_factory):
+def division(tmp_path_factory):
     so = tmp_path_factory.mktemp("division") / "division_check.so"
     subprocess.run(["nvcc", "-gencode", "arch=compute_103a,code=sm_103a", "-O3", "-std=c++17", "-shared", "-Xcompiler", "-fPIC",
                     "-I", str(CSRC), "-I", str(ROOT / "include"), str(ROOT / "tests" / "division_check.cu"), "-o", str(so)],
@@ -43,9 +43,9 @@ def _same(q, exact):
 
 
 @pytest.mark.parametrize("e0,e1", [(1003, 1043), (723, 1323), (1023, 1023)])
-def test_random_quotients(checker, e0, e1):
+def test_random_quotients(division, e0, e1):
     # (2^28 of them; one lies within 2^-50 of an ulp of a midpoint with a probability below 2^-20)
-    assert checker.division_random(12345 + e0, 1 << 28, e0, e1) == 0
+    assert division.division_random(12345 + e0, 1 << 28, e0, e1) == 0
 
 
 def _operands():
@@ -60,10 +60,10 @@ DIVISORS = [-1.0, -0.25, -2.0 ** 40, -(2.0 - 2.0 ** -52), -(1.0 + 2.0 ** -52), -
 
 @pytest.mark.parametrize("one", [0, 1])
 @pytest.mark.parametrize("d", DIVISORS)
-def test_edges(checker, d, one):
+def test_edges(division, d, one):
     a = np.concatenate([_operands(), -_operands()])
     with np.errstate(all="ignore"):
-        q, exact = _list(checker, one, a, np.full_like(a, d))
+        q, exact = _list(division, one, a, np.full_like(a, d))
     small = np.isfinite(a) & (a != 0) & ((np.abs(a) < 2.0 ** -969) | (np.abs(exact) < np.finfo(float).tiny))
     assert _same(q, exact)[~small].all(), (a[~small][~_same(q, exact)[~small]], d)
     assert (np.abs(q.view(np.int64) - exact.view(np.int64))[small] <= 1).all()
