@@ -4,6 +4,7 @@ quotient or the dividend is subnormal or nearly so (below 2^-969, where the resi
 from __future__ import annotations
 
 import ctypes as C
+import shutil
 import subprocess
 from pathlib import Path
 
@@ -18,7 +19,7 @@ CSRC = ROOT / "qg-ybjp-model_gb300" / "csrc"
 @pytest.fixture(scope="module")
 def division(tmp_path_factory):
     so = tmp_path_factory.mktemp("division") / "division_check.so"
-    subprocess.run(["nvcc", "-gencode", "arch=compute_103a,code=sm_103a", "-O3", "-std=c++17", "-shared", "-Xcompiler", "-fPIC",
+    subprocess.run([shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc", "-gencode", "arch=compute_103a,code=sm_103a", "-O3", "-std=c++17", "-shared", "-Xcompiler", "-fPIC",
                     "-I", str(CSRC), "-I", str(ROOT / "include"), str(ROOT / "tests" / "division_check.cu"), "-o", str(so)],
                    check=True, capture_output=True)
     L = C.CDLL(str(so))
