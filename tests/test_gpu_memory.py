@@ -2,6 +2,8 @@
 back what it keeps unused before a later call fails."""
 from __future__ import annotations
 
+import gc
+
 import numpy as np
 import pytest
 
@@ -18,10 +20,7 @@ class _Leave:
 
     def __init__(self, free):
         import torch
-        torch.cuda.synchronize()
-        torch.cuda.empty_cache()
-        n = torch.cuda.mem_get_info()[0] - free
-        self.held = torch.empty(n, dtype=torch.uint8, device="cuda")
+        self.held = torch.empty(_free() - free, dtype=torch.uint8, device="cuda")
 
     def __enter__(self):
         return self
@@ -34,6 +33,8 @@ class _Leave:
 
 def _free():
     import torch
+    gc.collect()               # (handles that an earlier test left to it)
+    torch.cuda.synchronize()
     torch.cuda.empty_cache()
     return torch.cuda.mem_get_info()[0]
 
